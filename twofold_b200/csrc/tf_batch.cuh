@@ -64,11 +64,10 @@ struct Batch {
     uint32_t* impactRestLevel;
     uint8_t* color;           // by contact
     Axis* axes;               // by contact, kAxesPerContact each; built for the contacts solved one at a time
-    // The laned contacts' solver records: kRowWords float4 components, component k of slot s at
-    // rows[k * rowStride + s], a laned contact's slot being contactFirst + its position in the world's colored
-    // list; slotOf maps a contact (contactFirst + i) to its slot.
+    // The laned contacts' solver records: kRowWords float4 components each (rowOf finds them), a laned contact's
+    // slot being contactFirst + its position in the world's colored list; slotOf maps a contact (contactFirst +
+    // i) to its slot.
     float4* rows;
-    size_t rowStride;
     uint32_t* slotOf;
     // The flat solve of batches of many worlds: every body's solver state (kFlatBodyWords float4 per body:
     // velocity, spin, displacement and turn of the substep, type and awake flags), and per color the record

@@ -1634,7 +1634,7 @@ public:
         TF_ALLOC(dColor, ncon);
         TF_ALLOC(dCflags, ncon);
         TF_ALLOC(dAxes, ncon * kAxesPerContact);
-        TF_ALLOC(dRows, ncon * kRowWords);
+        TF_ALLOC(dRows, (ncon + kRowTile - 1) / kRowTile * kRowTile * kRowWords);
         TF_ALLOC(dSlotOf, ncon);
         TF_ALLOC(dFlatBodies, nb * kFlatBodyWords);
         TF_ALLOC(dFlatPose, nb * kFlatPoseWords);
@@ -1834,7 +1834,6 @@ public:
         B.cflags = dCflags.ptr;
         B.axes = dAxes.ptr;
         B.rows = dRows.ptr;
-        B.rowStride = dContacts[0].n;
         B.slotOf = dSlotOf.ptr;
         B.flatBodies = dFlatBodies.ptr;
         B.flatPose = dFlatPose.ptr;

@@ -1460,8 +1460,10 @@ constexpr uint32_t kNotColorable = 0x80000000u;
 //
 // The reference solves a color's contacts from a packed per-batch record rather than from its Contact
 // (ContactLanes, src/internal.h:579-621, built by prepareBatch, src/lanes.cpp:66-110). Here each laned contact
-// has one at its slot (contactFirst + its position in the world's colored list), component-major: component k
-// of every slot is one float4 array, so the lanes of a color read consecutive 16-byte words. It holds what the
+// has one at its slot (contactFirst + its position in the world's colored list), component-major within tiles of
+// kRowTile slots: component k of a tile's slots is 128 consecutive bytes, so the eight contacts a warp solves read
+// consecutive 16-byte words, and every component of a record lies at a constant offset from its first (one array
+// per component took a 64-bit offset each, 45 of them, which the passes kept in registers and spilled). It holds what the
 // substep's passes read of a contact and its points, and the impulses, which stay in it from k_prepare to
 // k_finish (k_finish writes them back into the contact; a mid-step refresh takes them back first and builds
 // the record again). Of each axis (makeAxis, src/solver.cpp:5-17) it keeps the velocity changes per unit
@@ -1482,12 +1484,18 @@ enum RowWord : int {
     kRowWords = kRowPoint + 4 * kRowPointWords
 };
 constexpr uint32_t kNoSlot = 0xffffffffu;
+constexpr uint32_t kRowTile = 8;  // slots of a tile; a record's next component is this many float4 on
+
+__device__ __forceinline__ float4* rowOf(const Batch& B, uint32_t slot) {
+    return B.rows + (size_t)(slot / kRowTile) * (kRowTile * kRowWords) + slot % kRowTile;
+}
 
 __device__ __forceinline__ float4 f4(const Vec3& v, float w) { return make_float4(v.x, v.y, v.z, w); }
 __device__ __forceinline__ Vec3 xyz(const float4& v) { return Vec3{ v.x, v.y, v.z }; }
 
-// Six vectors (18 floats) into 5 consecutive components at R + first * S, and back.
-__device__ __forceinline__ void putSix(float4* R, size_t S, int first, const Vec3 (&v)[6]) {
+// Six vectors (18 floats) into 5 consecutive components of a record, from component `first`, and back.
+__device__ __forceinline__ void putSix(float4* R, int first, const Vec3 (&v)[6]) {
+    constexpr int S = kRowTile;
     R[first * S] = make_float4(v[0].x, v[0].y, v[0].z, v[1].x);
     R[(first + 1) * S] = make_float4(v[1].y, v[1].z, v[2].x, v[2].y);
     R[(first + 2) * S] = make_float4(v[2].z, v[3].x, v[3].y, v[3].z);
@@ -1499,7 +1507,8 @@ struct SixVec {
     Vec3 v[6];
 };
 
-__device__ __forceinline__ SixVec getSix(const float4* R, size_t S, int first) {
+__device__ __forceinline__ SixVec getSix(const float4* R, int first) {
+    constexpr int S = kRowTile;
     const float4 a = R[first * S], b = R[(first + 1) * S], c = R[(first + 2) * S], d = R[(first + 3) * S],
                  e = R[(first + 4) * S];
     SixVec x;
@@ -1517,8 +1526,8 @@ __device__ __forceinline__ SixVec getSix(const float4* R, size_t S, int first) {
 static __device__ void buildRow(const Batch& B, const WorldInfo& wi, uint32_t slot, uint32_t ci) {
     const DContact& c = B.contacts[wi.contactFirst + ci];
     const AxisBody xa = axisBodyOf(B.bodies[c.bodyA]), xb = axisBodyOf(B.bodies[c.bodyB]);
-    float4* R = B.rows + slot;
-    const size_t S = B.rowStride;
+    constexpr int S = kRowTile;
+    float4* R = rowOf(B, slot);
     const int n = c.count;
     R[kRowHead * S] = make_float4(__uint_as_float(c.bodyA), __uint_as_float(c.bodyB), __uint_as_float((uint32_t)n),
                                   __uint_as_float(ci));
@@ -1527,7 +1536,7 @@ static __device__ void buildRow(const Batch& B, const WorldInfo& wi, uint32_t sl
     R[kRowT2 * S] = f4(c.tangent2, 0.0f);
     const Vec3 linear[6] = { xa.invMassWorld * c.normal, xb.invMassWorld * c.normal, xa.invMassWorld * c.tangent1,
                              xb.invMassWorld * c.tangent1, xa.invMassWorld * c.tangent2, xb.invMassWorld * c.tangent2 };
-    putSix(R, S, kRowLinear, linear);
+    putSix(R, kRowLinear, linear);
     for (int i = 0; i < n; ++i) {
         const DPoint& p = c.points[i];
         const Axis xn = makeAxis(xa, xb, p.anchorA, p.anchorB, c.normal);
@@ -1539,14 +1548,14 @@ static __device__ void buildRow(const Batch& B, const WorldInfo& wi, uint32_t sl
         R[(at + 2) * S] = make_float4(x1.mass, x2.mass, p.normalImpulse, p.maxNormalImpulse);
         R[(at + 3) * S] = f4(p.tangentImpulse, 0.0f);
         const Vec3 angular[6] = { xn.angularA, xn.angularB, x1.angularA, x1.angularB, x2.angularA, x2.angularB };
-        putSix(R, S, at + 4, angular);
+        putSix(R, at + 4, angular);
     }
 }
 
 // The impulses a laned contact's record holds, back into the contact.
 __device__ __forceinline__ void returnImpulses(const Batch& B, uint32_t slot, DContact& c) {
-    const float4* R = B.rows + slot;
-    const size_t S = B.rowStride;
+    constexpr int S = kRowTile;
+    const float4* R = rowOf(B, slot);
     for (int i = 0; i < c.count; ++i) {
         const int at = kRowPoint + kRowPointWords * i;
         const float4 m = R[(at + 2) * S];
@@ -1951,12 +1960,12 @@ __device__ void forEachColor(const Group& g, const uint32_t* list, const uint32_
     }
 }
 
-// Calls f(slot) for the record slot (first + position) of every laned contact, a color at a time.
+// Calls f(position) for every position of each color's range, a color at a time.
 template <class F>
-__device__ void forEachColorSlot(const Group& g, uint32_t first, const uint32_t* start, uint32_t colors, F f) {
+__device__ __forceinline__ void forEachColorSlot(const Group& g, const uint32_t* start, uint32_t colors, F f) {
     for (uint32_t k = 0; k < colors; ++k) {
         const uint32_t end = start[k + 1];
-        for (uint32_t x = start[k] + g.tid; x < end; x += g.size) { f(first + x); }
+        for (uint32_t x = start[k] + g.tid; x < end; x += g.size) { f(x); }
         g.sync();
     }
 }
@@ -2281,16 +2290,17 @@ __device__ __forceinline__ Axis rowAxis(const Vec3& ra, const Vec3& rb, const Ve
 
 // warmStartLaned from the record: each point's normal and tangent impulses pushed in point order
 // (src/lanes.cpp:195-217).
-__device__ __forceinline__ void warmStartRow(const float4* R, size_t S, LanedBody& a, LanedBody& b, int n) {
+__device__ __forceinline__ void warmStartRow(const float4* R, LanedBody& a, LanedBody& b, int n) {
+    constexpr int S = kRowTile;
     const bool moveA = !anchored(a), moveB = !anchored(b);
     const Vec3 normal = xyz(R[kRowNormal * S]), t1 = xyz(R[kRowT1 * S]), t2 = xyz(R[kRowT2 * S]);
-    const SixVec lin = getSix(R, S, kRowLinear);
+    const SixVec lin = getSix(R, kRowLinear);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         if (i < n) {
             const int at = kRowPoint + kRowPointWords * i;
             const float4 pa = R[at * S], pb = R[(at + 1) * S], pm = R[(at + 2) * S], pt = R[(at + 3) * S];
-            const SixVec ang = getSix(R, S, at + 4);
+            const SixVec ang = getSix(R, at + 4);
             const Vec3 ra = xyz(pa), rb = xyz(pb), ti = xyz(pt);
             pushMoving(a, b, rowAxis(ra, rb, normal, lin.v[0], ang.v[0], lin.v[1], ang.v[1], pb.w), pm.z, moveA, moveB);
             pushMoving(a, b, rowAxis(ra, rb, t1, lin.v[2], ang.v[2], lin.v[3], ang.v[3], pm.x), dot(ti, t1), moveA, moveB);
@@ -2302,14 +2312,15 @@ __device__ __forceinline__ void warmStartRow(const float4* R, size_t S, LanedBod
 // solveLaned from the record: the soft normal rows, then friction forward in the biased pass and in reverse in
 // relax, with the operations and order of solveContact (src/solver.cpp:360-421, src/lanes.cpp:220-315). The
 // impulses go back to the record.
-__device__ __forceinline__ void solveRow(float4* R, size_t S, LanedBody& a, LanedBody& b, int n, const StepParams& P,
+__device__ __forceinline__ void solveRow(float4* R, LanedBody& a, LanedBody& b, int n, const StepParams& P,
                                          bool useBias) {
+    constexpr int S = kRowTile;
     const bool moveA = !anchored(a), moveB = !anchored(b);
     const Softness soft = (!moveA || !moveB) ? P.staticSoft : P.contactSoft;
     const float4 nf = R[kRowNormal * S];
     const Vec3 normal = xyz(nf), t1 = xyz(R[kRowT1 * S]), t2 = xyz(R[kRowT2 * S]);
     const float friction = nf.w;
-    const SixVec lin = getSix(R, S, kRowLinear);
+    const SixVec lin = getSix(R, kRowLinear);
     float ni[4] = { 0, 0, 0, 0 }, mi[4] = { 0, 0, 0, 0 };
     Vec3 ti[4] = {};
     const Vec3 dp = b.dp - a.dp;
@@ -2348,7 +2359,7 @@ __device__ __forceinline__ void solveRow(float4* R, size_t S, LanedBody& a, Lane
         const int at = kRowPoint + kRowPointWords * i;
         const Vec3 ra = xyz(R[at * S]), rb = xyz(R[(at + 1) * S]);
         const float4 pm = R[(at + 2) * S];
-        const SixVec ang = getSix(R, S, at + 4);
+        const SixVec ang = getSix(R, at + 4);
         const Axis x1 = rowAxis(ra, rb, t1, lin.v[2], ang.v[2], lin.v[3], ang.v[3], pm.x);
         const Axis x2 = rowAxis(ra, rb, t2, lin.v[4], ang.v[4], lin.v[5], ang.v[5], pm.y);
         const float old1 = dot(ti[i], t1), old2 = dot(ti[i], t2);
@@ -2591,9 +2602,8 @@ static __device__ void flatPosition(const FlatStore& f, uint32_t i, const StepPa
 template <class Store>
 __device__ __forceinline__ void warmRowAt(const Batch& B, const Store& st, uint32_t base, uint32_t limit,
                                           uint32_t slot) {
-    const size_t S = B.rowStride;
-    const float4* R = B.rows + slot;
-    const float4 h = R[kRowHead * S];
+    const float4* R = rowOf(B, slot);
+    const float4 h = R[kRowHead * kRowTile];
     const uint32_t ia = __float_as_uint(h.x) - base, ib = __float_as_uint(h.y) - base;
     const int n = (int)__float_as_uint(h.z);
 #if defined(TF_DEVICE_CHECKS)
@@ -2601,7 +2611,7 @@ __device__ __forceinline__ void warmRowAt(const Batch& B, const Store& st, uint3
 #endif
     if (n == 0) { return; }
     LanedBody a = st.loadLaned(ia), b = st.loadLaned(ib);
-    warmStartRow(R, S, a, b, n);
+    warmStartRow(R, a, b, n);
     if (!anchored(a)) { st.storeVW(ia, a); }
     if (!anchored(b)) { st.storeVW(ib, b); }
 }
@@ -2609,9 +2619,8 @@ __device__ __forceinline__ void warmRowAt(const Batch& B, const Store& st, uint3
 template <class Store>
 __device__ __forceinline__ void solveRowAt(const Batch& B, const StepParams& P, const Store& st, uint32_t base,
                                            uint32_t limit, uint32_t slot, bool bias) {
-    const size_t S = B.rowStride;
-    float4* R = B.rows + slot;
-    const float4 h = R[kRowHead * S];
+    float4* R = rowOf(B, slot);
+    const float4 h = R[kRowHead * kRowTile];
     const uint32_t ia = __float_as_uint(h.x) - base, ib = __float_as_uint(h.y) - base;
     const int n = (int)__float_as_uint(h.z);
 #if defined(TF_DEVICE_CHECKS)
@@ -2619,7 +2628,7 @@ __device__ __forceinline__ void solveRowAt(const Batch& B, const StepParams& P, 
 #endif
     if (n == 0) { return; }
     LanedBody a = st.loadLaned(ia), b = st.loadLaned(ib);
-    solveRow(R, S, a, b, n, P, bias);
+    solveRow(R, a, b, n, P, bias);
     if (!anchored(a)) { st.storeVW(ia, a); }
     if (!anchored(b)) { st.storeVW(ib, b); }
 }
@@ -2867,52 +2876,56 @@ __global__ void __launch_bounds__(kMaxBlock) k_substep(const __grid_constant__ B
             for (uint32_t i = g.tid; i < nb; i += g.size) { st.stage(i); }
             g.sync();
         }
-        for (uint32_t i = g.tid; i < nb; i += g.size) { st.integrateVelocityAt(i, P); }
-        g.sync();
         const uint32_t nj = wi.jointCount;
-        if constexpr (Joints) {
-            if (nj > 0) {
-                if (g.tid == 0) { runJoints(B, P, wi, st, 0); }
-                g.sync();
-            }
-        }
         const uint32_t base = wi.bodyFirst;
-        auto warmRow = [&](uint32_t slot) { warmRowAt(B, st, base, nb, slot); };
-        auto solveRowAtSlot = [&](uint32_t slot, bool bias) { solveRowAt(B, P, st, base, nb, slot, bias); };
-        auto warm = [&](uint32_t ci) { warmOne(B, wi, wc, st, ci); };
-        auto solve = [&](uint32_t ci, bool bias) { solveOne(B, P, wi, wc, st, ci, bias); };
         const uint32_t* rest = B.rest + cf;
         const uint32_t* icolored = B.impactColored + cf;
         const uint32_t* irest = B.impactRest + cf;
         const uint32_t* slotOf = B.slotOf + cf;
-        forEachColorSlot(g, cf, wc.colorStart, wc.colorCount, [&](uint32_t slot) { warmRow(slot); });
-        forEachLevel(g, rest, B.restLevel + cf, wc.restLevels, [&](uint32_t ci) { warm(ci); });
-        for (int pass = 0; pass < 2; ++pass) {
-            const bool bias = pass == 0;
+        bool refreshNext = false;
+        for (int s = sub;; ++s) {
+            for (uint32_t i = g.tid; i < nb; i += g.size) { st.integrateVelocityAt(i, P); }
+            g.sync();
             if constexpr (Joints) {
                 if (nj > 0) {
-                    if (g.tid == 0) { runJoints(B, P, wi, st, bias ? 1 : 2); }
+                    if (g.tid == 0) { runJoints(B, P, wi, st, 0); }
                     g.sync();
                 }
             }
-            forEachColorSlot(g, cf, wc.colorStart, wc.colorCount, [&](uint32_t slot) { solveRowAtSlot(slot, bias); });
-            forEachLevel(g, rest, B.restLevel + cf, wc.restLevels, [&](uint32_t ci) { solve(ci, bias); });
-            if (wc.impactCount > 0) {
-                forEachColor(g, icolored, wc.impactColorStart, wc.impactColorCount,
-                             [&](uint32_t ci) { solveRowAtSlot(slotOf[ci], bias); });
-                forEachLevel(g, irest, B.impactRestLevel + cf, wc.impactRestLevels,
-                             [&](uint32_t ci) { solve(ci, bias); });
+            forEachColorSlot(g, wc.colorStart, wc.colorCount, [&](uint32_t x) { warmRowAt(B, st, base, nb, cf + x); });
+            forEachLevel(g, rest, B.restLevel + cf, wc.restLevels, [&](uint32_t ci) { warmOne(B, wi, wc, st, ci); });
+            for (int pass = 0; pass < 2; ++pass) {
+                const bool bias = pass == 0;
+                if constexpr (Joints) {
+                    if (nj > 0) {
+                        if (g.tid == 0) { runJoints(B, P, wi, st, bias ? 1 : 2); }
+                        g.sync();
+                    }
+                }
+                // The active contacts, then the struck ones again (one call site: the solve is inlined once).
+                for (int struck = 0; struck < (wc.impactCount > 0 ? 2 : 1); ++struck) {
+                    forEachColorSlot(g, struck ? wc.impactColorStart : wc.colorStart,
+                                     struck ? wc.impactColorCount : wc.colorCount, [&](uint32_t x) {
+                                         solveRowAt(B, P, st, base, nb, struck ? slotOf[icolored[x]] : cf + x, bias);
+                                     });
+                    forEachLevel(g, struck ? irest : rest, (struck ? B.impactRestLevel : B.restLevel) + cf,
+                                 struck ? wc.impactRestLevels : wc.restLevels,
+                                 [&](uint32_t ci) { solveOne(B, P, wi, wc, st, ci, bias); });
+                }
+                if (bias) {
+                    for (uint32_t i = g.tid; i < nb; i += g.size) { st.integratePositionAt(i, P); }
+                    g.sync();
+                }
             }
-            if (bias) {
-                for (uint32_t i = g.tid; i < nb; i += g.size) { st.integratePositionAt(i, P); }
-                g.sync();
-            }
+            if (s + 1 >= P.substeps) { break; }
+            refreshNext = refreshedAt(wc, s + 1, P.substeps);
+            if (refreshNext) { break; }
         }
         if (st.staged) {
             for (uint32_t i = g.tid; i < nb; i += g.size) { st.unstage(i); }
             g.sync();
         }
-        if (sub + 1 < P.substeps && refreshedAt(wc, sub + 1, P.substeps)) {
+        if (refreshNext) {
             // The next substep starts with a refresh, whose axes use the inverse inertia at the new pose
             // (src/world.cpp:1660-1662).
             for (uint32_t i = g.tid; i < nb; i += g.size) {
@@ -3081,13 +3094,15 @@ __global__ void __launch_bounds__(256, 2) k_substep_flat(const __grid_constant__
             gridBarrier(B);
         }
     };
-    // Each color's contacts of every world, a color at a time.
+    // Each color's contacts of every world, a color at a time; the warps take them in turn over the CTAs, so that a
+    // color of few contacts still spreads over every SM.
+    const uint32_t spread = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + lane;
     auto colorsPass = [&](const uint32_t* list, const uint32_t* totals, uint32_t count, auto&& f) {
         uint32_t from = 0;
         for (uint32_t k = 0; k < count; ++k) {
             const uint32_t n = totals[k];
             if (!skip) {
-                for (uint32_t i = tid; i < n; i += threads) { f(list[from + i]); }
+                for (uint32_t i = spread; i < n; i += threads) { f(list[from + i]); }
             }
             from += n;
             gridBarrier(B);
@@ -3121,14 +3136,14 @@ __global__ void __launch_bounds__(256, 2) k_substep_flat(const __grid_constant__
     for (int pass = 0; pass < 2; ++pass) {
         const bool bias = pass == 0;
         jointsPass(bias ? 1 : 2);
-        colorsPass(B.flatColored, colorTotal, colors, [&](uint32_t slot) { solveRowAt(B, P, all, 0u, limit, slot, bias); });
-        restPass(false, [&](const WorldInfo& wi, const WorldCounts& wc, const FlatStore& st, uint32_t ci) {
-            solveOne(B, P, wi, wc, st, ci, bias);
-        });
-        colorsPass(B.flatImpact, impactTotal, impactColors, [&](uint32_t slot) { solveRowAt(B, P, all, 0u, limit, slot, bias); });
-        restPass(true, [&](const WorldInfo& wi, const WorldCounts& wc, const FlatStore& st, uint32_t ci) {
-            solveOne(B, P, wi, wc, st, ci, bias);
-        });
+        for (int struck = 0; struck < 2; ++struck) {
+            colorsPass(struck ? B.flatImpact : B.flatColored, struck ? impactTotal : colorTotal,
+                       struck ? impactColors : colors,
+                       [&](uint32_t slot) { solveRowAt(B, P, all, 0u, limit, slot, bias); });
+            restPass(struck != 0, [&](const WorldInfo& wi, const WorldCounts& wc, const FlatStore& st, uint32_t ci) {
+                solveOne(B, P, wi, wc, st, ci, bias);
+            });
+        }
         if (bias) {
             if (!skip) {
                 for (uint32_t gb = tid; gb < nb; gb += threads) { flatPosition(all, gb, P); }
@@ -3529,7 +3544,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
         // The laned contacts' impulses come back from their records.
         const uint32_t nColored = wc.colorStart[kColors];
         for (uint32_t x = g.tid; x < nColored; x += g.size) {
-            const uint32_t ci = __float_as_uint(B.rows[kRowHead * B.rowStride + cf + x].w);
+            const uint32_t ci = __float_as_uint(rowOf(B, cf + x)[kRowHead * kRowTile].w);
             if (!contactOk(B, wi, wc, ci, 18)) { continue; }
             returnImpulses(B, cf + x, cs[ci]);
         }
