@@ -234,6 +234,7 @@ public:
     DevArray<uint32_t> dSweepOrder, dSweepStart, dBigWorlds, dBigBodyStart;
     DevArray<SweepRec> dSweepRecs;
     std::vector<uint32_t> bigWorlds, bigBodyStart;  // worlds of more than kSweepBodies bodies
+    uint32_t bigCtas = 0;                           // CTAs of the cluster that steps each of them; 0: one CTA does
     DevArray<uint32_t> dSweepList, dHitParent;
     DevArray<unsigned long long> dHitKey, dGroupKey;
     DevArray<uint2> dCandItems, dContactItems;
@@ -368,6 +369,24 @@ public:
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeCooperative;
         attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelExC(&cfg, kernelEntry(id), ptrs);
+    }
+
+    // A launch of a cluster of bigCtas CTAs for every big world.
+    template <class... Args>
+    void launchClusters(int id, unsigned block, Args... args) {
+        void* ptrs[] = { (void*)&args... };
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)bigWorlds.size() * bigCtas);
+        cfg.blockDim = dim3(block);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = bigCtas;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         cudaLaunchKernelExC(&cfg, kernelEntry(id), ptrs);
@@ -1889,11 +1908,18 @@ public:
         auto smem = [&](int k) { return (size_t)splits[k].smemBytes; };
         cudaMemsetAsync(dWork.ptr, 0, kSlotCount * sizeof(uint32_t), stream);
         if (marks) { cudaEventRecord(marks[0], stream); }
+        const bool clusters = bigCtas > 0;                              // big worlds have launches of their own
+        const bool others = !clusters || bigWorlds.size() < worlds.size();  // and other worlds are left
         timed(0, rec, [&] {
-            launch(kKBroadphase, grids[0], threads(0), smem(0), B, P, splits[0], serial);
+            if (clusters) { launchClusters(kKBroadBig, threads(0), B, P, serial); }
+            if (others) { launch(kKBroadphase, grids[0], threads(0), smem(0), B, P, splits[0], serial); }
             if (!bigWorlds.empty()) {
                 launch(kKBroadPairs, smCount * 8, 256, 0, B, serial);
-                launch(kKBroadFinish, grids[0], threads(0), 0, B, splits[0], serial);
+                if (clusters) {
+                    launchClusters(kKBroadFinishBig, threads(0), B, splits[0], serial);
+                } else {
+                    launch(kKBroadFinish, grids[0], threads(0), 0, B, splits[0], serial);
+                }
             }
         });
         if (marks) { cudaEventRecord(marks[1], stream); }
@@ -1904,10 +1930,16 @@ public:
             }
             for (int c = 0; c < kPairClasses; ++c) { launch(kKCollide + c, flatGrids[c], flatThreads(c), 0, B, P, serial); }
         });
-        timed(1, rec, [&] { launch(kKNarrowphase, grids[1], threads(1), 0, B, P, splits[1], serial); });
+        timed(1, rec, [&] {
+            if (clusters) { launchClusters(kKNarrowphaseBig, threads(1), B, P, splits[1], serial); }
+            if (others) { launch(kKNarrowphase, grids[1], threads(1), 0, B, P, splits[1], serial); }
+        });
         timed(2, rec, [&] { launch(kKWake, grids[2], threads(2), 0, B, splits[2], serial); });
         if (marks) { cudaEventRecord(marks[2], stream); }
-        timed(3, rec, [&] { launch(kKPrepare, grids[3], threads(3), smem(3), B, P, splits[3], serial); });
+        timed(3, rec, [&] {
+            if (clusters) { launchClusters(kKPrepareBig, threads(3), B, P, splits[3], serial); }
+            if (others) { launch(kKPrepare, grids[3], threads(3), smem(3), B, P, splits[3], serial); }
+        });
         if (recording && !capturing) {
             const int rc = recordStep(B, serial);
             if (rc != TF_OK) { return rc; }
@@ -1934,12 +1966,13 @@ public:
             });
         }
         timed(6, rec, [&] {
-            launch(hasJoints ? kKFinishJoints : kKFinish, grids[6], threads(6), smem(6), B, P, splits[6], serial);
+            if (clusters) { launchClusters(hasJoints ? kKFinishJointsBig : kKFinishBig, threads(6), B, P, splits[6], serial); }
+            if (others) { launch(hasJoints ? kKFinishJoints : kKFinish, grids[6], threads(6), smem(6), B, P, splits[6], serial); }
         });
         if (marks) { cudaEventRecord(marks[3], stream); }
-        launches += smallBatch ? 5 + 1 + P.substeps + (P.substeps - 1) + (bigWorlds.empty() ? 0 : 2)
-                               : 5 + kPairClasses + P.substeps + (kPairClasses + 1) * (P.substeps - 1) +
-                                     (bigWorlds.empty() ? 0 : 2);
+        launches += smallBatch ? 5 + 1 + P.substeps + (P.substeps - 1)
+                               : 5 + kPairClasses + P.substeps + (kPairClasses + 1) * (P.substeps - 1);
+        launches += (bigWorlds.empty() ? 0 : 2) + (clusters && others ? 4 : 0);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) { return fail(TF_E_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e)); }
         return TF_OK;
@@ -1962,7 +1995,47 @@ public:
         for (int id : { kKBroadphase, kKSubstep, kKSubstepJoints, kKPrepare, kKFinish, kKFinishJoints }) {
             if ((rc = allow(kernelEntry(id))) != TF_OK) { return rc; }
         }
+        for (int id : kBigKernels) {
+            TF_CUDA(cudaFuncSetAttribute(kernelEntry(id), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        }
         done = true;
+        return TF_OK;
+    }
+
+    // The kernels that step big worlds by clusters, and the launch shape (kernel) each takes its threads from.
+    static constexpr int kBigKernels[6] = { kKBroadBig, kKBroadFinishBig, kKNarrowphaseBig, kKPrepareBig, kKFinishBig,
+                                            kKFinishJointsBig };
+    static constexpr int kBigShapes[6] = { 0, 0, 1, 3, 6, 6 };
+
+    // The clusters the big worlds' kernels run on: as many CTAs a world as leaves every world's cluster an SM a CTA
+    // (a power of two, at most kMaxCluster and what the device can place), none if that is one.
+    int configureBigWorlds() {
+        bigCtas = 0;
+        const size_t n = (size_t)(std::upper_bound(sortedSizes.begin(), sortedSizes.end(), kSweepBodies,
+                                                   std::greater<uint32_t>()) - sortedSizes.begin());
+        if (n > 0) {
+            for (uint32_t ctas = kMaxCluster; ctas >= 2 && bigCtas == 0; ctas /= 2) {
+                if (n * ctas > (size_t)smCount) { continue; }
+                bool fits = true;
+                for (int i = 0; i < 6 && fits; ++i) {
+                    cudaLaunchConfig_t cfg = {};
+                    cfg.gridDim = dim3(ctas);
+                    cfg.blockDim = dim3(shapes[kBigShapes[i]].threads);
+                    cudaLaunchAttribute attr[1];
+                    attr[0].id = cudaLaunchAttributeClusterDimension;
+                    attr[0].val.clusterDim.x = ctas;
+                    attr[0].val.clusterDim.y = 1;
+                    attr[0].val.clusterDim.z = 1;
+                    cfg.attrs = attr;
+                    cfg.numAttrs = 1;
+                    int active = 0;
+                    fits = cudaOccupancyMaxActiveClusters(&active, kernelEntry(kBigKernels[i]), &cfg) == cudaSuccess && active >= 1;
+                }
+                cudaGetLastError();  // a cluster size the device does not take is not an error of the step
+                if (fits) { bigCtas = ctas; }
+            }
+        }
+        for (int k : { 0, 1, 3, 6 }) { splits[k].firstWorld = bigCtas > 0 ? (uint32_t)n : 0u; }
         return TF_OK;
     }
 
@@ -2051,6 +2124,7 @@ public:
             const uint32_t bytes = std::min(sh.smemBytes, limit) / (16 * warps) * (16 * warps);
             Split& sp = splits[k];
             sp.bigBodies = sh.bigBodies;
+            sp.firstWorld = 0;
             sp.smemBytes = bytes;
             sp.big = stageFor(k, bytes);
             sp.small = stageFor(k, bytes / warps);
@@ -2064,6 +2138,7 @@ public:
             grids[k] = flatKernel(k) ? smCount * perSm
                                      : (int)std::max<size_t>(1, std::min<size_t>(needed, (size_t)smCount * perSm));
         }
+        if ((rc = configureBigWorlds()) != TF_OK) { return rc; }
         // The flat kernels, one grid per instantiation: as many CTAs as fit on the device at once.
         const void* flat[kFlatGrids] = {
             kernelEntry(kKCollide + kClassSpheres),  kernelEntry(kKCollide + kClassSpherePoly),
@@ -2154,7 +2229,9 @@ public:
         }
         const TapeStep ts{ T.worlds.ptr, T.contacts.ptr, T.colored.ptr, T.impactColored.ptr, T.rest.ptr, T.impactRest.ptr,
                            T.awake.ptr };
-        launch(kKTapeRecord, grids[3], shapes[3].threads, 0, B, splits[3], ts, serial);
+        Split every = splits[3];
+        every.firstWorld = 0;
+        launch(kKTapeRecord, grids[3], shapes[3].threads, 0, B, every, ts, serial);
         return TF_OK;
     }
 

@@ -6,8 +6,10 @@ namespace tfb {
 
 const void* finishKernels(int id) {
     switch (id) {
-        case kKFinish: return (const void*)k_finish<false>;
-        case kKFinishJoints: return (const void*)k_finish<true>;
+        case kKFinish: return (const void*)k_finish<false, false>;
+        case kKFinishJoints: return (const void*)k_finish<true, false>;
+        case kKFinishBig: return (const void*)k_finish<false, true>;
+        case kKFinishJointsBig: return (const void*)k_finish<true, true>;
         case kKTapeRecord: return (const void*)k_tape_record<0>;
         case kKAddForces: return (const void*)k_add_forces<0>;
         case kKPackPoses: return (const void*)k_pack_poses<0>;

@@ -6,7 +6,8 @@ namespace tfb {
 
 const void* solveKernels(int id) {
     switch (id) {
-        case kKPrepare: return (const void*)k_prepare<0>;
+        case kKPrepare: return (const void*)k_prepare<false>;
+        case kKPrepareBig: return (const void*)k_prepare<true>;
         case kKSubstep: return (const void*)k_substep<false>;
         case kKSubstepJoints: return (const void*)k_substep<true>;
         default: return nullptr;

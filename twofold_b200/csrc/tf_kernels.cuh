@@ -27,6 +27,7 @@ namespace tfb {
 
 constexpr int kMaxBlock = 512;
 constexpr int kMaxGroups = kMaxBlock / 32;
+constexpr uint32_t kMaxCluster = 16;  // CTAs of a cluster that steps a big world
 constexpr uint32_t kDevPairOverflow = 1u << 0, kDevContactOverflow = 1u << 1, kDevNonFinite = 1u << 2,
                    kDevTimeout = 1u << 3, kDevUnsupported = 1u << 4, kDevListOverflow = 1u << 6;
 
@@ -56,12 +57,17 @@ enum WorkSlot : int {
     kSlotCount = kSlotFlatBarrier + 2
 };
 
-// A group of threads that steps one world at a time: one warp, several warps, or the whole CTA.
-struct Group {
+// A group of threads that steps one world at a time: one warp, several warps, the whole CTA, or (Cluster) the CTAs
+// of a thread-block cluster.
+template <bool Cluster>
+struct GroupOf {
+    static constexpr bool kCluster = Cluster;
     uint32_t tid, size, id, count, lane, warp, warps;
 
     __device__ __forceinline__ void sync() const {
-        if (count == 1) {
+        if constexpr (Cluster) {
+            asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else if (count == 1) {
             __syncthreads();
         } else if (size == 32) {
             __syncwarp();
@@ -69,8 +75,25 @@ struct Group {
             asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "r"(size) : "memory");
         }
     }
-    // A barrier (as sync) that also tells every thread whether p held on any thread of the group.
-    __device__ __forceinline__ bool any(bool p) const {
+    // The group's one copy of a shared variable: a cluster's lies in its first CTA's shared memory.
+    template <class T>
+    __device__ __forceinline__ T* shared(T* p) const {
+        if constexpr (Cluster) {
+            uint64_t out;
+            asm("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"((uint64_t)p), "r"(0));
+            return reinterpret_cast<T*>(out);
+        } else {
+            return p;
+        }
+    }
+    // A barrier (as sync) that also tells every thread whether p held on any thread of the group. Clusters tell it
+    // through flag, a word of the group's shared memory that is zero beforehand and left as it is.
+    __device__ __forceinline__ bool any(bool p, uint32_t* flag) const {
+        if constexpr (Cluster) {
+            if (__any_sync(0xffffffffu, p) && lane == 0) { *(volatile uint32_t*)flag = 1u; }
+            sync();
+            return *(volatile uint32_t*)flag != 0u;
+        }
         if (count == 1) { return __syncthreads_or(p) != 0; }
         if (size == 32) {
             __syncwarp();
@@ -86,6 +109,7 @@ struct Group {
         return r != 0;
     }
 };
+using Group = GroupOf<false>;
 
 // blockDim.x is a multiple of size, size a multiple of 32, at most kMaxGroups groups.
 __device__ __forceinline__ Group makeGroup(uint32_t size) {
@@ -100,6 +124,29 @@ __device__ __forceinline__ Group makeGroup(uint32_t size) {
     return g;
 }
 
+__device__ __forceinline__ uint32_t clusterRank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t clusterSize() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+
+__device__ __forceinline__ GroupOf<true> makeClusterGroup() {
+    GroupOf<true> g;
+    g.size = blockDim.x * clusterSize();
+    g.count = 1;
+    g.id = 0;
+    g.tid = clusterRank() * blockDim.x + threadIdx.x;
+    g.lane = threadIdx.x & 31;
+    g.warp = g.tid >> 5;
+    g.warps = g.size >> 5;
+    return g;
+}
+
 // How a launch hands out worlds. A CTA takes worlds in largest-first order (B.order) and steps a world with
 // more than bigBodies bodies with all its threads; once it draws a world at or under that size every later
 // world is too, and its warps go on alone, a world each. Each mode has its own shared-memory staging
@@ -111,12 +158,25 @@ struct Split {
     uint32_t bigBodies;
     StageSizes big, small;
     uint32_t smemBytes;
+    uint32_t firstWorld;  // the worlds before it in largest-first order belong to another launch (forBigWorlds)
 };
 
 __device__ __forceinline__ uint32_t grabWarp(uint32_t* counter) {
     uint32_t v = 0;
     if ((threadIdx.x & 31) == 0) { v = atomicAdd(counter, 1u); }
     return __shfl_sync(0xffffffffu, v, 0);
+}
+
+// Takes one place from counters[c] for each calling thread and returns it: one atomic for the threads of a warp that
+// share a counter (most contacts and pairs of a world are of one class, and a cluster's counters are another SM's
+// shared memory).
+__device__ __forceinline__ uint32_t takePlace(uint32_t* counters, uint32_t c) {
+    const uint32_t active = __activemask(), lane = threadIdx.x & 31;
+    const uint32_t same = __match_any_sync(active, c);
+    const int leader = __ffs(same) - 1;
+    uint32_t at = 0;
+    if ((int)lane == leader) { at = atomicAdd(&counters[c], (uint32_t)__popc(same)); }
+    return __shfl_sync(same, at, leader) + __popc(same & ((1u << lane) - 1u));
 }
 
 // Calls body(group, world, slice, stage sizes) for every world of the batch, each exactly once. The body has
@@ -132,7 +192,7 @@ __device__ __forceinline__ void forWorlds(const Batch& B, int slotIndex, const S
         uint32_t o;
         if (!warpMode) {
             if (threadIdx.x == 0) {
-                const uint32_t t = atomicAdd(counter, 1u);
+                const uint32_t t = sp.firstWorld + atomicAdd(counter, 1u);
                 s_world = t;
                 s_big = (t < nw && B.info[B.order[t]].bodyCount > sp.bigBodies) ? 1u : 0u;
             }
@@ -144,10 +204,10 @@ __device__ __forceinline__ void forWorlds(const Batch& B, int slotIndex, const S
             if (!big) {
                 // Every later world is small too: from here on each warp takes worlds on its own.
                 warpMode = true;
-                if ((threadIdx.x >> 5) != 0) { o = grabWarp(counter); }
+                if ((threadIdx.x >> 5) != 0) { o = sp.firstWorld + grabWarp(counter); }
             }
         } else {
-            o = grabWarp(counter);
+            o = sp.firstWorld + grabWarp(counter);
         }
         if (o >= nw) { return; }
         const Group g = makeGroup(warpMode ? 32u : blockDim.x);
@@ -156,39 +216,93 @@ __device__ __forceinline__ void forWorlds(const Batch& B, int slotIndex, const S
     }
 }
 
+// Calls body(group, world, no slice, no stage sizes) for each big world (B.bigWorlds), a cluster a world: the CTAs of
+// a cluster are one group, apart by the cluster's hardware barrier. One CTA a world left 147 of 148 SMs idle in the
+// step of one large world.
+template <class Body>
+__device__ __forceinline__ void forBigWorlds(const Batch& B, Body&& body) {
+    const GroupOf<true> g = makeClusterGroup();
+    const uint32_t clusters = gridDim.x / clusterSize();
+    for (uint32_t k = blockIdx.x / clusterSize(); k < B.nBigWorlds; k += clusters) {
+        body(g, B.bigWorlds[k], (unsigned char*)nullptr, StageSizes{ 0u, 0u });
+        g.sync();
+    }
+    g.sync();  // no CTA leaves while another may still reach its shared memory
+}
+
 // Exclusive prefix sum over the group; every thread of the group calls it.
-__device__ __forceinline__ uint32_t groupScan(const Group& g, uint32_t v, uint32_t& total) {
+template <class G>
+__device__ __forceinline__ uint32_t groupScan(const G& g, uint32_t v, uint32_t& total) {
     __shared__ uint32_t sums[kMaxGroups][kMaxBlock / 32];
     uint32_t x = v;
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
         if ((int)g.lane >= o) { x += y; }
     }
-    if (g.warps == 1) {
-        total = __shfl_sync(0xffffffffu, x, 31);
-        return x - v;
-    }
-    if (g.lane == 31) { sums[g.id][g.warp] = x; }
-    g.sync();
-    if (g.warp == 0) {
-        uint32_t s = g.lane < g.warps ? sums[g.id][g.lane] : 0u;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-            if ((int)g.lane >= o) { s += y; }
+    if constexpr (G::kCluster) {
+        // The warps of each CTA, then the CTAs' totals, every CTA's in the first one's shared memory.
+        __shared__ uint32_t s_ctas[kMaxCluster];
+        const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, rank = clusterRank(), ctas = clusterSize();
+        if (g.lane == 31) { sums[0][warp] = x; }
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t s = g.lane < warps ? sums[0][g.lane] : 0u;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
+                if ((int)g.lane >= o) { s += y; }
+            }
+            if (g.lane < warps) { sums[0][g.lane] = s; }
+            if (g.lane == warps - 1) { g.shared(s_ctas)[rank] = s; }
         }
-        if (g.lane < g.warps) { sums[g.id][g.lane] = s; }
+        g.sync();
+        const uint32_t mine = g.lane < ctas ? g.shared(s_ctas)[g.lane] : 0u;
+        total = __reduce_add_sync(0xffffffffu, mine);
+        const uint32_t before = __reduce_add_sync(0xffffffffu, g.lane < rank ? mine : 0u);
+        const uint32_t prefix = before + (warp > 0 ? sums[0][warp - 1] : 0u) + x - v;
+        g.sync();
+        return prefix;
+    } else {
+        if (g.warps == 1) {
+            total = __shfl_sync(0xffffffffu, x, 31);
+            return x - v;
+        }
+        if (g.lane == 31) { sums[g.id][g.warp] = x; }
+        g.sync();
+        if (g.warp == 0) {
+            uint32_t s = g.lane < g.warps ? sums[g.id][g.lane] : 0u;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
+                if ((int)g.lane >= o) { s += y; }
+            }
+            if (g.lane < g.warps) { sums[g.id][g.lane] = s; }
+        }
+        g.sync();
+        const uint32_t prefix = (g.warp > 0 ? sums[g.id][g.warp - 1] : 0u) + x - v;
+        total = sums[g.id][g.warps - 1];
+        g.sync();
+        return prefix;
+    }
+}
+
+// Exclusive prefix sums of the n words at v, in place; ends with a group barrier.
+template <class G>
+__device__ void groupScanWords(const G& g, uint32_t* v, uint32_t n) {
+    uint32_t base = 0;
+    for (uint32_t first = 0; first < n; first += g.size) {
+        const uint32_t k = first + g.tid;
+        const uint32_t x = k < n ? v[k] : 0u;
+        uint32_t tot;
+        const uint32_t pre = groupScan(g, x, tot);
+        if (k < n) { v[k] = base + pre; }
+        base += tot;
     }
     g.sync();
-    const uint32_t prefix = (g.warp > 0 ? sums[g.id][g.warp - 1] : 0u) + x - v;
-    total = sums[g.id][g.warps - 1];
-    g.sync();
-    return prefix;
 }
 
 // Calls emit(i, position) for every i < n where pred(i) holds, positions dense and in index order. Ends with
 // a group barrier, so everything emit wrote is visible to the whole group on return.
-template <class Pred, class Emit>
-__device__ uint32_t groupCompact(const Group& g, uint32_t n, Pred pred, Emit emit) {
+template <class G, class Pred, class Emit>
+__device__ uint32_t groupCompact(const G& g, uint32_t n, Pred pred, Emit emit) {
     uint32_t base = 0;
     for (uint32_t start = 0; start < n; start += g.size) {
         const uint32_t i = start + g.tid;
@@ -204,8 +318,8 @@ __device__ uint32_t groupCompact(const Group& g, uint32_t n, Pred pred, Emit emi
 
 // Calls emit(i, position, k) for k < count(i) of every i < n, positions dense and in (i, k) order. Ends with a
 // group barrier.
-template <class Count, class Emit>
-__device__ uint32_t groupExpand(const Group& g, uint32_t n, Count count, Emit emit) {
+template <class G, class Count, class Emit>
+__device__ uint32_t groupExpand(const G& g, uint32_t n, Count count, Emit emit) {
     uint32_t base = 0;
     for (uint32_t start = 0; start < n; start += g.size) {
         const uint32_t i = start + g.tid;
@@ -219,10 +333,19 @@ __device__ uint32_t groupExpand(const Group& g, uint32_t n, Count count, Emit em
     return base;
 }
 
-// Reads the abort word once per CTA at a kernel's start: true when an earlier step of this launch sequence
+// Reads the abort word once per CTA (with Cluster, once per cluster: its CTAs have to agree) at a kernel's start: true when an earlier step of this launch sequence
 // overflowed a list, or this step did in an earlier kernel.
+template <bool Cluster = false>
 __device__ __forceinline__ bool stepAborted(const Batch& B, int serial) {
     __shared__ int s_skip;
+    if constexpr (Cluster) {
+        const GroupOf<true> g = makeClusterGroup();
+        if (g.tid == 0) { s_skip = *(volatile uint32_t*)B.abortStep <= (uint32_t)serial; }
+        g.sync();
+        const bool skip = *g.shared(&s_skip) != 0;
+        g.sync();
+        return skip;
+    }
     if (threadIdx.x == 0) { s_skip = *(volatile uint32_t*)B.abortStep <= (uint32_t)serial; }
     __syncthreads();
     const bool skip = s_skip != 0;
@@ -464,7 +587,8 @@ __device__ __forceinline__ uint32_t sweepBucket(const SweepGrid& s, float x) {
 // The first half of a big world's broadphase, after the growth: each live body's interval along x, their
 // range, and the bodies counted into buckets by where their intervals start. Bucket b then holds
 // sweepOrder[start[b - 1] .. start[b]), start[-1] being 0.
-static __device__ void prepareSweep(const Batch& B, const Group& g, const WorldInfo& wi, WorldCounts& wc, uint32_t w) {
+template <class G>
+static __device__ void prepareSweep(const Batch& B, const G& g, const WorldInfo& wi, WorldCounts& wc, uint32_t w) {
     const uint32_t n = wi.bodyCount;
     if (g.tid == 0) {
         wc.sweepMinKey = 0xffffffffu;
@@ -472,6 +596,7 @@ static __device__ void prepareSweep(const Batch& B, const Group& g, const WorldI
         wc.candRaw = 0;
     }
     g.sync();
+    uint32_t least = 0xffffffffu, most = 0u;
     for (uint32_t i = g.tid; i < n; i += g.size) {
         const uint32_t gb = wi.bodyFirst + i;
         const DBody& b = B.bodies[gb];
@@ -480,11 +605,17 @@ static __device__ void prepareSweep(const Batch& B, const Group& g, const WorldI
             const float gr = B.grow[gb];
             lo = b.lo.x - gr - sweepSlack(b.lo.x);
             hi = b.hi.x + gr + sweepSlack(b.hi.x);
-            atomicMin(&wc.sweepMinKey, orderedKey(lo));
-            atomicMax(&wc.sweepMaxKey, orderedKey(hi));
+            least = min(least, orderedKey(lo));
+            most = max(most, orderedKey(hi));
         }
         B.sweepLo[gb] = lo;
         B.sweepHi[gb] = hi;
+    }
+    least = __reduce_min_sync(0xffffffffu, least);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (g.lane == 0) {
+        atomicMin(&wc.sweepMinKey, least);
+        atomicMax(&wc.sweepMaxKey, most);
     }
     g.sync();
     const SweepGrid grid = sweepGrid(wi, wc);
@@ -493,16 +624,7 @@ static __device__ void prepareSweep(const Batch& B, const Group& g, const WorldI
     g.sync();
     for (uint32_t i = g.tid; i < n; i += g.size) { atomicAdd(&start[sweepBucket(grid, B.sweepLo[wi.bodyFirst + i])], 1u); }
     g.sync();
-    uint32_t base = 0;
-    for (uint32_t first = 0; first < grid.buckets; first += g.size) {
-        const uint32_t k = first + g.tid;
-        const uint32_t v = k < grid.buckets ? start[k] : 0u;
-        uint32_t tot;
-        const uint32_t pre = groupScan(g, v, tot);
-        if (k < grid.buckets) { start[k] = base + pre; }
-        base += tot;
-    }
-    g.sync();
+    groupScanWords(g, start, grid.buckets);
     // Scattering advances each bucket's start to its end.
     for (uint32_t i = g.tid; i < n; i += g.size) {
         const uint32_t k = sweepBucket(grid, B.sweepLo[wi.bodyFirst + i]);
@@ -523,7 +645,8 @@ static __device__ void prepareSweep(const Batch& B, const Group& g, const WorldI
 // into B.cand. Returns the unique count.
 constexpr uint32_t kShortRow = 48;  // rows of keys at most this long are sorted by one thread
 
-static __device__ uint32_t sortKeys(const Group& g, const Batch& B, const WorldInfo& wi, uint32_t count) {
+template <class G>
+static __device__ uint32_t sortKeys(const G& g, const Batch& B, const WorldInfo& wi, uint32_t count) {
     uint32_t* row = B.rowScratch + wi.shapeFirst;
     uint64_t* tmp = B.mergeKeyA + wi.contactFirst;
     uint64_t* keys = B.cand + wi.candFirst;
@@ -532,16 +655,7 @@ static __device__ uint32_t sortKeys(const Group& g, const Batch& B, const WorldI
     g.sync();
     for (uint32_t i = g.tid; i < count; i += g.size) { atomicAdd(&row[(uint32_t)(keys[i] >> 32)], 1u); }
     g.sync();
-    uint32_t base = 0;
-    for (uint32_t start = 0; start < rows; start += g.size) {
-        const uint32_t r = start + g.tid;
-        const uint32_t v = r < rows ? row[r] : 0u;
-        uint32_t tot;
-        const uint32_t pre = groupScan(g, v, tot);
-        if (r < rows) { row[r] = base + pre; }
-        base += tot;
-    }
-    g.sync();
+    groupScanWords(g, row, rows);
     // Scattering advances each row's start to its end.
     for (uint32_t i = g.tid; i < count; i += g.size) {
         const uint64_t k = keys[i];
@@ -602,8 +716,37 @@ static __device__ uint32_t sortKeys(const Group& g, const Batch& B, const WorldI
 // Body pairs whose grown bounds overlap, then their shapes (src/world.cpp:788-842), and half-space pairs
 // (:844-867); the keys are sorted and made unique (:868-869). A warp of the group takes one body and its
 // lanes the bodies after it. Bodies are staged in the group's shared slice when at most stageN of them.
-static __device__ void finishCandidates(const Batch& B, const Group& g, const WorldInfo& wi, WorldCounts& wc, uint32_t w,
+template <class G>
+static __device__ void finishCandidates(const Batch& B, const G& g, const WorldInfo& wi, WorldCounts& wc, uint32_t w,
                                  uint32_t total, int serial, uint32_t* cls, uint32_t* classBase);
+
+// Growth by the speculative distance and the travel over the step (src/world.cpp:754-765).
+__device__ __forceinline__ float growthOf(const DBody& b, const StepParams& P) {
+    float gr = P.tol.speculative;
+    if (b.alive && b.type != kStatic && !(lengthSquared(b.v) == 0.0f && lengthSquared(b.w) == 0.0f)) {
+        gr += (length(b.v) + length(b.w) * b.extent) * P.dt;
+    }
+    return gr;
+}
+
+// The first half of the big worlds' broadphase, a cluster a world.
+template <int Unused = 0>
+__global__ void __launch_bounds__(kMaxBlock) k_broad_big(const __grid_constant__ Batch B, const __grid_constant__ StepParams P, int serial) {
+    if (stepAborted<true>(B, serial)) { return; }
+    forBigWorlds(B, [&](const GroupOf<true>& g, uint32_t w, unsigned char*, const StageSizes&) {
+        const WorldInfo wi = B.info[w];
+        WorldCounts& wc = B.counts[w];
+        if (wi.jointCount > 0) {
+            if (g.tid == 0) { wakeJointPulled(B, wi, wc); }
+            g.sync();
+        }
+        for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
+            B.grow[wi.bodyFirst + i] = growthOf(B.bodies[wi.bodyFirst + i], P);
+        }
+        g.sync();
+        prepareSweep(B, g, wi, wc, w);
+    });
+}
 
 template <int Unused = 0>
 __global__ void __launch_bounds__(kMaxBlock) k_broadphase(const __grid_constant__ Batch B, const __grid_constant__ StepParams P, const __grid_constant__ Split sp, int serial) {
@@ -623,13 +766,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_broadphase(const __grid_constant_
             g.sync();
         }
         if (g.tid == 0) { s_count[g.id] = 0; }
-        // Growth by the speculative distance and the travel over the step (src/world.cpp:754-765).
         for (uint32_t i = g.tid; i < n; i += g.size) {
             const DBody& b = B.bodies[wi.bodyFirst + i];
-            float gr = P.tol.speculative;
-            if (b.alive && b.type != kStatic && !(lengthSquared(b.v) == 0.0f && lengthSquared(b.w) == 0.0f)) {
-                gr += (length(b.v) + length(b.w) * b.extent) * P.dt;
-            }
+            const float gr = growthOf(b, P);
             B.grow[wi.bodyFirst + i] = gr;
             if (useStage) {
                 PairBody p;
@@ -674,7 +813,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_broadphase(const __grid_constant_
 // The end of a world's broadphase: the raw keys sorted and made unique (src/world.cpp:868-869), then the
 // pairs join the flat list of their class: counted per class, a block of each list reserved for the
 // world, then scattered into it. A list that did not fit stops this step, and the host grows it.
-static __device__ void finishCandidates(const Batch& B, const Group& g, const WorldInfo& wi, WorldCounts& wc, uint32_t w,
+template <class G>
+static __device__ void finishCandidates(const Batch& B, const G& g, const WorldInfo& wi, WorldCounts& wc, uint32_t w,
                                  uint32_t total, int serial, uint32_t* cls, uint32_t* classBase) {
     {
         if (total > wi.candCap) {
@@ -700,7 +840,7 @@ static __device__ void finishCandidates(const Batch& B, const Group& g, const Wo
             const uint64_t key = B.cand[wi.candFirst + i];
             return pairClassOf(B, wi.shapeFirst + (uint32_t)(key >> 32), wi.shapeFirst + (uint32_t)(key & 0xffffffffu));
         };
-        for (uint32_t i = g.tid; i < unique; i += g.size) { atomicAdd(&cls[classOf(i)], 1u); }
+        for (uint32_t i = g.tid; i < unique; i += g.size) { takePlace(cls, (uint32_t)classOf(i)); }
         g.sync();
         if (g.tid < kPairClasses) {
             classBase[g.tid] = atomicAdd(B.work + kSlotCandItems + g.tid, cls[g.tid]);
@@ -709,7 +849,7 @@ static __device__ void finishCandidates(const Batch& B, const Group& g, const Wo
         g.sync();
         for (uint32_t i = g.tid; i < unique; i += g.size) {
             const int c = classOf(i);
-            const uint32_t pos = classBase[c] + atomicAdd(&cls[c], 1u);
+            const uint32_t pos = classBase[c] + takePlace(cls, (uint32_t)c);
             B.candItems[(size_t)c * B.candItemStride + pos] = make_uint2(w, i);
         }
         g.sync();
@@ -758,12 +898,22 @@ __global__ void __launch_bounds__(256) k_broad_pairs(const __grid_constant__ Bat
     }
 }
 
+// Calls body for every world of a launch: the big ones by cluster, or the others by CTA and warp.
+template <bool Cluster, class Body>
+__device__ __forceinline__ void forSomeWorlds(const Batch& B, int slotIndex, const Split& sp, unsigned char* smem, Body&& body) {
+    if constexpr (Cluster) {
+        forBigWorlds(B, body);
+    } else {
+        forWorlds(B, slotIndex, sp, smem, body);
+    }
+}
+
 // The rest of a big world's broadphase: half-space pairs, then the keys sorted and sent to their lists.
-template <int Unused = 0>
+template <bool Cluster>
 __global__ void __launch_bounds__(kMaxBlock) k_broad_finish(const __grid_constant__ Batch B, const __grid_constant__ Split sp, int serial) {
     __shared__ uint32_t s_class[kMaxGroups][kPairClasses], s_classBase[kMaxGroups][kPairClasses];
-    if (stepAborted(B, serial)) { return; }
-    forWorlds(B, kSlotBroadFinish, sp, nullptr, [&](const Group& g, uint32_t w, unsigned char*, const StageSizes&) {
+    if (stepAborted<Cluster>(B, serial)) { return; }
+    forSomeWorlds<Cluster>(B, kSlotBroadFinish, sp, nullptr, [&](const auto& g, uint32_t w, unsigned char*, const StageSizes&) {
         const WorldInfo wi = B.info[w];
         if (wi.bodyCount <= kSweepBodies) { return; }
         WorldCounts& wc = B.counts[w];
@@ -773,7 +923,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_broad_finish(const __grid_constan
         }
         g.sync();
         const uint32_t total = *(volatile uint32_t*)&wc.candRaw;
-        finishCandidates(B, g, wi, wc, w, total, serial, s_class[g.id], s_classBase[g.id]);
+        finishCandidates(B, g, wi, wc, w, total, serial, g.shared(s_class[g.id]), g.shared(s_classBase[g.id]));
     });
 }
 
@@ -869,7 +1019,8 @@ static __device__ __noinline__ int collidePlanarPair(const Batch& B, const StepP
 
 // Stores the placements of the round of collisions that just ended for the bodies of one world that were
 // placed in it; nothing reads a body's pose while its world is here.
-static __device__ void keepPlacements(const Batch& B, const Group& g, const WorldInfo& wi) {
+template <class G>
+static __device__ void keepPlacements(const Batch& B, const G& g, const WorldInfo& wi) {
     if (wi.planeBody == UINT32_MAX) { return; }
     if (!TF_OK_INDEX(B, wi.planeBody < B.totalBodies, 31, wi.bodyFirst, wi.planeBody)) { return; }
     const Vec3 n = planeNormal(B.bodies[wi.planeBody]);
@@ -1299,10 +1450,10 @@ __device__ __forceinline__ bool keyLess(uint64_t ka, uint32_t pa, uint64_t kb, u
     return ka != kb ? ka < kb : pa < pb;
 }
 
-template <int Unused = 0>
+template <bool Cluster>
 __global__ void __launch_bounds__(kMaxBlock) k_narrowphase(const __grid_constant__ Batch B, const __grid_constant__ StepParams P, const __grid_constant__ Split sp, int serial) {
-    if (stepAborted(B, serial)) { return; }
-    forWorlds(B, kSlotNarrow, sp, nullptr, [&](const Group& g, uint32_t w, unsigned char*, const StageSizes&) {
+    if (stepAborted<Cluster>(B, serial)) { return; }
+    forSomeWorlds<Cluster>(B, kSlotNarrow, sp, nullptr, [&](const auto& g, uint32_t w, unsigned char*, const StageSizes&) {
         const WorldInfo wi = B.info[w];
         WorldCounts& wc = B.counts[w];
         if (g.tid == 0) {
@@ -1461,9 +1612,8 @@ constexpr uint32_t kNotColorable = 0x80000000u;
 // The reference solves a color's contacts from a packed per-batch record rather than from its Contact
 // (ContactLanes, src/internal.h:579-621, built by prepareBatch, src/lanes.cpp:66-110). Here each laned contact
 // has one at its slot (contactFirst + its position in the world's colored list), component-major within tiles of
-// kRowTile slots: component k of a tile's slots is 128 consecutive bytes, so the eight contacts a warp solves read
-// consecutive 16-byte words, and every component of a record lies at a constant offset from its first (one array
-// per component took a 64-bit offset each, 45 of them, which the passes kept in registers and spilled). It holds what the
+// kRowTile slots: component k of a tile's slots is 128 consecutive bytes, so the lanes of a color read consecutive
+// 16-byte words, and every component of a record lies at a constant offset from its first. It holds what the
 // substep's passes read of a contact and its points, and the impulses, which stay in it from k_prepare to
 // k_finish (k_finish writes them back into the contact; a mid-step refresh takes them back first and builds
 // the record again). Of each axis (makeAxis, src/solver.cpp:5-17) it keeps the velocity changes per unit
@@ -1581,14 +1731,20 @@ constexpr uint8_t kColorPending = 0xff;
 // that property: the entries visited so far include every entry before them at a shared body. ends(x, a, b)
 // gives an entry's bodies (kNone for one that does not count); firstAt holds a word per body, set to kNone
 // beforehand.
-template <class Ends, class Pending, class Visit>
-static __device__ void visitInBodyOrder(const Group& g, uint32_t n, uint32_t* firstAt, Ends ends, Pending pending,
+template <class G, class Ends, class Pending, class Visit>
+static __device__ void visitInBodyOrder(const G& g, uint32_t n, uint32_t* firstAt, Ends ends, Pending pending,
                                         Visit visit) {
-    __shared__ uint32_t s_visits[kMaxGroups][2];
+    __shared__ uint32_t s_visits[kMaxGroups][2], s_left[3];
     if (n >= kOrderRoundsMin && n < (1u << 24)) {
         // A round costs two passes of n / size entries per thread; one thread takes an entry in about as long.
         const uint32_t worth = (n + g.size - 1) / g.size + 4;
-        if (g.tid == 0) { s_visits[g.id][0] = 0; }
+        uint32_t* visits = g.shared(s_visits[g.id]);
+        uint32_t* leftFlag = g.shared(s_left);
+        if (g.tid == 0) { visits[0] = 0; }
+        if constexpr (G::kCluster) {
+            if (g.tid == 0) { leftFlag[0] = 0; }
+            g.sync();
+        }
         for (uint32_t r = 0; r < kOrderRounds; ++r) {
             const uint32_t tag = (kOrderRounds - 1 - r) << 24;
             bool left = false;
@@ -1600,8 +1756,11 @@ static __device__ void visitInBodyOrder(const Group& g, uint32_t n, uint32_t* fi
                 if (a != kNone) { atomicMin(&firstAt[a], tag | x); }
                 if (b != kNone) { atomicMin(&firstAt[b], tag | x); }
             }
-            if (!g.any(left)) { return; }
-            if (g.tid == 0) { s_visits[g.id][(r + 1) & 1] = 0; }
+            if (!g.any(left, leftFlag + r % 3)) { return; }
+            if (g.tid == 0) {
+                visits[(r + 1) & 1] = 0;
+                if constexpr (G::kCluster) { leftFlag[(r + 1) % 3] = 0; }
+            }
             uint32_t visited = 0;
             for (uint32_t x = g.tid; x < n; x += g.size) {
                 if (!pending(x)) { continue; }
@@ -1612,9 +1771,9 @@ static __device__ void visitInBodyOrder(const Group& g, uint32_t n, uint32_t* fi
                     ++visited;
                 }
             }
-            if (visited) { atomicAdd(&s_visits[g.id][r & 1], visited); }
+            if (visited) { atomicAdd(&visits[r & 1], visited); }
             g.sync();
-            if (s_visits[g.id][r & 1] < worth) { break; }
+            if (*(volatile uint32_t*)&visits[r & 1] < worth) { break; }
         }
     }
     if (g.tid == 0) {
@@ -1628,7 +1787,8 @@ static __device__ void visitInBodyOrder(const Group& g, uint32_t n, uint32_t* fi
 // Greedy lowest free color of 32 over the moving bodies, in list order (src/lanes.cpp:356-374). endA/endB
 // hold each contact's moving bodies (kNone for one that does not move); endA carries kNotColorable for a
 // planar or rolling contact, which takes no color. masks (a word per body) start at 0, firstAt at kNone.
-static __device__ void colorInOrder(const Group& g, uint32_t n, const uint32_t* endA, const uint32_t* endB,
+template <class G>
+static __device__ void colorInOrder(const G& g, uint32_t n, const uint32_t* endA, const uint32_t* endB,
                                     uint32_t* masks, uint32_t* firstAt, uint8_t* color) {
     for (uint32_t x = g.tid; x < n; x += g.size) { color[x] = (endA[x] & kNotColorable) ? kNoColor : kColorPending; }
     g.sync();
@@ -1651,15 +1811,16 @@ static __device__ void colorInOrder(const Group& g, uint32_t n, const uint32_t* 
 
 // Groups a contact list by color: every color's contacts (any order within a color, which solves the same)
 // into colored, colors in ascending order, the uncolored ones into rest in list order.
-static __device__ void bucketByColor(const Group& g, uint32_t n, const uint32_t* list, const uint8_t* colorOf, uint32_t* colored,
+template <class G>
+static __device__ void bucketByColor(const G& g, uint32_t n, const uint32_t* list, const uint8_t* colorOf, uint32_t* colored,
                               uint32_t* rest, uint32_t* startOut, uint32_t& colorsUsed, uint32_t& restCount) {
     __shared__ uint32_t s_size[kMaxGroups][kColors + 1];
     __shared__ uint32_t s_fill[kMaxGroups][kColors + 1];
-    uint32_t* size = s_size[g.id];
-    uint32_t* fill = s_fill[g.id];
+    uint32_t* size = g.shared(s_size[g.id]);
+    uint32_t* fill = g.shared(s_fill[g.id]);
     for (uint32_t k = g.tid; k <= kColors; k += g.size) { size[k] = 0; }
     g.sync();
-    for (uint32_t x = g.tid; x < n; x += g.size) { atomicAdd(&size[colorOf[list[x]]], 1u); }
+    for (uint32_t x = g.tid; x < n; x += g.size) { takePlace(size, colorOf[list[x]]); }
     g.sync();
     if (g.tid == 0) {
         uint32_t sum = 0, used = 0;
@@ -1675,7 +1836,7 @@ static __device__ void bucketByColor(const Group& g, uint32_t n, const uint32_t*
     for (uint32_t x = g.tid; x < n; x += g.size) {
         const uint8_t k = colorOf[list[x]];
         if (k != kNoColor) {
-            const uint32_t at = atomicAdd(&fill[k], 1u);
+            const uint32_t at = takePlace(fill, k);
 #if defined(TF_DEVICE_CHECKS)
             if (at >= n) { continue; }
 #endif
@@ -1692,10 +1853,11 @@ static __device__ void bucketByColor(const Group& g, uint32_t n, const uint32_t*
 // contacts that share a moving body depend on that order: each takes a level one past the last earlier
 // contact on either of its moving bodies, so that the contacts of a level share no moving body and run
 // together while every body still meets its contacts in list order, which gives the sweep's own bits. The
-// levels come from visitInBodyOrder; one thread then reorders list by level (stably, within the level in list
+// levels come from visitInBodyOrder; one warp then reorders list by level (stably, within the level in list
 // order) and writes each level's end. last and firstAt (one word per body, zero and kNone on entry), tmp and
 // out (one word per entry) are scratch. Returns the levels.
-static __device__ uint32_t levelList(const Group& g, const Batch& B, const WorldInfo& wi, const DContact* cs,
+template <class G>
+static __device__ uint32_t levelList(const G& g, const Batch& B, const WorldInfo& wi, const DContact* cs,
                                      uint32_t* list, uint32_t n, uint32_t* levelEnd, uint32_t* last,
                                      uint32_t* firstAt, uint32_t* tmp, uint32_t* out) {
     __shared__ uint32_t s_levels[kMaxGroups];
@@ -1707,7 +1869,8 @@ static __device__ uint32_t levelList(const Group& g, const Batch& B, const World
         out[x] = b < wi.bodyCount && movingBody(B.bodies[c.bodyB]) ? b : kNone;
         levelEnd[x] = kNone;
     }
-    if (g.tid == 0) { s_levels[g.id] = 0; }
+    uint32_t* deepest = g.shared(&s_levels[g.id]);
+    if (g.tid == 0) { *deepest = 0; }
     g.sync();
     visitInBodyOrder(
         g, n, firstAt, [&](uint32_t x, uint32_t& a, uint32_t& b) { a = tmp[x], b = out[x]; },
@@ -1720,21 +1883,28 @@ static __device__ uint32_t levelList(const Group& g, const Batch& B, const World
             if (a != kNone) { last[a] = lev + 1; }
             if (b != kNone) { last[b] = lev + 1; }
             levelEnd[x] = lev;
-            atomicMax(&s_levels[g.id], lev + 1);
+            atomicMax(deepest, lev + 1);
         });
     for (uint32_t x = g.tid; x < n; x += g.size) { tmp[x] = levelEnd[x]; }
     g.sync();
-    const uint32_t levels = s_levels[g.id];
-    if (g.tid == 0) {
-        for (uint32_t l = 0; l < levels; ++l) { levelEnd[l] = 0; }
-        for (uint32_t x = 0; x < n; ++x) { ++levelEnd[tmp[x]]; }
-        uint32_t sum = 0;
-        for (uint32_t l = 0; l < levels; ++l) {
-            const uint32_t size = levelEnd[l];
-            levelEnd[l] = sum;  // the level's fill position, its end once filled
-            sum += size;
+    const uint32_t levels = *(volatile uint32_t*)deepest;
+    for (uint32_t l = g.tid; l < levels; l += g.size) { levelEnd[l] = 0; }
+    g.sync();
+    for (uint32_t x = g.tid; x < n; x += g.size) { atomicAdd(&levelEnd[tmp[x]], 1u); }
+    g.sync();
+    groupScanWords(g, levelEnd, levels);
+    // One warp fills the levels, 32 entries of the list at a time: an entry's place is its level's fill position
+    // plus the entries of that level before it among the 32. A level's fill position is its end once filled.
+    if (g.warp == 0) {
+        for (uint32_t first = 0; first < n; first += 32) {
+            const uint32_t x = first + g.lane;
+            const uint32_t lev = x < n ? tmp[x] : kNone;
+            const uint32_t same = __match_any_sync(0xffffffffu, lev);
+            if (x < n) { out[levelEnd[lev] + __popc(same & ((1u << g.lane) - 1u))] = list[x]; }
+            __syncwarp();
+            if (x < n && (same >> g.lane) == 1u) { levelEnd[lev] += __popc(same); }
+            __syncwarp();
         }
-        for (uint32_t x = 0; x < n; ++x) { out[levelEnd[tmp[x]]++] = list[x]; }
     }
     g.sync();
     for (uint32_t x = g.tid; x < n; x += g.size) { list[x] = out[x]; }
@@ -1743,8 +1913,8 @@ static __device__ uint32_t levelList(const Group& g, const Batch& B, const World
 }
 
 // Runs f on every entry of a leveled list, a level at a time.
-template <class F>
-__device__ void forEachLevel(const Group& g, const uint32_t* list, const uint32_t* levelEnd, uint32_t levels, F f) {
+template <class G, class F>
+__device__ void forEachLevel(const G& g, const uint32_t* list, const uint32_t* levelEnd, uint32_t levels, F f) {
     uint32_t begin = 0;
     for (uint32_t l = 0; l < levels; ++l) {
         const uint32_t end = levelEnd[l];
@@ -1756,23 +1926,26 @@ __device__ void forEachLevel(const Group& g, const uint32_t* list, const uint32_
 
 // Coloring is staged in the group's shared slice (masks by body, endpoints by active contact) when the world
 // fits stageBodies bodies and stageContacts active contacts, else in the world's global scratch.
-template <int Unused = 0>
+template <bool Cluster>
 __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ Batch B, const __grid_constant__ StepParams P, const __grid_constant__ Split sp, int serial) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ uint32_t s_fast[kMaxGroups], s_fastSolid[kMaxGroups], s_points[kMaxGroups];
     __shared__ uint32_t s_class[kMaxGroups][kPairClasses + 1], s_classBase[kMaxGroups][kPairClasses + 1];
-    if (stepAborted(B, serial)) { return; }
-    forWorlds(B, kSlotPrepare, sp, s_raw, [&](const Group& g, uint32_t w, unsigned char* slice, const StageSizes& ss) {
+    if (stepAborted<Cluster>(B, serial)) { return; }
+    forSomeWorlds<Cluster>(B, kSlotPrepare, sp, s_raw, [&](const auto& g, uint32_t w, unsigned char* slice, const StageSizes& ss) {
         const uint32_t stageBodies = ss.bodies, stageContacts = ss.contacts;
         const WorldInfo wi = B.info[w];
         WorldCounts& wc = B.counts[w];
         uint32_t nc = wc.nextContactCount;
         if (!TF_OK_INDEX(B, nc <= wi.contactCap, 6, w, nc)) { nc = 0; }
+        uint32_t* fast = g.shared(&s_fast[g.id]);
+        uint32_t* fastSolid = g.shared(&s_fastSolid[g.id]);
+        uint32_t* pointSum = g.shared(&s_points[g.id]);
         if (g.tid == 0) {
             wc.contactCount = nc;
-            s_fast[g.id] = 0;
-            s_fastSolid[g.id] = 0;
-            s_points[g.id] = 0;
+            *fast = 0;
+            *fastSolid = 0;
+            *pointSum = 0;
         }
         for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
             const uint32_t gb = wi.bodyFirst + i;
@@ -1815,10 +1988,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
                 uint8_t f = 0;
                 if (on && relativeTravel(a, b, P.dt) > P.tol.speculative) {
                     f |= kFlagFast;
-                    atomicAdd(&s_fast[g.id], 1u);
+                    atomicAdd(fast, 1u);
                     if (!isPlanar(a) && !isPlanar(b)) {
                         f |= kFlagFastSolid;
-                        atomicAdd(&s_fastSolid[g.id], 1u);
+                        atomicAdd(fastSolid, 1u);
                     }
                 }
                 B.cflags[cf + i] = f | (on ? kFlagActive : 0);
@@ -1828,8 +2001,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
         const uint32_t* act = B.active + cf;
         // A world with fast contacts is refreshed between substeps: its fast contacts join the flat list of
         // their pair class, its other active contacts the light list.
-        if (s_fast[g.id] > 0) {
-            uint32_t* cls = s_class[g.id];
+        const uint32_t nFast = *(volatile uint32_t*)fast;
+        if (nFast > 0) {
+            uint32_t* cls = g.shared(s_class[g.id]);
+            uint32_t* classBase = g.shared(s_classBase[g.id]);
             if (g.tid <= kPairClasses) { cls[g.tid] = 0; }
             g.sync();
             auto listOf = [&](uint32_t x) {
@@ -1837,16 +2012,16 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
                 if (!(B.cflags[cf + ci] & kFlagFast)) { return kPairClasses; }
                 return pairClassOf(B, cs[ci].shapeA, cs[ci].shapeB);
             };
-            for (uint32_t x = g.tid; x < nActive; x += g.size) { atomicAdd(&cls[listOf(x)], 1u); }
+            for (uint32_t x = g.tid; x < nActive; x += g.size) { takePlace(cls, (uint32_t)listOf(x)); }
             g.sync();
             if (g.tid <= kPairClasses) {
-                s_classBase[g.id][g.tid] = atomicAdd(B.work + kSlotFastItems + g.tid, cls[g.tid]);
+                classBase[g.tid] = atomicAdd(B.work + kSlotFastItems + g.tid, cls[g.tid]);
                 cls[g.tid] = 0;
             }
             g.sync();
             for (uint32_t x = g.tid; x < nActive; x += g.size) {
                 const int l = listOf(x);
-                const uint32_t pos = s_classBase[g.id][l] + atomicAdd(&cls[l], 1u);
+                const uint32_t pos = classBase[l] + takePlace(cls, (uint32_t)l);
                 B.contactItems[(size_t)l * B.contactItemStride + pos] = make_uint2(w, act[x]);
             }
             g.sync();
@@ -1883,7 +2058,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
                 break;
             }
         }
-        atomicAdd(&s_points[g.id], points);
+        points = __reduce_add_sync(0xffffffffu, points);
+        if (g.lane == 0) { atomicAdd(pointSum, points); }
         g.sync();
         colorInOrder(g, nActive, endA, endB, masks, firstAt, colorTmp);
         uint8_t* colorOf = B.color + cf;
@@ -1940,9 +2116,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
         if (g.tid == 0) {
             wc.activeCount = nActive;
             wc.impactCount = nImpact;
-            wc.fastCount = s_fast[g.id];
-            wc.fastSolidCount = s_fastSolid[g.id];
-            wc.activePoints = s_points[g.id];
+            wc.fastCount = *fast;
+            wc.fastSolidCount = *fastSolid;
+            wc.activePoints = *pointSum;
         }
         g.sync();
     });
@@ -1951,8 +2127,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
 // The substep (src/world.cpp:1658-1681).
 
 // Calls f(contact index) for every contact of each color in turn, the colors apart by a group barrier.
-template <class F>
-__device__ void forEachColor(const Group& g, const uint32_t* list, const uint32_t* start, uint32_t colors, F f) {
+template <class G, class F>
+__device__ void forEachColor(const G& g, const uint32_t* list, const uint32_t* start, uint32_t colors, F f) {
     for (uint32_t k = 0; k < colors; ++k) {
         const uint32_t end = start[k + 1];
         for (uint32_t x = start[k] + g.tid; x < end; x += g.size) { f(list[x]); }
@@ -2399,15 +2575,6 @@ __device__ __forceinline__ void solveRow(float4* R, LanedBody& a, LanedBody& b, 
     }
 }
 
-// In checked builds, whether a record's bodies lie in the world and its point count is at most 4.
-__device__ __forceinline__ bool rowOk(const Batch& B, const WorldInfo& wi, uint32_t ia, uint32_t ib, int n, int code) {
-#if defined(TF_DEVICE_CHECKS)
-    return TF_OK_INDEX(B, ia < wi.bodyCount && ib < wi.bodyCount && n >= 0 && n <= 4, code, wi.bodyFirst, ia);
-#else
-    return true;
-#endif
-}
-
 // A refresh works on the contact itself: a laned contact first takes its impulses back from its record, and
 // afterwards gets its record built again; a contact solved on its own gets its axes built again.
 __device__ __forceinline__ void takeImpulsesBack(const Batch& B, const WorldInfo& wi, uint32_t ci, DContact& c) {
@@ -2851,16 +3018,24 @@ template <bool Joints>
 __global__ void __launch_bounds__(kMaxBlock) k_substep(const __grid_constant__ Batch B, const __grid_constant__ StepParams P, const __grid_constant__ Split sp, int sub, int serial) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     if (stepAborted(B, serial)) { return; }
+    if (sub > 0) {
+        // No world has fast contacts: the first launch ran every substep.
+        uint32_t items = 0;
+        for (int l = 0; l <= kPairClasses; ++l) { items |= *(volatile uint32_t*)(B.work + kSlotFastItems + l); }
+        if (items == 0) { return; }
+    }
     forWorlds(B, kSlotSubstep + sub, sp, s_raw, [&](const Group& g, uint32_t w, unsigned char* sliceRaw, const StageSizes& ss) {
         float* slice = reinterpret_cast<float*>(sliceRaw);
         const uint32_t stageN = ss.bodies;
         const WorldInfo wi = B.info[w];
         const WorldCounts& wc = B.counts[w];
+        // A world's launch runs its substeps up to the next refresh, its solver state staged throughout; the
+        // launches of the substeps it ran pass it over.
+        if (sub > 0 && !refreshedAt(wc, sub, P.substeps)) { return; }
         const uint32_t cf = wi.contactFirst;
-        DContact* cs = B.contacts + cf;
         const uint32_t nb = wi.bodyCount;
         const SolverStore st{ slice, stageN, nb <= stageN, B.bodies + wi.bodyFirst };
-        if (refreshedAt(wc, sub, P.substeps)) {
+        if (sub > 0) {
             // The body half of this substep's refresh: the planar placements of its collisions are kept, and
             // every body takes a new base pose (src/world.cpp:1663-1666).
             keepPlacements(B, g, wi);
@@ -3245,18 +3420,19 @@ constexpr float kWideSweep = 16.0f;
 // x (a counting sort into the world's per-shape scratch), and each fast shape, a warp at a time, runs test on
 // the shapes of the buckets its bounds can overlap (low x within the widest narrow shape's extent below its
 // own low x, up to its high x) and on every wide shape. Each pair is visited once, as the full scan would.
-template <class Test>
-__device__ void sweepCandidates(const Batch& B, const Group& g, const WorldInfo& wi, uint32_t nf, Test& test) {
-    __shared__ uint32_t s_minX[kMaxGroups], s_maxX[kMaxGroups], s_ext[kMaxGroups], s_wide[kMaxGroups];
+template <class G, class Test>
+__device__ void sweepCandidates(const Batch& B, const G& g, const WorldInfo& wi, uint32_t nf, Test& test) {
+    __shared__ uint32_t s_range[kMaxGroups][4];  // lowest and highest x, widest extent, wide shapes
+    uint32_t* range = g.shared(s_range[g.id]);
     const uint32_t sf = wi.shapeFirst, ns = wi.shapeCount;
     uint32_t* order = B.rowScratch + sf;
     uint32_t* ends = B.rowLong + sf;
     uint32_t* wide = B.rowCount + sf;
     if (g.tid == 0) {
-        s_minX[g.id] = orderedKey(FLT_MAX);
-        s_maxX[g.id] = orderedKey(-FLT_MAX);
-        s_ext[g.id] = 0;
-        s_wide[g.id] = 0;
+        range[0] = orderedKey(FLT_MAX);
+        range[1] = orderedKey(-FLT_MAX);
+        range[2] = 0;
+        range[3] = 0;
     }
     g.sync();
     auto kindOf = [&](uint32_t i) {  // 0 skipped, 1 narrow, 2 wide
@@ -3265,17 +3441,26 @@ __device__ void sweepCandidates(const Batch& B, const Group& g, const WorldInfo&
         const float w = B.sweptHi[sf + i].x - B.sweptLo[sf + i].x;
         return (s.kind == kHalfSpace || s.kind == kMesh || !(w <= kWideSweep)) ? 2 : 1;
     };
+    uint32_t least = orderedKey(FLT_MAX), most = orderedKey(-FLT_MAX), widest = 0;
     for (uint32_t i = g.tid; i < ns; i += g.size) {
         const int k = kindOf(i);
-        if (k == 2) { wide[atomicAdd(&s_wide[g.id], 1u)] = i; }
+        if (k == 2) { wide[atomicAdd(&range[3], 1u)] = i; }
         if (k != 1) { continue; }
-        atomicMin(&s_minX[g.id], orderedKey(B.sweptLo[sf + i].x));
-        atomicMax(&s_maxX[g.id], orderedKey(B.sweptHi[sf + i].x));
-        atomicMax(&s_ext[g.id], __float_as_uint(B.sweptHi[sf + i].x - B.sweptLo[sf + i].x));
+        least = min(least, orderedKey(B.sweptLo[sf + i].x));
+        most = max(most, orderedKey(B.sweptHi[sf + i].x));
+        widest = max(widest, __float_as_uint(B.sweptHi[sf + i].x - B.sweptLo[sf + i].x));
+    }
+    least = __reduce_min_sync(0xffffffffu, least);
+    most = __reduce_max_sync(0xffffffffu, most);
+    widest = __reduce_max_sync(0xffffffffu, widest);
+    if (g.lane == 0) {
+        atomicMin(&range[0], least);
+        atomicMax(&range[1], most);
+        atomicMax(&range[2], widest);
     }
     g.sync();
     const uint32_t buckets = max(1u, ns / 4);
-    const float minX = fromOrderedKey(s_minX[g.id]), maxX = fromOrderedKey(s_maxX[g.id]);
+    const float minX = fromOrderedKey(range[0]), maxX = fromOrderedKey(range[1]);
     const float scale = (float)buckets / fmaxf(maxX - minX, 1e-6f);
     auto bucketOf = [&](float x) {
         const float t = fminf(fmaxf((x - minX) * scale, 0.0f), (float)(buckets - 1));
@@ -3287,22 +3472,14 @@ __device__ void sweepCandidates(const Batch& B, const Group& g, const WorldInfo&
         if (kindOf(i) == 1) { atomicAdd(&ends[bucketOf(B.sweptLo[sf + i].x)], 1u); }
     }
     g.sync();
-    if (g.tid == 0) {
-        uint32_t sum = 0;
-        for (uint32_t b = 0; b < buckets; ++b) {
-            const uint32_t n = ends[b];
-            ends[b] = sum;  // the bucket's fill position, its end once filled
-            sum += n;
-        }
-    }
-    g.sync();
+    groupScanWords(g, ends, buckets);  // each bucket's fill position, its end once filled
     for (uint32_t i = g.tid; i < ns; i += g.size) {
         if (kindOf(i) == 1) { order[atomicAdd(&ends[bucketOf(B.sweptLo[sf + i].x)], 1u)] = i; }
     }
     g.sync();
     // Padded, so that rounding in the widths and the subtraction below never drops a pair.
-    const float ext = __uint_as_float(s_ext[g.id]) * 1.001f + 1e-3f;
-    const uint32_t nWide = s_wide[g.id];
+    const float ext = __uint_as_float(range[2]) * 1.001f + 1e-3f;
+    const uint32_t nWide = range[3];
     for (uint32_t k = g.warp; k < nf; k += g.warps) {
         const uint32_t fi = B.sweepList[sf + k];
         const uint32_t b0 = bucketOf(B.sweptLo[sf + fi].x - ext), b1 = bucketOf(B.sweptHi[sf + fi].x);
@@ -3312,7 +3489,8 @@ __device__ void sweepCandidates(const Batch& B, const Group& g, const WorldInfo&
     }
 }
 
-static __device__ void sweepWorld(const Batch& B, const StepParams& P, const Group& g, const WorldInfo& wi, WorldCounts& wc,
+template <class G>
+static __device__ void sweepWorld(const Batch& B, const StepParams& P, const G& g, const WorldInfo& wi, WorldCounts& wc,
                            uint32_t* pairs, uint32_t* impacts) {
     const uint32_t sf = wi.shapeFirst, ns = wi.shapeCount, bf = wi.bodyFirst, nb = wi.bodyCount;
     uint32_t* parent = B.hitParent + bf;
@@ -3410,7 +3588,8 @@ static __device__ void sweepWorld(const Batch& B, const StepParams& P, const Gro
 // and break past their limits (src/world.cpp:1543-1560), the rest settle positions in order, twice over, and
 // every awake dynamic body's world inverse mass is built again at its settled pose. One thread runs the
 // joints; every thread first finds whether any joint was active.
-static __device__ void finishJoints(const Batch& B, const StepParams& P, const Group& g, const WorldInfo& wi) {
+template <class G>
+static __device__ void finishJoints(const Batch& B, const StepParams& P, const G& g, const WorldInfo& wi) {
     DJoint* js = B.joints + wi.jointFirst;
     auto endOf = [&](uint32_t gbody) { return gbody == kWorldEnd ? worldEnd() : jointBodyOf(B.bodies[gbody]); };
     bool anyActive = false;
@@ -3464,7 +3643,8 @@ static __device__ void finishJoints(const Batch& B, const StepParams& P, const G
 // a pair touches where the solver pushed on a point or a point overlaps (by more than the linear slop once it
 // touched); a hit is a pushed point approaching faster than the threshold in a contact solved this step.
 // Runs after restitution, on the poses the solve left, before kinematic bodies snap to their targets.
-static __device__ void reportTouches(const Batch& B, const StepParams& P, const Group& g, const WorldInfo& wi, WorldCounts& wc) {
+template <class G>
+static __device__ void reportTouches(const Batch& B, const StepParams& P, const G& g, const WorldInfo& wi, WorldCounts& wc) {
     const uint32_t nc = wc.contactCount;
     DContact* cs = B.contacts + wi.contactFirst;
     uint32_t touchingHere = 0;
@@ -3523,23 +3703,29 @@ static __device__ void reportTouches(const Batch& B, const StepParams& P, const 
     if (touchingHere > 0) { atomicAdd(&wc.touching, touchingHere); }
 }
 
-template <bool Joints>
+template <bool Joints, bool Cluster>
 __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Batch B, const __grid_constant__ StepParams P, const __grid_constant__ Split sp, int serial) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ uint32_t s_awake[kMaxGroups], s_islands[kMaxGroups], s_sweep[kMaxGroups], s_pairs[kMaxGroups],
         s_impacts[kMaxGroups], s_linked[kMaxGroups];
-    if (stepAborted(B, serial)) { return; }
-    forWorlds(B, kSlotFinish, sp, s_raw, [&](const Group& g, uint32_t w, unsigned char* slice, const StageSizes& ss) {
+    if (stepAborted<Cluster>(B, serial)) { return; }
+    forSomeWorlds<Cluster>(B, kSlotFinish, sp, s_raw, [&](const auto& g, uint32_t w, unsigned char* slice, const StageSizes& ss) {
         const uint32_t stageBodies = ss.bodies, stageContacts = ss.contacts;
         const WorldInfo wi = B.info[w];
         WorldCounts& wc = B.counts[w];
         const uint32_t cf = wi.contactFirst;
         DContact* cs = B.contacts + cf;
         const Axis* axes = B.axes + (size_t)cf * kAxesPerContact;
+        uint32_t* awakeSum = g.shared(&s_awake[g.id]);
+        uint32_t* islandSum = g.shared(&s_islands[g.id]);
+        uint32_t* sweepSum = g.shared(&s_sweep[g.id]);
+        uint32_t* pairSum = g.shared(&s_pairs[g.id]);
+        uint32_t* impactSum = g.shared(&s_impacts[g.id]);
+        uint32_t* linked = g.shared(&s_linked[g.id]);
         if (g.tid == 0) {
-            s_awake[g.id] = 0;
-            s_islands[g.id] = 0;
-            s_sweep[g.id] = 0;
+            *awakeSum = 0;
+            *islandSum = 0;
+            *sweepSum = 0;
         }
         // The laned contacts' impulses come back from their records.
         const uint32_t nColored = wc.colorStart[kColors];
@@ -3597,7 +3783,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
                     const float angle = sweepOf(b).angle;
                     for (uint32_t x = 0; x < b.shapeCount; ++x) {
                         const DShape& s = B.shapes[B.shapeList[b.shapeFirst + x]];
-                        if (sweepsShape(B.cx.pt, s, b, moved, angle)) { atomicAdd(&s_sweep[g.id], 1u); }
+                        if (sweepsShape(B.cx.pt, s, b, moved, angle)) { atomicAdd(sweepSum, 1u); }
                     }
                 }
             }
@@ -3616,10 +3802,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
         }
         g.sync();
         if (g.tid == 0) {
-            s_pairs[g.id] = 0;
-            s_impacts[g.id] = 0;
+            *pairSum = 0;
+            *impactSum = 0;
         }
-        if (P.continuous && s_sweep[g.id] > 0) { sweepWorld(B, P, g, wi, wc, &s_pairs[g.id], &s_impacts[g.id]); }
+        if (P.continuous && *(volatile uint32_t*)sweepSum > 0) { sweepWorld(B, P, g, wi, wc, pairSum, impactSum); }
         // Islands over contacts with points (src/world.cpp:1187-1233). The roots are each component's lowest
         // body whatever order the unions run in, so only the unions themselves run on one thread.
         const uint32_t nu = groupCompact(
@@ -3649,18 +3835,18 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
         // its root, until a round links nothing. Each component ends rooted at its lowest body, which is what
         // the reference's sequential unions give.
         for (;;) {
-            if (g.tid == 0) { s_linked[g.id] = 0; }
+            if (g.tid == 0) { *linked = 0; }
             g.sync();
             for (uint32_t x = g.tid; x < nu; x += g.size) {
                 if (!TF_OK_INDEX(B, uA[x] < wi.bodyCount && uB[x] < wi.bodyCount, 24, w, x)) { continue; }
                 const uint32_t ra = rootOf(parent, uA[x]), rb = rootOf(parent, uB[x]);
                 if (ra != rb) {
                     atomicMin(&parent[ra > rb ? ra : rb], ra < rb ? ra : rb);
-                    s_linked[g.id] = 1;
+                    *(volatile uint32_t*)linked = 1;
                 }
             }
             g.sync();
-            const bool again = s_linked[g.id] != 0;
+            const bool again = *(volatile uint32_t*)linked != 0;
             for (uint32_t i = g.tid; again && i < wi.bodyCount; i += g.size) { parent[i] = rootOf(parent, i); }
             g.sync();
             if (!again) { break; }
@@ -3686,14 +3872,21 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
             }
         }
         g.sync();
+        uint32_t awakeHere = 0, islandsHere = 0;
         for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
             DBody& b = B.bodies[wi.bodyFirst + i];
             if (!b.alive || b.type != kDynamic || !b.awake) { continue; }
             const uint32_t r = rootOf(parent, i);
             b.island = r;
-            atomicAdd(&s_awake[g.id], 1u);
-            if (r == i) { atomicAdd(&s_islands[g.id], 1u); }
+            ++awakeHere;
+            if (r == i) { ++islandsHere; }
             atomicMin(&islandTime[r], __float_as_uint(b.sleepTime));
+        }
+        awakeHere = __reduce_add_sync(0xffffffffu, awakeHere);
+        islandsHere = __reduce_add_sync(0xffffffffu, islandsHere);
+        if (g.lane == 0) {
+            atomicAdd(awakeSum, awakeHere);
+            atomicAdd(islandSum, islandsHere);
         }
         g.sync();
         for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
@@ -3707,12 +3900,12 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
         }
         g.sync();
         if (g.tid == 0) {
-            wc.awakeBodies = s_awake[g.id];
-            wc.awakeIslands = s_islands[g.id];
-            wc.bodySteps += s_awake[g.id];
-            wc.sweepShapes += s_sweep[g.id];
-            wc.sweptPairs = s_pairs[g.id];
-            wc.impacts = s_impacts[g.id];
+            wc.awakeBodies = *awakeSum;
+            wc.awakeIslands = *islandSum;
+            wc.bodySteps += *awakeSum;
+            wc.sweepShapes += *sweepSum;
+            wc.sweptPairs = *pairSum;
+            wc.impacts = *impactSum;
         }
         g.sync();
     });

@@ -12,18 +12,24 @@ namespace tfb {
 enum KernelId : int {
     kKBroadphase = 0,
     kKBroadPairs,
+    kKBroadBig,  // the big worlds', a cluster a world, here and below
     kKBroadFinish,
+    kKBroadFinishBig,
     kKNarrowphase,
+    kKNarrowphaseBig,
     kKWake,
     kKCollideAll,
     kKCollide,  // + pair class (kClassSpheres .. kClassMesh)
     kKRefreshAll = kKCollide + 6,
     kKRefresh,  // + pair class, kClassAny (the other active contacts) last
     kKPrepare = kKRefresh + 7,
+    kKPrepareBig,
     kKSubstep,
     kKSubstepJoints,
     kKFinish,
     kKFinishJoints,
+    kKFinishBig,
+    kKFinishJointsBig,
     kKTapeRecord,
     kKAddForces,
     kKPackPoses,
