@@ -204,6 +204,11 @@ public:
     LaunchShape shapes[kKernels];
     Split splits[kKernels];
     int grids[kKernels] = {};
+    // The world substep's launch with rooms for contact records (kRoomWarps): the same shape with at most
+    // kRoomWarps warps, staging what the rooms leave.
+    Split roomsSplit{};
+    uint32_t roomsThreads = 0;
+    int roomsGrid = 0;
     // k_collide per pair class, then k_refresh for the light list and per pair class.
     static constexpr int kFlatGrids = 2 * kPairClasses + 1;
     int flatGrids[kFlatGrids] = {};
@@ -1962,6 +1967,8 @@ public:
                     launchCooperative(hasJoints ? kKSubstepFlatJoints : kKSubstepFlat, grids[5], threads(5), B, P, i, serial);
                 } else {
                     launch(hasJoints ? kKSubstepJoints : kKSubstep, grids[5], threads(5), smem(5), B, P, splits[5], i, serial);
+                    launch(hasJoints ? kKSubstepRoomsJoints : kKSubstepRooms, roomsGrid, roomsThreads,
+                           roomsSplit.smemBytes + roomsThreads / 32 * kRoomBytes, B, P, roomsSplit, i, serial);
                 }
             });
         }
@@ -1972,7 +1979,7 @@ public:
         if (marks) { cudaEventRecord(marks[3], stream); }
         launches += smallBatch ? 5 + 1 + P.substeps + (P.substeps - 1)
                                : 5 + kPairClasses + P.substeps + (kPairClasses + 1) * (P.substeps - 1);
-        launches += (bigWorlds.empty() ? 0 : 2) + (clusters && others ? 4 : 0);
+        launches += (bigWorlds.empty() ? 0 : 2) + (clusters && others ? 4 : 0) + (shapes[5].flat ? 0 : P.substeps);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) { return fail(TF_E_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e)); }
         return TF_OK;
@@ -1992,13 +1999,33 @@ public:
             return TF_OK;
         };
         int rc;
-        for (int id : { kKBroadphase, kKSubstep, kKSubstepJoints, kKPrepare, kKFinish, kKFinishJoints }) {
+        for (int id : { kKBroadphase, kKSubstep, kKSubstepJoints, kKSubstepRooms, kKSubstepRoomsJoints, kKPrepare, kKFinish, kKFinishJoints }) {
             if ((rc = allow(kernelEntry(id))) != TF_OK) { return rc; }
         }
         for (int id : kBigKernels) {
             TF_CUDA(cudaFuncSetAttribute(kernelEntry(id), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         }
         done = true;
+        return TF_OK;
+    }
+
+    // The world substep's launch with rooms. A batch of more worlds than the device has warps for at a CTA a world
+    // gives worlds up to 96 bodies a warp each, whatever the shape without rooms gives them: 1024 impact worlds of 66
+    // bodies take 2760 us of substeps that way and 8455 with a CTA each.
+    int configureRooms() {
+        const LaunchShape& sh = shapes[5];
+        if (sh.flat) { return TF_OK; }
+        const void* fn = kernelEntry(hasJoints ? kKSubstepRoomsJoints : kKSubstepRooms);
+        const size_t limit = dynSmemLimit[fn];
+        roomsThreads = std::min(sh.threads, kRoomWarps * 32u);
+        if (manyWorlds() && !sh.chosen) { roomsThreads = kRoomWarps * 32u; }
+        const uint32_t warps = roomsThreads / 32, rooms = warps * kRoomBytes;
+        roomsSplit = Split{};
+        roomsSplit.bigBodies = manyWorlds() && !sh.chosen ? 96u : sh.bigBodies;
+        roomsSplit.smemBytes = (uint32_t)std::min<size_t>(std::max(sh.smemBytes, 32u * 1024u), limit - rooms) / (16 * warps) * (16 * warps);
+        roomsSplit.big = stageFor(5, roomsSplit.smemBytes);
+        roomsSplit.small = stageFor(5, roomsSplit.smemBytes / warps);
+        roomsGrid = std::min<int>(worldsGrid(roomsSplit.bigBodies, warps), smCount);
         return TF_OK;
     }
 
@@ -2042,25 +2069,46 @@ public:
     static bool flatKernel(int k) { return k == 4 || k == 7; }
     static constexpr uint32_t kMaxFlatBlock = 256;
 
+    bool manyWorlds() const { return worlds.size() >= (size_t)smCount * 4; }
+
+    // CTAs of `warps` warps that step every world at once: one for each world of more than bigBodies bodies, a warp
+    // for each of the others.
+    int worldsGrid(uint32_t bigBodies, uint32_t warps) const {
+        const size_t big = (size_t)(std::upper_bound(sortedSizes.begin(), sortedSizes.end(), bigBodies,
+                                                     std::greater<uint32_t>()) - sortedSizes.begin());
+        return (int)std::max<size_t>(1, std::min<size_t>(big + (sortedSizes.size() - big + warps - 1) / warps, 1u << 30));
+    }
+
     // Default launch shapes: batches of few worlds give every world a whole CTA (512 threads when a world
     // has more than 512 bodies); batches of many worlds give worlds of up to 96 bodies a warp each and the
     // larger ones the CTA. 64 KB of staging per CTA leaves room for three CTAs on an SM.
+    //
+    // The substep's, measured (us of substeps a step): many worlds take 128 threads and a CTA past 32 bodies (4096
+    // uneven worlds: 1952 at step 18 and 2576 at step 40, against 2168 and 3068 solved flat and 2331 and 3012 with
+    // 256 threads and 96 bodies; 600 jointed worlds: 1097 against 2439 flat). A few worlds take a CTA each, unless
+    // one has so many bodies that one SM holds up the step: then the whole batch is solved flat (planar piles of 1000
+    // bodies: 208 with a CTA and 225 flat, 2083 bodies: 470 and 310, 4163: 798 and 334; pyramids of 1036 boxes: 677
+    // and 676, 2081: 1609 and 659).
     LaunchShape defaultShape(int k) const {
         LaunchShape s;
-        const bool many = worlds.size() >= (size_t)smCount * 4;
+        const bool many = manyWorlds();
         s.threads = !many && maxWorldBodies > 512 && !flatKernel(k) ? 512u : 256u;
         s.bigBodies = many ? 96u : 0u;
         const bool stages = k == 0 || k == 3 || k == 5 || k == 6;
         s.smemBytes = stages ? 64u * 1024u : 0u;
-        if (k == 5 && many) {
-            // Batches of many worlds solve flat (k_substep_flat).
+        if (k == 5 && !many && maxWorldBodies > kFlatBodies) {
             s.threads = 256u;
             s.bigBodies = 0u;
             s.smemBytes = 0u;
             s.flat = true;
+        } else if (k == 5 && many) {
+            s.threads = 128u;
+            s.bigBodies = 32u;
+            s.smemBytes = 32u * 1024u;
         }
         return s;
     }
+    static constexpr uint32_t kFlatBodies = 1500;
 
     // Bodies (and active contacts) one staging slice of `bytes` holds, for the kernels that stage.
     static StageSizes stageFor(int k, uint32_t bytes) {
@@ -2131,13 +2179,9 @@ public:
             int perSm = 0;
             TF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fns[k], (int)sh.threads, bytes));
             if (perSm < 1) { return fail(TF_E_INVALID, "launch shape does not fit on an SM"); }
-            const size_t big = (size_t)(std::upper_bound(sortedSizes.begin(), sortedSizes.end(), sh.bigBodies,
-                                                         std::greater<uint32_t>()) -
-                                        sortedSizes.begin());
-            const size_t needed = big + (sortedSizes.size() - big + warps - 1) / warps;
-            grids[k] = flatKernel(k) ? smCount * perSm
-                                     : (int)std::max<size_t>(1, std::min<size_t>(needed, (size_t)smCount * perSm));
+            grids[k] = flatKernel(k) ? smCount * perSm : std::min(worldsGrid(sh.bigBodies, warps), smCount * perSm);
         }
+        if ((rc = configureRooms()) != TF_OK) { return rc; }
         if ((rc = configureBigWorlds()) != TF_OK) { return rc; }
         // The flat kernels, one grid per instantiation: as many CTAs as fit on the device at once.
         const void* flat[kFlatGrids] = {

@@ -8,8 +8,10 @@ const void* solveKernels(int id) {
     switch (id) {
         case kKPrepare: return (const void*)k_prepare<false>;
         case kKPrepareBig: return (const void*)k_prepare<true>;
-        case kKSubstep: return (const void*)k_substep<false>;
-        case kKSubstepJoints: return (const void*)k_substep<true>;
+        case kKSubstep: return (const void*)k_substep<false, false>;
+        case kKSubstepJoints: return (const void*)k_substep<true, false>;
+        case kKSubstepRooms: return (const void*)k_substep<false, true>;
+        case kKSubstepRoomsJoints: return (const void*)k_substep<true, true>;
         default: return nullptr;
     }
 }

@@ -54,7 +54,8 @@ enum WorkSlot : int {
     kSlotFlatMaxRestLevels = kSlotFlatMaxImpact + 1,
     kSlotFlatMaxImpactRestLevels = kSlotFlatMaxRestLevels + 1,
     kSlotFlatBarrier = kSlotFlatMaxImpactRestLevels + 1,  // arrivals, then barriers passed
-    kSlotCount = kSlotFlatBarrier + 2
+    kSlotActive = kSlotFlatBarrier + 2,  // active contacts of every world
+    kSlotCount = kSlotActive + 1
 };
 
 // A group of threads that steps one world at a time: one warp, several warps, the whole CTA, or (Cluster) the CTAs
@@ -1657,8 +1658,8 @@ struct SixVec {
     Vec3 v[6];
 };
 
+template <int S = kRowTile>
 __device__ __forceinline__ SixVec getSix(const float4* R, int first) {
-    constexpr int S = kRowTile;
     const float4 a = R[first * S], b = R[(first + 1) * S], c = R[(first + 2) * S], d = R[(first + 3) * S],
                  e = R[(first + 4) * S];
     SixVec x;
@@ -2114,6 +2115,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
             g.sync();
         }
         if (g.tid == 0) {
+            atomicAdd(B.work + kSlotActive, nActive);
             wc.activeCount = nActive;
             wc.impactCount = nImpact;
             wc.fastCount = *fast;
@@ -2136,15 +2138,6 @@ __device__ void forEachColor(const G& g, const uint32_t* list, const uint32_t* s
     }
 }
 
-// Calls f(position) for every position of each color's range, a color at a time.
-template <class F>
-__device__ __forceinline__ void forEachColorSlot(const Group& g, const uint32_t* start, uint32_t colors, F f) {
-    for (uint32_t k = 0; k < colors; ++k) {
-        const uint32_t end = start[k + 1];
-        for (uint32_t x = start[k] + g.tid; x < end; x += g.size) { f(x); }
-        g.sync();
-    }
-}
 // In checked builds, whether contact ci of a world can be read: in the list, with bodies in the world.
 __device__ __forceinline__ bool contactOk(const Batch& B, const WorldInfo& wi, const WorldCounts& wc,
                                           uint32_t ci, int code) {
@@ -2464,114 +2457,165 @@ __device__ __forceinline__ Axis rowAxis(const Vec3& ra, const Vec3& rb, const Ve
     return x;
 }
 
-// warmStartLaned from the record: each point's normal and tangent impulses pushed in point order
-// (src/lanes.cpp:195-217).
-__device__ __forceinline__ void warmStartRow(const float4* R, LanedBody& a, LanedBody& b, int n) {
-    constexpr int S = kRowTile;
-    const bool moveA = !anchored(a), moveB = !anchored(b);
-    const Vec3 normal = xyz(R[kRowNormal * S]), t1 = xyz(R[kRowT1 * S]), t2 = xyz(R[kRowT2 * S]);
-    const SixVec lin = getSix(R, kRowLinear);
+// A warp's room in shared memory for the records of the contacts it is about to solve, a lane's own record words a
+// lane apart (word k of lane l at [k * 32 + l]). The copies are asynchronous and each lane waits for its own, so a
+// color's records arrive while the group is still at the color before it. Rooms pay where contacts outweigh bodies:
+// 16 impact worlds (66 bodies, 490 contacts in 26 colors each) take 1840 us of substeps a step with them and 2570
+// without, 1024 of them 2760 and 4281, the box pyramid 344 and 377; but they leave an SM eight warps, and the 121-body
+// worlds of the uneven batch (0.2 to 0.5 contacts a body) then take 3312 us where they take 1952 without.
+constexpr uint32_t kRoomWarps = 8;  // warps of a CTA with rooms
+constexpr uint32_t kRoomBytes = kRowWords * 32 * (uint32_t)sizeof(float4);
+
+__device__ __forceinline__ void roomLoad(float4* mine, const float4* R) {
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(mine);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if (i < n) {
-            const int at = kRowPoint + kRowPointWords * i;
-            const float4 pa = R[at * S], pb = R[(at + 1) * S], pm = R[(at + 2) * S], pt = R[(at + 3) * S];
-            const SixVec ang = getSix(R, at + 4);
-            const Vec3 ra = xyz(pa), rb = xyz(pb), ti = xyz(pt);
-            pushMoving(a, b, rowAxis(ra, rb, normal, lin.v[0], ang.v[0], lin.v[1], ang.v[1], pb.w), pm.z, moveA, moveB);
-            pushMoving(a, b, rowAxis(ra, rb, t1, lin.v[2], ang.v[2], lin.v[3], ang.v[3], pm.x), dot(ti, t1), moveA, moveB);
-            pushMoving(a, b, rowAxis(ra, rb, t2, lin.v[4], ang.v[4], lin.v[5], ang.v[5], pm.y), dot(ti, t2), moveA, moveB);
-        }
+    for (int k = 0; k < kRowWords; ++k) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + k * 32 * 16), "l"(R + k * kRowTile) : "memory");
     }
 }
+__device__ __forceinline__ void roomWait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// solveLaned from the record: the soft normal rows, then friction forward in the biased pass and in reverse in
-// relax, with the operations and order of solveContact (src/solver.cpp:360-421, src/lanes.cpp:220-315). The
-// impulses go back to the record.
-__device__ __forceinline__ void solveRow(float4* R, LanedBody& a, LanedBody& b, int n, const StepParams& P,
-                                         bool useBias) {
-    constexpr int S = kRowTile;
+// One contact's passes, for either store, with body indices counted from the store's first body (`base`: the same
+// first body). The record's words are read at W, S apart: from a lane's room, or from the record itself (W = R); the
+// impulses go to the record. A laned contact's bodies are stored only where they move, so a static body shared by a
+// color's contacts is never written concurrently. The points' loops stay rolled: unrolled, a pass is 1,600
+// instructions of straight code, and a world with few warps waited for them 1.8 of every 8.4 cycles it was not at a
+// barrier (0.3 of 5.9 now; box pyramid).
+//
+// warmStartLaned: each point's normal and tangent impulses pushed in point order (src/lanes.cpp:195-217).
+template <int S, class Store>
+__device__ __forceinline__ void warmRecord(const Batch& B, const Store& st, uint32_t base, uint32_t limit, const float4* W) {
+    const float4 h = W[kRowHead * S];
+    const uint32_t ia = __float_as_uint(h.x) - base, ib = __float_as_uint(h.y) - base;
+    const int n = (int)__float_as_uint(h.z);
+#if defined(TF_DEVICE_CHECKS)
+    if (!TF_OK_INDEX(B, ia < limit && ib < limit && n >= 0 && n <= 4, 10, base, ia)) { return; }
+#endif
+    if (n == 0) { return; }
+    LanedBody a = st.loadLaned(ia), b = st.loadLaned(ib);
+    const bool moveA = !anchored(a), moveB = !anchored(b);
+    const Vec3 t1 = xyz(W[kRowT1 * S]), t2 = xyz(W[kRowT2 * S]);
+    const SixVec lin = getSix<S>(W, kRowLinear);
+    const float4* pt = W + kRowPoint * S;
+#pragma unroll 1
+    for (int i = 0; i < n; ++i, pt += kRowPointWords * S) {
+        const float in = pt[2 * S].z;
+        const Vec3 ti = xyz(pt[3 * S]);
+        const SixVec ang = getSix<S>(pt, 4);
+        auto push = [&](int k, float impulse) {
+            if (moveA) {
+                a.v -= lin.v[k] * impulse;
+                a.w -= ang.v[k] * impulse;
+            }
+            if (moveB) {
+                b.v += lin.v[k + 1] * impulse;
+                b.w += ang.v[k + 1] * impulse;
+            }
+        };
+        push(0, in);
+        push(2, dot(ti, t1));
+        push(4, dot(ti, t2));
+    }
+    if (moveA) { st.storeVW(ia, a); }
+    if (moveB) { st.storeVW(ib, b); }
+}
+
+// solveLaned: the soft normal rows, then friction forward in the biased pass and in reverse in relax, with the
+// operations and order of solveContact (src/solver.cpp:360-421, src/lanes.cpp:220-315).
+template <int S, class Store>
+__device__ __forceinline__ void solveRecord(const Batch& B, const StepParams& P, const Store& st, uint32_t base,
+                                            uint32_t limit, float4* W, float4* R, bool useBias) {
+    const float4 h = W[kRowHead * S];
+    const uint32_t ia = __float_as_uint(h.x) - base, ib = __float_as_uint(h.y) - base;
+    const int n = (int)__float_as_uint(h.z);
+#if defined(TF_DEVICE_CHECKS)
+    if (!TF_OK_INDEX(B, ia < limit && ib < limit && n >= 0 && n <= 4, 12, base, ia)) { return; }
+#endif
+    if (n == 0) { return; }
+    LanedBody a = st.loadLaned(ia), b = st.loadLaned(ib);
     const bool moveA = !anchored(a), moveB = !anchored(b);
     const Softness soft = (!moveA || !moveB) ? P.staticSoft : P.contactSoft;
-    const float4 nf = R[kRowNormal * S];
-    const Vec3 normal = xyz(nf), t1 = xyz(R[kRowT1 * S]), t2 = xyz(R[kRowT2 * S]);
-    const float friction = nf.w;
-    const SixVec lin = getSix(R, kRowLinear);
-    float ni[4] = { 0, 0, 0, 0 }, mi[4] = { 0, 0, 0, 0 };
-    Vec3 ti[4] = {};
+    const float4 nf = W[kRowNormal * S];
+    const Vec3 normal = xyz(nf);
+    const SixVec lin = getSix<S>(W, kRowLinear);
     const Vec3 dp = b.dp - a.dp;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if (i < n) {
-            const int at = kRowPoint + kRowPointWords * i;
-            const float4 pa = R[at * S], pb = R[(at + 1) * S], pm = R[(at + 2) * S];
-            ti[i] = xyz(R[(at + 3) * S]);
-            ni[i] = pm.z;
-            mi[i] = pm.w;
-            const float4 g0 = R[(at + 4) * S], g1 = R[(at + 5) * S];
-            const Vec3 ra = xyz(pa), rb = xyz(pb);
-            const Vec3 d = dp + turned(b, rb) - turned(a, ra);
-            const float sep = dot(d, normal) + pa.w;
-            float bias = 0.0f, massScale = 1.0f, impulseScale = 0.0f;
-            if (sep > 0.0f) {
-                bias = sep * P.invH;
-            } else if (useBias) {
-                bias = maxf(soft.biasRate * sep, -P.maxPushout);
-                massScale = soft.massScale;
-                impulseScale = soft.impulseScale;
-            }
-            const Axis x = rowAxis(ra, rb, normal, lin.v[0], Vec3{ g0.x, g0.y, g0.z }, lin.v[1],
-                                   Vec3{ g0.w, g1.x, g1.y }, pb.w);
-            const float vn = speedAlong(a, b, normal, x);
-            float impulse = -x.mass * massScale * (vn + bias) - impulseScale * ni[i];
-            const float total = maxf(ni[i] + impulse, 0.0f);
-            impulse = total - ni[i];
-            ni[i] = total;
-            mi[i] = maxf(mi[i], impulse);
-            pushMoving(a, b, x, impulse, moveA, moveB);
+    float4* pt = W + kRowPoint * S;
+#pragma unroll 1
+    for (int i = 0; i < n; ++i, pt += kRowPointWords * S) {
+        const float4 pa = pt[0], pb = pt[S];
+        const float2 im = reinterpret_cast<const float2*>(pt + 2 * S)[1];
+        const float4 g0 = pt[4 * S], g1 = pt[5 * S];
+        const Vec3 ra = xyz(pa), rb = xyz(pb);
+        const Vec3 d = dp + turned(b, rb) - turned(a, ra);
+        const float sep = dot(d, normal) + pa.w;
+        float bias = 0.0f, massScale = 1.0f, impulseScale = 0.0f;
+        if (sep > 0.0f) {
+            bias = sep * P.invH;
+        } else if (useBias) {
+            bias = maxf(soft.biasRate * sep, -P.maxPushout);
+            massScale = soft.massScale;
+            impulseScale = soft.impulseScale;
         }
+        const Axis x = rowAxis(ra, rb, normal, lin.v[0], Vec3{ g0.x, g0.y, g0.z }, lin.v[1], Vec3{ g0.w, g1.x, g1.y }, pb.w);
+        const float vn = speedAlong(a, b, normal, x);
+        float impulse = -x.mass * massScale * (vn + bias) - impulseScale * im.x;
+        const float total = maxf(im.x + impulse, 0.0f);
+        impulse = total - im.x;
+        reinterpret_cast<float2*>(pt + 2 * S)[1] = make_float2(total, maxf(im.y, impulse));
+        pushMoving(a, b, x, impulse, moveA, moveB);
     }
-    auto row = [&](int i) {
-        const int at = kRowPoint + kRowPointWords * i;
-        const Vec3 ra = xyz(R[at * S]), rb = xyz(R[(at + 1) * S]);
-        const float4 pm = R[(at + 2) * S];
-        const SixVec ang = getSix(R, at + 4);
+    const Vec3 t1 = xyz(W[kRowT1 * S]), t2 = xyz(W[kRowT2 * S]);
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        const int i = useBias ? k : n - 1 - k;
+        const float4* q = W + (kRowPoint + kRowPointWords * i) * S;
+        float4* out = R + (kRowPoint + kRowPointWords * i) * kRowTile;
+        const Vec3 ra = xyz(q[0]), rb = xyz(q[S]), old = xyz(q[3 * S]);
+        const float4 pm = q[2 * S];
+        const SixVec ang = getSix<S>(q, 4);
         const Axis x1 = rowAxis(ra, rb, t1, lin.v[2], ang.v[2], lin.v[3], ang.v[3], pm.x);
         const Axis x2 = rowAxis(ra, rb, t2, lin.v[4], ang.v[4], lin.v[5], ang.v[5], pm.y);
-        const float old1 = dot(ti[i], t1), old2 = dot(ti[i], t2);
+        const float old1 = dot(old, t1), old2 = dot(old, t2);
         float f1 = old1 - x1.mass * speedAlong(a, b, t1, x1);
         float f2 = old2 - x2.mass * speedAlong(a, b, t2, x2);
-        const float limit = friction * ni[i];
+        const float most = nf.w * pm.z;
         const float mag = sqrtf(f1 * f1 + f2 * f2);
-        if (mag > limit) {
-            const float scale = mag > 0.0f ? limit / mag : 0.0f;
+        if (mag > most) {
+            const float scale = mag > 0.0f ? most / mag : 0.0f;
             f1 *= scale;
             f2 *= scale;
         }
-        ti[i] = t1 * f1 + t2 * f2;
         pushMoving(a, b, x1, f1 - old1, moveA, moveB);
         pushMoving(a, b, x2, f2 - old2, moveA, moveB);
-    };
-    if (useBias) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            if (i < n) { row(i); }
-        }
-    } else {
-#pragma unroll
-        for (int i = 3; i >= 0; --i) {
-            if (i < n) { row(i); }
-        }
+        // The tangent masses stay; only the impulses are written.
+        if (S != kRowTile) { reinterpret_cast<float2*>(out + 2 * kRowTile)[1] = make_float2(pm.z, pm.w); }
+        out[3 * kRowTile] = f4(t1 * f1 + t2 * f2, 0.0f);
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if (i < n) {
-            const int at = kRowPoint + kRowPointWords * i;
-            float4* m = R + (at + 2) * S;
-            // The tangent masses stay; only the impulses are written.
-            reinterpret_cast<float2*>(m)[1] = make_float2(ni[i], mi[i]);
-            R[(at + 3) * S] = f4(ti[i], 0.0f);
+    if (moveA) { st.storeVW(ia, a); }
+    if (moveB) { st.storeVW(ib, b); }
+}
+
+// Runs f(words, record) on every contact of each color, a color at a time; slotAt gives the record slot of a
+// position. With rooms, the records are solved from the lane's room (mine) and a color's first ones are asked for
+// before the barrier that ends the color before it: contacts of a pass write only their own records, each in one
+// color.
+template <bool Rooms, class Slot, class F>
+__device__ __forceinline__ void forEachColorRecord(const Batch& B, const Group& g, const uint32_t* start, uint32_t colors,
+                                                   float4* mine, Slot slotAt, F f) {
+    auto ask = [&](uint32_t x, uint32_t end) {
+        if (Rooms && x < end) { roomLoad(mine, rowOf(B, slotAt(x))); }
+    };
+    if (colors > 0) { ask(start[0] + g.tid, start[1]); }
+    for (uint32_t k = 0; k < colors; ++k) {
+        const uint32_t end = start[k + 1];
+        for (uint32_t x = start[k] + g.tid; x < end; x += g.size) {
+            float4* R = rowOf(B, slotAt(x));
+            if constexpr (Rooms) { roomWait(); }
+            f(Rooms ? mine : R, R);
+            ask(x + g.size, end);
         }
+        if (k + 1 < colors) { ask(end + g.tid, start[k + 2]); }
+        g.sync();
     }
 }
 
@@ -2761,45 +2805,8 @@ static __device__ void flatPosition(const FlatStore& f, uint32_t i, const StepPa
     d.kept = b.kept;
 }
 
-// One contact's passes, for either store, with body indices counted from the store's first body (`base`: the
-// same first body). A laned contact runs from its record, by slot; a contact solved on its own from the contact
-// and its stored axes. A laned contact's bodies are stored only where they move, so a static body shared by a
-// color's contacts is never written concurrently; a contact solved on its own stores both, as the reference
-// does.
-template <class Store>
-__device__ __forceinline__ void warmRowAt(const Batch& B, const Store& st, uint32_t base, uint32_t limit,
-                                          uint32_t slot) {
-    const float4* R = rowOf(B, slot);
-    const float4 h = R[kRowHead * kRowTile];
-    const uint32_t ia = __float_as_uint(h.x) - base, ib = __float_as_uint(h.y) - base;
-    const int n = (int)__float_as_uint(h.z);
-#if defined(TF_DEVICE_CHECKS)
-    if (!TF_OK_INDEX(B, ia < limit && ib < limit && n >= 0 && n <= 4, 10, base, ia)) { return; }
-#endif
-    if (n == 0) { return; }
-    LanedBody a = st.loadLaned(ia), b = st.loadLaned(ib);
-    warmStartRow(R, a, b, n);
-    if (!anchored(a)) { st.storeVW(ia, a); }
-    if (!anchored(b)) { st.storeVW(ib, b); }
-}
-
-template <class Store>
-__device__ __forceinline__ void solveRowAt(const Batch& B, const StepParams& P, const Store& st, uint32_t base,
-                                           uint32_t limit, uint32_t slot, bool bias) {
-    float4* R = rowOf(B, slot);
-    const float4 h = R[kRowHead * kRowTile];
-    const uint32_t ia = __float_as_uint(h.x) - base, ib = __float_as_uint(h.y) - base;
-    const int n = (int)__float_as_uint(h.z);
-#if defined(TF_DEVICE_CHECKS)
-    if (!TF_OK_INDEX(B, ia < limit && ib < limit && n >= 0 && n <= 4, 12, base, ia)) { return; }
-#endif
-    if (n == 0) { return; }
-    LanedBody a = st.loadLaned(ia), b = st.loadLaned(ib);
-    solveRow(R, a, b, n, P, bias);
-    if (!anchored(a)) { st.storeVW(ia, a); }
-    if (!anchored(b)) { st.storeVW(ib, b); }
-}
-
+// The passes of a contact solved on its own, for either store, from the contact and its stored axes; both bodies are
+// stored, as the reference does.
 template <class Store>
 __device__ __forceinline__ void warmOne(const Batch& B, const WorldInfo& wi, const WorldCounts& wc, const Store& st,
                                         uint32_t ci) {
@@ -3010,12 +3017,19 @@ __device__ void runJoints(const Batch& B, const StepParams& P, const WorldInfo& 
     }
 }
 
+// Whether the batch's active contacts outweigh its bodies, two to one: solved with rooms then (kRoomWarps). The
+// lines measured lie at 7.4 contacts a body (impact walls) and 2.8 (the pyramid) on one side, 0.5 and less on the
+// other.
+__device__ __forceinline__ bool contactsOutweigh(const Batch& B) {
+    return *(volatile uint32_t*)(B.work + kSlotActive) >= 2 * B.totalBodies;
+}
+
 // Integrate velocities, warm start, biased solve, integrate positions, relax (src/world.cpp:1669-1680). The
 // world's solver state is staged in the group's shared slice when it has at most stageN bodies.
 // Joints is false for batches without joints: that instantiation carries no joint code, which would cost the
 // contact solve registers.
-template <bool Joints>
-__global__ void __launch_bounds__(kMaxBlock) k_substep(const __grid_constant__ Batch B, const __grid_constant__ StepParams P, const __grid_constant__ Split sp, int sub, int serial) {
+template <bool Joints, bool Rooms>
+__global__ void __launch_bounds__(Rooms ? kRoomWarps * 32 : kMaxBlock) k_substep(const __grid_constant__ Batch B, const __grid_constant__ StepParams P, const __grid_constant__ Split sp, int sub, int serial) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     if (stepAborted(B, serial)) { return; }
     if (sub > 0) {
@@ -3024,6 +3038,12 @@ __global__ void __launch_bounds__(kMaxBlock) k_substep(const __grid_constant__ B
         for (int l = 0; l <= kPairClasses; ++l) { items |= *(volatile uint32_t*)(B.work + kSlotFastItems + l); }
         if (items == 0) { return; }
     }
+    // The launches with rooms and without take turns by step: which of them steps the batch is decided when its
+    // contacts are known.
+    if (Rooms != contactsOutweigh(B)) { return; }
+    // The warps' rooms for records lie after the staging slices.
+    float4* room = reinterpret_cast<float4*>(s_raw + sp.smemBytes + (Rooms ? threadIdx.x >> 5 : 0u) * kRoomBytes) +
+                   (threadIdx.x & 31);
     forWorlds(B, kSlotSubstep + sub, sp, s_raw, [&](const Group& g, uint32_t w, unsigned char* sliceRaw, const StageSizes& ss) {
         float* slice = reinterpret_cast<float*>(sliceRaw);
         const uint32_t stageN = ss.bodies;
@@ -3057,6 +3077,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_substep(const __grid_constant__ B
         const uint32_t* icolored = B.impactColored + cf;
         const uint32_t* irest = B.impactRest + cf;
         const uint32_t* slotOf = B.slotOf + cf;
+        constexpr int kStride = Rooms ? 32 : kRowTile;
         bool refreshNext = false;
         for (int s = sub;; ++s) {
             for (uint32_t i = g.tid; i < nb; i += g.size) { st.integrateVelocityAt(i, P); }
@@ -3067,7 +3088,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_substep(const __grid_constant__ B
                     g.sync();
                 }
             }
-            forEachColorSlot(g, wc.colorStart, wc.colorCount, [&](uint32_t x) { warmRowAt(B, st, base, nb, cf + x); });
+            forEachColorRecord<Rooms>(B, g, wc.colorStart, wc.colorCount, room, [&](uint32_t x) { return cf + x; },
+                                      [&](float4* W, float4*) { warmRecord<kStride>(B, st, base, nb, W); });
             forEachLevel(g, rest, B.restLevel + cf, wc.restLevels, [&](uint32_t ci) { warmOne(B, wi, wc, st, ci); });
             for (int pass = 0; pass < 2; ++pass) {
                 const bool bias = pass == 0;
@@ -3079,10 +3101,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_substep(const __grid_constant__ B
                 }
                 // The active contacts, then the struck ones again (one call site: the solve is inlined once).
                 for (int struck = 0; struck < (wc.impactCount > 0 ? 2 : 1); ++struck) {
-                    forEachColorSlot(g, struck ? wc.impactColorStart : wc.colorStart,
-                                     struck ? wc.impactColorCount : wc.colorCount, [&](uint32_t x) {
-                                         solveRowAt(B, P, st, base, nb, struck ? slotOf[icolored[x]] : cf + x, bias);
-                                     });
+                    forEachColorRecord<Rooms>(
+                        B, g, struck ? wc.impactColorStart : wc.colorStart, struck ? wc.impactColorCount : wc.colorCount,
+                        room, [&](uint32_t x) { return struck ? slotOf[icolored[x]] : cf + x; },
+                        [&](float4* W, float4* R) { solveRecord<kStride>(B, P, st, base, nb, W, R, bias); });
                     forEachLevel(g, struck ? irest : rest, (struck ? B.impactRestLevel : B.restLevel) + cf,
                                  struck ? wc.impactRestLevels : wc.restLevels,
                                  [&](uint32_t ci) { solveOne(B, P, wi, wc, st, ci, bias); });
@@ -3304,7 +3326,7 @@ __global__ void __launch_bounds__(256, 2) k_substep_flat(const __grid_constant__
     };
     const uint32_t limit = nb;
     jointsPass(0);
-    colorsPass(B.flatColored, colorTotal, colors, [&](uint32_t slot) { warmRowAt(B, all, 0u, limit, slot); });
+    colorsPass(B.flatColored, colorTotal, colors, [&](uint32_t slot) { warmRecord<kRowTile>(B, all, 0u, limit, rowOf(B, slot)); });
     restPass(false, [&](const WorldInfo& wi, const WorldCounts& wc, const FlatStore& st, uint32_t ci) {
         warmOne(B, wi, wc, st, ci);
     });
@@ -3314,7 +3336,10 @@ __global__ void __launch_bounds__(256, 2) k_substep_flat(const __grid_constant__
         for (int struck = 0; struck < 2; ++struck) {
             colorsPass(struck ? B.flatImpact : B.flatColored, struck ? impactTotal : colorTotal,
                        struck ? impactColors : colors,
-                       [&](uint32_t slot) { solveRowAt(B, P, all, 0u, limit, slot, bias); });
+                       [&](uint32_t slot) {
+                           float4* R = rowOf(B, slot);
+                           solveRecord<kRowTile>(B, P, all, 0u, limit, R, R, bias);
+                       });
             restPass(struck != 0, [&](const WorldInfo& wi, const WorldCounts& wc, const FlatStore& st, uint32_t ci) {
                 solveOne(B, P, wi, wc, st, ci, bias);
             });

@@ -26,6 +26,8 @@ enum KernelId : int {
     kKPrepareBig,
     kKSubstep,
     kKSubstepJoints,
+    kKSubstepRooms,
+    kKSubstepRoomsJoints,
     kKFinish,
     kKFinishJoints,
     kKFinishBig,
