@@ -8,7 +8,7 @@
 
 namespace tfb {
 
-// A body of a big world as the sweep reads it, stored in bucket order: its pair-test record, where its
+// A body of a big world as the sweep reads it, stored in cell order: its pair-test record, where its
 // interval along x starts, and which body it is.
 struct SweepRec {
     Vec3 lo, hi;
@@ -88,6 +88,9 @@ struct Batch {
     // Joints and joined body pairs, per world from jointFirst.
     DJoint* joints;
     const uint64_t* joined;
+    // Per world from jointFirst: its joints (indices in the world) level by level, and each level's end.
+    const uint32_t* jointOrder;
+    const uint32_t* jointLevel;
     // The step's events: contact events from 2 * contactFirst (room for the pairs the narrowphase dropped
     // and for the end-of-step report), hits from contactFirst.
     TouchEvent* touchEvents;
@@ -107,16 +110,14 @@ struct Batch {
     uint32_t* rowCount;    // per shape, the sort's counts within one long row
 
     // Broadphase of worlds of more than kSweepBodies bodies: per body its interval along x (sweepLo, sweepHi)
-    // and, from bodyFirst, the bodies bucketed by the interval's start (sweepOrder); per world, from
-    // bodyFirst + world, the buckets' starts (sweepStart). bigWorlds lists those worlds, bigBodyStart the
-    // running total of their bodies.
+    // and, from bodyFirst, the bodies in cell order (sweepOrder; then the wide ones); per world, from bodyFirst +
+    // world, the cells' starts (sweepStart). bigWorlds lists those worlds.
     float* sweepLo;
     float* sweepHi;
     uint32_t* sweepOrder;
-    struct SweepRec* sweepRecs;  // per body, from bodyFirst, in bucket order: what the pair test reads
+    struct SweepRec* sweepRecs;  // per body, from bodyFirst, in cell order: what the pair test reads
     uint32_t* sweepStart;
     const uint32_t* bigWorlds;
-    const uint32_t* bigBodyStart;
     uint32_t nBigWorlds;
 
     // Continuous collision: per shape, its bounds over the whole step and (from shapeFirst) the world's fast

@@ -183,6 +183,7 @@ public:
     static constexpr size_t kSmallBatchCandidates = 8192;
     DevArray<DJoint> dJoints;
     DevArray<uint64_t> dJoined;
+    DevArray<uint32_t> dJointOrder, dJointLevel;
     DevArray<TouchEvent> dTouchEvents;
     DevArray<HitRecord> dHitEvents;
     DevArray<uint32_t> dAbort;
@@ -236,10 +237,10 @@ public:
     DevArray<uint32_t> dWork, dRowScratch, dRowLong, dRowCount;
     DevArray<Vec3> dSweptLo, dSweptHi;
     DevArray<float> dSweepLo, dSweepHi;
-    DevArray<uint32_t> dSweepOrder, dSweepStart, dBigWorlds, dBigBodyStart;
+    DevArray<uint32_t> dSweepOrder, dSweepStart, dBigWorlds;
     DevArray<SweepRec> dSweepRecs;
-    std::vector<uint32_t> bigWorlds, bigBodyStart;  // worlds of more than kSweepBodies bodies
-    uint32_t bigCtas = 0;                           // CTAs of the cluster that steps each of them; 0: one CTA does
+    std::vector<uint32_t> bigWorlds;  // worlds of more than kSweepBodies bodies
+    uint32_t bigCtas = 0;             // CTAs of the cluster that steps each of them; 0: one CTA does
     DevArray<uint32_t> dSweepList, dHitParent;
     DevArray<unsigned long long> dHitKey, dGroupKey;
     DevArray<uint2> dCandItems, dContactItems;
@@ -1424,6 +1425,33 @@ public:
         return TF_OK;
     }
 
+    // A world's joints level by level: each joint one level past the last earlier joint at either of its dynamic
+    // bodies, kinds together within a level. A body's type only changes with a new layout; whether it is awake, and
+    // whether a joint holds, does not matter (a joint that does nothing at a body may as well come in its turn).
+    static void levelJoints(const HostWorld& W, uint32_t* order, uint32_t* levelEnd, uint32_t& levels) {
+        const size_t n = W.joints.size();
+        std::vector<uint32_t> last(W.bodies.size(), 0u), level(n, 0u);
+        levels = 0;
+        for (size_t k = 0; k < n; ++k) {
+            const DJoint& j = W.joints[k].d;
+            if (!j.alive) { continue; }
+            for (const uint32_t b : { j.bodyA, j.bodyB }) {
+                if (b < W.bodies.size() && W.bodies[b].d.type == kDynamic) { level[k] = std::max(level[k], last[b]); }
+            }
+            for (const uint32_t b : { j.bodyA, j.bodyB }) {
+                if (b < W.bodies.size() && W.bodies[b].d.type == kDynamic) { last[b] = level[k] + 1; }
+            }
+        }
+        for (size_t k = 0; k < n; ++k) {
+            order[k] = (uint32_t)k;
+            levels = std::max(levels, level[k] + 1);
+        }
+        std::stable_sort(order, order + n, [&](uint32_t a, uint32_t b) {
+            return level[a] != level[b] ? level[a] < level[b] : W.joints[a].d.type < W.joints[b].d.type;
+        });
+        for (size_t k = 0; k < n; ++k) { levelEnd[level[order[k]]] = (uint32_t)k + 1; }
+    }
+
     int layout() {
         ++layoutGen;
         bodyStepsBase = bodyStepsTotal;
@@ -1490,6 +1518,7 @@ public:
         std::vector<uint32_t> shapeList(ns), planeList(std::max<size_t>(nplanes, 1));
         std::vector<DJoint> joints(std::max<size_t>(njoints, 1));
         std::vector<uint64_t> joined(std::max<size_t>(njoints, 1));
+        std::vector<uint32_t> jointOrder(std::max<size_t>(njoints, 1)), jointLevel(std::max<size_t>(njoints, 1));
         // Contacts carried over from the device: packed, with one (slot, first, count) run per world.
         std::vector<DContact> packed;
         std::vector<size_t> runSlot, runFirst, runCount;
@@ -1553,6 +1582,7 @@ public:
                 j.bodyB += wi.bodyFirst;
                 joints[wi.jointFirst + k] = j;
             }
+            levelJoints(W, jointOrder.data() + wi.jointFirst, jointLevel.data() + wi.jointFirst, info[w].jointLevels);
             std::sort(keys.begin(), keys.end());
             info[w].joinedCount = (uint32_t)keys.size();
             for (size_t k = 0; k < keys.size(); ++k) { joined[wi.jointFirst + k] = keys[k]; }
@@ -1673,6 +1703,8 @@ public:
         TF_ALLOC(dMergeIdxB, ncon);
         TF_ALLOC(dJoints, joints.size());
         TF_ALLOC(dJoined, joined.size());
+        TF_ALLOC(dJointOrder, jointOrder.size());
+        TF_ALLOC(dJointLevel, jointLevel.size());
         TF_ALLOC(dTouchEvents, 2 * ncon);
         TF_ALLOC(dHitEvents, ncon);
         TF_ALLOC(dWork, kSlotCount);
@@ -1682,12 +1714,8 @@ public:
         TF_ALLOC(dRowLong, ns);
         TF_ALLOC(dRowCount, ns);
         bigWorlds.clear();
-        bigBodyStart.assign(1, 0u);
         for (uint32_t w : order) {
-            if (info[w].bodyCount > kSweepBodies) {
-                bigWorlds.push_back(w);
-                bigBodyStart.push_back(bigBodyStart.back() + info[w].bodyCount);
-            }
+            if (info[w].bodyCount > kSweepBodies) { bigWorlds.push_back(w); }
         }
         TF_ALLOC(dSweepLo, nb);
         TF_ALLOC(dSweepHi, nb);
@@ -1695,7 +1723,6 @@ public:
         TF_ALLOC(dSweepRecs, nb);
         TF_ALLOC(dSweepStart, nb + nw);
         TF_ALLOC(dBigWorlds, bigWorlds.size());
-        TF_ALLOC(dBigBodyStart, bigBodyStart.size());
         TF_ALLOC(dSweptLo, ns);
         TF_ALLOC(dSweptHi, ns);
         TF_ALLOC(dSweepList, ns);
@@ -1722,6 +1749,8 @@ public:
         if ((rc = up(dPlaneList.ptr, planeList.data(), planeList.size() * sizeof(uint32_t))) != TF_OK) { return rc; }
         if ((rc = up(dJoints.ptr, joints.data(), joints.size() * sizeof(DJoint))) != TF_OK) { return rc; }
         if ((rc = up(dJoined.ptr, joined.data(), joined.size() * sizeof(uint64_t))) != TF_OK) { return rc; }
+        if ((rc = up(dJointOrder.ptr, jointOrder.data(), jointOrder.size() * sizeof(uint32_t))) != TF_OK) { return rc; }
+        if ((rc = up(dJointLevel.ptr, jointLevel.data(), jointLevel.size() * sizeof(uint32_t))) != TF_OK) { return rc; }
         if ((rc = up(dPolys.ptr, polys.data(), polys.size() * sizeof(DPoly))) != TF_OK) { return rc; }
         if ((rc = up(dVerts.ptr, verts.data(), verts.size() * sizeof(Vec3))) != TF_OK) { return rc; }
         if ((rc = up(dNormals.ptr, normals.data(), normals.size() * sizeof(Vec3))) != TF_OK) { return rc; }
@@ -1731,7 +1760,6 @@ public:
         if ((rc = up(dOffsets.ptr, offsets.data(), offsets.size() * sizeof(float))) != TF_OK) { return rc; }
         if ((rc = up(dEdges.ptr, edges.data(), edges.size() * sizeof(DEdge))) != TF_OK) { return rc; }
         if ((rc = up(dBigWorlds.ptr, bigWorlds.data(), bigWorlds.size() * sizeof(uint32_t))) != TF_OK) { return rc; }
-        if ((rc = up(dBigBodyStart.ptr, bigBodyStart.data(), bigBodyStart.size() * sizeof(uint32_t))) != TF_OK) { return rc; }
         if ((rc = up(dMeshes.ptr, meshRecs.data(), meshRecs.size() * sizeof(DMesh))) != TF_OK) { return rc; }
         if ((rc = up(dMeshVerts.ptr, meshVerts.data(), meshVerts.size() * sizeof(Vec3))) != TF_OK) { return rc; }
         if ((rc = up(dMeshIndices.ptr, meshIndices.data(), meshIndices.size() * sizeof(uint32_t))) != TF_OK) { return rc; }
@@ -1872,6 +1900,8 @@ public:
         B.mergeIdxB = dMergeIdxB.ptr;
         B.joints = dJoints.ptr;
         B.joined = dJoined.ptr;
+        B.jointOrder = dJointOrder.ptr;
+        B.jointLevel = dJointLevel.ptr;
         B.touchEvents = dTouchEvents.ptr;
         B.hitEvents = dHitEvents.ptr;
         B.work = dWork.ptr;
@@ -1888,7 +1918,6 @@ public:
         B.sweepRecs = dSweepRecs.ptr;
         B.sweepStart = dSweepStart.ptr;
         B.bigWorlds = dBigWorlds.ptr;
-        B.bigBodyStart = dBigBodyStart.ptr;
         B.nBigWorlds = (uint32_t)bigWorlds.size();
         B.sweptLo = dSweptLo.ptr;
         B.sweptHi = dSweptHi.ptr;

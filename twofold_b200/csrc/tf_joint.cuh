@@ -1,14 +1,20 @@
 // Joints in the substep loop (src/joint.cpp): warm start, the biased and relaxing solves, the reaction each
 // relaxing solve adds, the position-level settle after the step and the speed-limit scaling of warm starts.
 // Every function restates its reference counterpart's arithmetic in order; the world end of a joint is a
-// static body at the origin. Joints of a world run one after another in index order on one thread, before
-// the world's contacts in each pass, as the reference solves them.
+// static body at the origin. The joints at a body run one after another in index order, before the world's
+// contacts in each pass, as the reference solves them.
 #pragma once
 
 #include "tf_continuous.cuh"
 #include "tf_solver.cuh"
 
 namespace tfb {
+
+#if defined(__CUDACC__)
+#define TF_HD_OUTLINE __host__ __device__ __noinline__ static
+#else
+#define TF_HD_OUTLINE static
+#endif
 
 constexpr float kJointPi = 3.14159265358979f;
 constexpr int kSettleIterations = 2;  // src/world.cpp:16
@@ -70,46 +76,59 @@ TF_HD float traceOf(const Mat3& m) { return m.r[0].x + m.r[1].y + m.r[2].z; }
 // The inverse of m on the directions it acts in (src/joint.cpp:21-70): the plain inverse when m is well
 // conditioned, else cyclic Jacobi rotations of its symmetric part and the reciprocals of its eigenvalues above
 // a relative floor.
-TF_HD Mat3 pseudoInverse(const Mat3& m) {
+// One Jacobi rotation of rows and columns p and q, known to the compiler so that the matrices stay in registers.
+template <int p, int q>
+TF_HD void jacobiTurn(float (&a)[3][3], float (&v)[3][3]) {
+    if (a[p][q] == 0.0f) { return; }
+    const float theta = (a[q][q] - a[p][p]) / (2.0f * a[p][q]);
+    const float t = (theta >= 0.0f ? 1.0f : -1.0f) / (fabsf(theta) + sqrtf(theta * theta + 1.0f));
+    const float c = 1.0f / sqrtf(t * t + 1.0f), s = t * c;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float kp = a[k][p], kq = a[k][q];
+        a[k][p] = c * kp - s * kq;
+        a[k][q] = s * kp + c * kq;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float pk = a[p][k], qk = a[q][k];
+        a[p][k] = c * pk - s * qk;
+        a[q][k] = s * pk + c * qk;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float kp = v[k][p], kq = v[k][q];
+        v[k][p] = c * kp - s * kq;
+        v[k][q] = s * kp + c * kq;
+    }
+}
+
+// Out of line: the joints of a pass reach it from a dozen places, and inlined its copies overran the instruction
+// cache.
+TF_HD_OUTLINE Mat3 pseudoInverse(const Mat3& m) {
     const float tr = traceOf(m);
     if (tr <= 0.0f) { return mzero(); }
     const float third = tr / 3.0f;
     if (dot(m.r[0], cross(m.r[1], m.r[2])) > 1e-3f * third * third * third) { return inverse(m); }
     float a[3][3], v[3][3];
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
+#pragma unroll
         for (int k = 0; k < 3; ++k) {
             a[i][k] = 0.5f * (comp(m.r[i], k) + comp(m.r[k], i));
             v[i][k] = i == k ? 1.0f : 0.0f;
         }
     }
+#pragma unroll 1
     for (int sweep = 0; sweep < 8; ++sweep) {
         if (a[0][1] * a[0][1] + a[0][2] * a[0][2] + a[1][2] * a[1][2] <= 1e-14f * tr * tr) { break; }
-        for (int p = 0; p < 2; ++p) {
-            for (int q = p + 1; q < 3; ++q) {
-                if (a[p][q] == 0.0f) { continue; }
-                const float theta = (a[q][q] - a[p][p]) / (2.0f * a[p][q]);
-                const float t = (theta >= 0.0f ? 1.0f : -1.0f) / (fabsf(theta) + sqrtf(theta * theta + 1.0f));
-                const float c = 1.0f / sqrtf(t * t + 1.0f), s = t * c;
-                for (int k = 0; k < 3; ++k) {
-                    const float kp = a[k][p], kq = a[k][q];
-                    a[k][p] = c * kp - s * kq;
-                    a[k][q] = s * kp + c * kq;
-                }
-                for (int k = 0; k < 3; ++k) {
-                    const float pk = a[p][k], qk = a[q][k];
-                    a[p][k] = c * pk - s * qk;
-                    a[q][k] = s * pk + c * qk;
-                }
-                for (int k = 0; k < 3; ++k) {
-                    const float kp = v[k][p], kq = v[k][q];
-                    v[k][p] = c * kp - s * kq;
-                    v[k][q] = s * kp + c * kq;
-                }
-            }
-        }
+        jacobiTurn<0, 1>(a, v);
+        jacobiTurn<0, 2>(a, v);
+        jacobiTurn<1, 2>(a, v);
     }
     const float top = maxf(a[0][0], maxf(a[1][1], a[2][2]));
     Mat3 out = mzero();
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
         if (a[i][i] <= 1e-6f * top) { continue; }
         const Vec3 e{ v[0][i], v[1][i], v[2][i] };

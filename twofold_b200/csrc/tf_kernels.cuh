@@ -370,7 +370,7 @@ __device__ __forceinline__ uint64_t pairKey(uint32_t a, uint32_t b) {
 }
 
 __device__ __forceinline__ void emitCandidate(const Batch& B, const WorldInfo& wi, uint32_t* count, uint64_t key) {
-    const uint32_t pos = atomicAdd(count, 1u);
+    const uint32_t pos = takePlace(count, 0u);
     if (pos < wi.candCap) { B.cand[wi.candFirst + pos] = key; }
 }
 
@@ -443,27 +443,65 @@ static __device__ void wakeStack(const Batch& B, const WorldInfo& wi, const DCon
 }
 
 // At the start of a step a joint pulls its sleeping dynamic end awake when the other end moves
-// (src/world.cpp:1578-1585); runs on one thread, over the last step's contacts.
-static __device__ void wakeJointPulled(const Batch& B, const WorldInfo& wi, const WorldCounts& wc) {
-    uint32_t* stack = B.unionParent + wi.bodyFirst;
-    uint32_t top = 0;
+// (src/world.cpp:1578-1585), over the last step's contacts. The group looks for such a joint; one thread wakes.
+// flag: a word of the group's shared memory (clusters).
+template <class G>
+static __device__ void wakeJointPulled(const Batch& B, const G& g, const WorldInfo& wi, const WorldCounts& wc, uint32_t* flag) {
     const DJoint* js = B.joints + wi.jointFirst;
-    auto moving = [&](uint32_t g) { return g != kWorldEnd && movingAwake(B.bodies[g]); };
-    auto pull = [&](uint32_t g) {
-        if (g == kWorldEnd) { return; }
-        const DBody& b = B.bodies[g];
-        if (b.alive && b.type == kDynamic && !b.awake && !B.wakeMark[g] && top < wi.bodyCount) {
-            B.wakeMark[g] = 1;
-            stack[top++] = g;
-        }
+    auto moving = [&](uint32_t gb) { return gb != kWorldEnd && movingAwake(B.bodies[gb]); };
+    auto pulled = [&](uint32_t gb) {
+        if (gb == kWorldEnd) { return false; }
+        const DBody& b = B.bodies[gb];
+        return b.alive && b.type == kDynamic && !b.awake && !B.wakeMark[gb];
     };
-    for (uint32_t x = 0; x < wi.jointCount; ++x) {
+    if constexpr (G::kCluster) {
+        if (g.tid == 0) { *flag = 0; }
+        g.sync();
+    }
+    bool found = false;
+    for (uint32_t x = g.tid; x < wi.jointCount; x += g.size) {
         const DJoint& j = js[x];
         if (!j.alive || j.broken) { continue; }
-        if (moving(j.bodyB)) { pull(j.bodyA); }
-        if (moving(j.bodyA)) { pull(j.bodyB); }
+        found = found || (moving(j.bodyB) && pulled(j.bodyA)) || (moving(j.bodyA) && pulled(j.bodyB));
     }
-    wakeStack(B, wi, B.previous + wi.contactFirst, min(wc.contactCount, wi.contactCap), stack, top);
+    if (!g.any(found, flag)) { return; }
+    if (g.tid == 0) {
+        uint32_t* stack = B.unionParent + wi.bodyFirst;
+        uint32_t top = 0;
+        auto pull = [&](uint32_t gb) {
+            if (pulled(gb) && top < wi.bodyCount) {
+                B.wakeMark[gb] = 1;
+                stack[top++] = gb;
+            }
+        };
+        for (uint32_t x = 0; x < wi.jointCount; ++x) {
+            const DJoint& j = js[x];
+            if (!j.alive || j.broken) { continue; }
+            if (moving(j.bodyB)) { pull(j.bodyA); }
+            if (moving(j.bodyA)) { pull(j.bodyB); }
+        }
+        wakeStack(B, wi, B.previous + wi.contactFirst, min(wc.contactCount, wi.contactCap), stack, top);
+    }
+    g.sync();
+}
+
+// Calls f(joint index) for a world's joints, level by level (B.jointOrder): joints of a level share no dynamic body,
+// and every dynamic body meets its joints in index order, which is what the reference's pass in index order gives it;
+// other ends take nothing from a joint. A warp takes the joints of one kind among 32 of a level, which keeps it on one
+// code path. Bounded by the longest chain of joint solves: 256 worlds of 22 joints of every kind, chains of 6 at most,
+// take 601 us of substeps and 119 of end of step, against 868 and 202 with a world's joints on one thread.
+template <class G, class F>
+__device__ __forceinline__ void forEachJoint(const Batch& B, const G& g, const WorldInfo& wi, F&& f) {
+    uint32_t begin = 0;
+    for (uint32_t l = 0; l < wi.jointLevels; ++l) {
+        const uint32_t end = B.jointLevel[wi.jointFirst + l];
+        for (uint32_t i = begin + g.lane, k = 0; i < end; i += 32, ++k) {
+            const uint32_t x = B.jointOrder[wi.jointFirst + i];
+            if ((k + B.joints[wi.jointFirst + x].type) % g.warps == g.warp) { f(x); }
+        }
+        g.sync();
+        begin = end;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -564,81 +602,154 @@ __device__ __forceinline__ float fromOrderedKey(uint32_t k) {
 // millionth of the coordinate.
 __device__ __forceinline__ float sweepSlack(float x) { return 1e-3f + 1e-6f * fabsf(x); }
 
-// Buckets along x: a quarter as many as bodies, evenly over the range the intervals cover.
+// A big world's bodies lie in a grid of cells by where their intervals along x and along a second axis (the longer of
+// y and z) start, at most a cell a body, x-major: the cells of one x column from a low to a high second coordinate
+// are one contiguous run of bodies. A body whose interval covers an eighth of the second axis or more is wide: it can
+// start far from what it meets, so it stands in a list of its own as well. Where more than a sixteenth of the bodies
+// are wide (a single layer of bodies), the grid has x columns only and no body counts as wide. (Along x alone, a
+// body of the terrain's 32 x 32 columns met the 1,500 bodies of its x range: 65 million tests, 1.9 ms.)
+constexpr uint32_t kBodyWide = 8u;
+
 struct SweepGrid {
-    float lo, scale;
-    uint32_t buckets;
+    float lo[2], scale[2];
+    uint32_t cells[2];
+    int axis;     // the second axis
+    float width;  // no body that is not wide is wider along it
 };
 
 __device__ __forceinline__ SweepGrid sweepGrid(const WorldInfo& wi, const WorldCounts& wc) {
     SweepGrid s;
-    s.buckets = wi.bodyCount / 4 + 1;
-    s.lo = fromOrderedKey(wc.sweepMinKey);
-    const float hi = fromOrderedKey(wc.sweepMaxKey);
-    s.scale = hi > s.lo ? (float)s.buckets / (hi - s.lo) : 0.0f;
+    float lo[3], hi[3];
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = fromOrderedKey(wc.sweepMinKey[k]);
+        hi[k] = fromOrderedKey(wc.sweepMaxKey[k]);
+    }
+    s.axis = hi[2] - lo[2] > hi[1] - lo[1] ? 2 : 1;
+    const bool flat = wc.sweepWide > wi.bodyCount / 16;
+    const uint32_t side = (uint32_t)sqrtf((float)(wi.bodyCount / 4 + 1));
+    s.cells[0] = flat ? wi.bodyCount / 4 + 1 : side;
+    s.cells[1] = flat ? 1u : side;
+    const float a = lo[0], b = hi[0], c = s.axis == 2 ? lo[2] : lo[1], d = s.axis == 2 ? hi[2] : hi[1];
+    s.lo[0] = a;
+    s.lo[1] = c;
+    s.scale[0] = b > a ? (float)s.cells[0] / (b - a) : 0.0f;
+    s.scale[1] = d > c ? (float)s.cells[1] / (d - c) : 0.0f;
+    s.width = __uint_as_float(wc.sweepWidth);
     return s;
 }
 
-__device__ __forceinline__ uint32_t sweepBucket(const SweepGrid& s, float x) {
-    const float f = (x - s.lo) * s.scale;
+__device__ __forceinline__ uint32_t sweepCell(const SweepGrid& s, int k, float x) {
+    const float f = (x - s.lo[k]) * s.scale[k];
     if (!(f > 0.0f)) { return 0u; }
-    return f >= (float)(s.buckets - 1) ? s.buckets - 1 : (uint32_t)f;
+    return f >= (float)(s.cells[k] - 1) ? s.cells[k] - 1 : (uint32_t)f;
 }
 
-// The first half of a big world's broadphase, after the growth: each live body's interval along x, their
-// range, and the bodies counted into buckets by where their intervals start. Bucket b then holds
-// sweepOrder[start[b - 1] .. start[b]), start[-1] being 0.
+// A body's grown interval along an axis, widened so that rounding never loses a pair.
+__device__ __forceinline__ void sweepInterval(float lo, float hi, float grow, float& from, float& to) {
+    from = lo - grow - sweepSlack(lo);
+    to = hi + grow + sweepSlack(hi);
+}
+
+// The first half of a big world's broadphase, after the growth: each live body's interval along x, the ranges of the
+// intervals along every axis, and the bodies counted into cells. Cell c then holds the records from start[c - 1] to
+// start[c], start[-1] being 0.
 template <class G>
 static __device__ void prepareSweep(const Batch& B, const G& g, const WorldInfo& wi, WorldCounts& wc, uint32_t w) {
     const uint32_t n = wi.bodyCount;
     if (g.tid == 0) {
-        wc.sweepMinKey = 0xffffffffu;
-        wc.sweepMaxKey = 0u;
+        for (int k = 0; k < 3; ++k) {
+            wc.sweepMinKey[k] = 0xffffffffu;
+            wc.sweepMaxKey[k] = 0u;
+        }
         wc.candRaw = 0;
+        wc.sweepWide = 0;
+        wc.sweepWidth = 0;
     }
     g.sync();
-    uint32_t least = 0xffffffffu, most = 0u;
+    uint32_t least[3] = { 0xffffffffu, 0xffffffffu, 0xffffffffu }, most[3] = { 0u, 0u, 0u };
     for (uint32_t i = g.tid; i < n; i += g.size) {
         const uint32_t gb = wi.bodyFirst + i;
         const DBody& b = B.bodies[gb];
         float lo = FLT_MAX, hi = -FLT_MAX;
         if (b.alive && b.hasBounds) {
             const float gr = B.grow[gb];
-            lo = b.lo.x - gr - sweepSlack(b.lo.x);
-            hi = b.hi.x + gr + sweepSlack(b.hi.x);
-            least = min(least, orderedKey(lo));
-            most = max(most, orderedKey(hi));
+            const Vec3 bl = b.lo, bh = b.hi;
+            for (int k = 2; k >= 0; --k) {
+                sweepInterval(comp(bl, k), comp(bh, k), gr, lo, hi);
+                least[k] = min(least[k], orderedKey(lo));
+                most[k] = max(most[k], orderedKey(hi));
+            }
         }
         B.sweepLo[gb] = lo;
         B.sweepHi[gb] = hi;
     }
-    least = __reduce_min_sync(0xffffffffu, least);
-    most = __reduce_max_sync(0xffffffffu, most);
-    if (g.lane == 0) {
-        atomicMin(&wc.sweepMinKey, least);
-        atomicMax(&wc.sweepMaxKey, most);
+    for (int k = 0; k < 3; ++k) {
+        least[k] = __reduce_min_sync(0xffffffffu, least[k]);
+        most[k] = __reduce_max_sync(0xffffffffu, most[k]);
+        if (g.lane == 0) {
+            atomicMin(&wc.sweepMinKey[k], least[k]);
+            atomicMax(&wc.sweepMaxKey[k], most[k]);
+        }
     }
     g.sync();
-    const SweepGrid grid = sweepGrid(wi, wc);
-    uint32_t* start = B.sweepStart + wi.bodyFirst + w;
-    for (uint32_t k = g.tid; k < grid.buckets; k += g.size) { start[k] = 0; }
-    g.sync();
-    for (uint32_t i = g.tid; i < n; i += g.size) { atomicAdd(&start[sweepBucket(grid, B.sweepLo[wi.bodyFirst + i])], 1u); }
-    g.sync();
-    groupScanWords(g, start, grid.buckets);
-    // Scattering advances each bucket's start to its end.
+    SweepGrid grid = sweepGrid(wi, wc);
+    auto second = [&](uint32_t i, float& lo, float& hi) {
+        const uint32_t gb = wi.bodyFirst + i;
+        const DBody& b = B.bodies[gb];
+        lo = FLT_MAX, hi = -FLT_MAX;
+        if (!b.alive || !b.hasBounds) { return; }
+        const Vec3 bl = b.lo, bh = b.hi;
+        sweepInterval(grid.axis == 2 ? bl.z : bl.y, grid.axis == 2 ? bh.z : bh.y, B.grow[gb], lo, hi);
+    };
+    const float range = (float)grid.cells[1] / grid.scale[1];
+    auto wideAt = [&](float lo, float hi) { return !((hi - lo) * 8.0f < range); };
+    uint32_t wide = 0, width = 0;
     for (uint32_t i = g.tid; i < n; i += g.size) {
-        const uint32_t k = sweepBucket(grid, B.sweepLo[wi.bodyFirst + i]);
-        B.sweepOrder[wi.bodyFirst + atomicAdd(&start[k], 1u)] = i;
+        float lo, hi;
+        second(i, lo, hi);
+        if (!(hi >= lo)) { continue; }
+        if (wideAt(lo, hi)) {
+            ++wide;
+        } else {
+            width = max(width, __float_as_uint(hi - lo));
+        }
+    }
+    wide = __reduce_add_sync(0xffffffffu, wide);
+    width = __reduce_max_sync(0xffffffffu, width);
+    if (g.lane == 0) {
+        atomicAdd(&wc.sweepWide, wide);
+        atomicMax(&wc.sweepWidth, width);
     }
     g.sync();
-    // The records in bucket order, so a scan over neighbouring buckets reads one contiguous run.
+    grid = sweepGrid(wi, wc);
+    const uint32_t cells = grid.cells[0] * grid.cells[1];
+    uint32_t* start = B.sweepStart + wi.bodyFirst + w;
+    auto cellOf = [&](uint32_t i) {
+        float lo, hi;
+        second(i, lo, hi);
+        return sweepCell(grid, 0, B.sweepLo[wi.bodyFirst + i]) * grid.cells[1] + sweepCell(grid, 1, lo);
+    };
+    for (uint32_t k = g.tid; k < cells; k += g.size) { start[k] = 0; }
+    g.sync();
+    for (uint32_t i = g.tid; i < n; i += g.size) { atomicAdd(&start[cellOf(i)], 1u); }
+    g.sync();
+    groupScanWords(g, start, cells);
+    // Scattering advances each cell's start to its end.
+    for (uint32_t i = g.tid; i < n; i += g.size) { B.sweepOrder[wi.bodyFirst + atomicAdd(&start[cellOf(i)], 1u)] = i; }
+    g.sync();
+    // The records in cell order, so a scan over neighbouring cells reads one contiguous run.
     for (uint32_t q = g.tid; q < n; q += g.size) {
         const uint32_t i = B.sweepOrder[wi.bodyFirst + q];
-        const PairBody p = pairBodyOf(B, wi.bodyFirst + i);
+        PairBody p = pairBodyOf(B, wi.bodyFirst + i);
+        float lo, hi;
+        second(i, lo, hi);
+        if (grid.cells[1] > 1 && hi >= lo && wideAt(lo, hi)) { p.flags |= kBodyWide; }
         B.sweepRecs[wi.bodyFirst + q] = SweepRec{ p.lo, p.hi, p.grow, p.flags, B.sweepLo[wi.bodyFirst + i], i };
     }
     g.sync();
+    // The wide bodies' records, by position; the order has served.
+    groupCompact(g, n, [&](uint32_t q) { return (B.sweepRecs[wi.bodyFirst + q].flags & kBodyWide) != 0; },
+                 [&](uint32_t q, uint32_t pos) { B.sweepOrder[wi.bodyFirst + pos] = q; });
 }
 
 // Sorts the world's count keys (minShape << 32 | maxShape, at B.cand) ascending and removes repeats: a
@@ -733,14 +844,12 @@ __device__ __forceinline__ float growthOf(const DBody& b, const StepParams& P) {
 // The first half of the big worlds' broadphase, a cluster a world.
 template <int Unused = 0>
 __global__ void __launch_bounds__(kMaxBlock) k_broad_big(const __grid_constant__ Batch B, const __grid_constant__ StepParams P, int serial) {
+    __shared__ uint32_t s_pulled;
     if (stepAborted<true>(B, serial)) { return; }
     forBigWorlds(B, [&](const GroupOf<true>& g, uint32_t w, unsigned char*, const StageSizes&) {
         const WorldInfo wi = B.info[w];
         WorldCounts& wc = B.counts[w];
-        if (wi.jointCount > 0) {
-            if (g.tid == 0) { wakeJointPulled(B, wi, wc); }
-            g.sync();
-        }
+        if (wi.jointCount > 0) { wakeJointPulled(B, g, wi, wc, g.shared(&s_pulled)); }
         for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
             B.grow[wi.bodyFirst + i] = growthOf(B.bodies[wi.bodyFirst + i], P);
         }
@@ -762,10 +871,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_broadphase(const __grid_constant_
         WorldCounts& wc = B.counts[w];
         const uint32_t n = wi.bodyCount;
         const bool useStage = n <= stageN;
-        if (wi.jointCount > 0) {
-            if (g.tid == 0) { wakeJointPulled(B, wi, wc); }
-            g.sync();
-        }
+        if (wi.jointCount > 0) { wakeJointPulled(B, g, wi, wc, nullptr); }
         if (g.tid == 0) { s_count[g.id] = 0; }
         for (uint32_t i = g.tid; i < n; i += g.size) {
             const DBody& b = B.bodies[wi.bodyFirst + i];
@@ -857,44 +963,74 @@ static __device__ void finishCandidates(const Batch& B, const G& g, const WorldI
     }
 }
 
-// The pair half of a big world's broadphase: each body takes the bodies whose intervals along x start
-// within its own interval (the one starting first takes a pair, so each pair is taken once) and applies the
-// same pair test as the small worlds, in the pair's lower-body-first order. A warp per body, its lanes
-// across the contiguous run of records in the buckets its interval covers, over every big world.
+// The pair half of a big world's broadphase: each body takes the bodies whose intervals along x start within its own
+// (the one starting first takes a pair, so each pair is taken once) among the wide ones and those of the cells whose
+// bodies can reach it along the second axis, and applies the same pair test as the small worlds, in the pair's
+// lower-body-first order. A warp per body, its lanes across the contiguous run of records of each x column, over
+// every big world; a wide body's run is the whole of its x range, a warp a part of it (kSweepPart).
+constexpr uint32_t kSweepPart = 1024;  // records of a wide body's run a warp takes
+
 template <int Unused = 0>
 __global__ void __launch_bounds__(256) k_broad_pairs(const __grid_constant__ Batch B, int serial) {
     if (stepAborted(B, serial)) { return; }
-    const uint32_t total = B.bigBodyStart[B.nBigWorlds];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; item < total; item += warps) {
-        uint32_t k = 0;
-        while (k + 1 < B.nBigWorlds && B.bigBodyStart[k + 1] <= item) { ++k; }
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    for (uint32_t k = 0; k < B.nBigWorlds; ++k) {
         const uint32_t w = B.bigWorlds[k];
         const WorldInfo wi = B.info[w];
         WorldCounts& wc = B.counts[w];
+        const uint32_t n = wi.bodyCount, parts = (n + kSweepPart - 1) / kSweepPart;
         const SweepRec* recs = B.sweepRecs + wi.bodyFirst;
         const uint32_t* start = B.sweepStart + wi.bodyFirst + w;
-        const SweepRec ri = recs[item - B.bigBodyStart[k]];
-        if (!(ri.flags & kBodyLive)) { continue; }
-        const float lo = ri.start, hi = B.sweepHi[wi.bodyFirst + ri.body];
+        const uint32_t* wides = B.sweepOrder + wi.bodyFirst;
         const SweepGrid grid = sweepGrid(wi, wc);
-        const uint32_t b0 = sweepBucket(grid, lo), b1 = sweepBucket(grid, hi);
-        const uint32_t q0 = b0 ? start[b0 - 1] : 0u, q1 = start[b1];
-        for (uint32_t q = q0 + lane; q < q1; q += 32) {
-            const SweepRec rj = recs[q];
-            const uint32_t i = ri.body, j = rj.body;
-            if (j == i || !(rj.start > lo || (rj.start == lo && j > i)) || rj.start > hi) { continue; }
-            const SweepRec& A = i < j ? ri : rj;
-            const SweepRec& Bb = i < j ? rj : ri;
-            if (!(A.flags & kBodyLive) || !(Bb.flags & kBodyLive)) { continue; }
-            if (!((A.flags | Bb.flags) & kBodyDynamic)) { continue; }
-            if (!((A.flags | Bb.flags) & kBodyMoving)) { continue; }
-            const float gg = A.grow + Bb.grow;
-            const Vec3 reach{ gg, gg, gg };
-            if (!boxesOverlap(A.lo - reach, A.hi + reach, Bb.lo, Bb.hi)) { continue; }
-            pairShapes(B, wi, B.bodies[wi.bodyFirst + A.body], B.bodies[wi.bodyFirst + Bb.body], A.grow, Bb.grow, A.lo,
-                       A.hi, Bb.lo, Bb.hi, reach, &wc.candRaw);
+        const uint32_t wide = grid.cells[1] > 1 ? wc.sweepWide : 0u;
+        // Items: the records, then the wide ones' parts.
+        for (uint32_t item = warp; item < n + wide * parts; item += warps) {
+            const bool part = item >= n;
+            const SweepRec ri = recs[part ? wides[(item - n) / parts] : item];
+            if (!(ri.flags & kBodyLive)) { continue; }
+            const float lo = ri.start, hi = B.sweepHi[wi.bodyFirst + ri.body];
+            auto test = [&](const SweepRec& rj) {
+                const uint32_t i = ri.body, j = rj.body;
+                if (j == i || !(rj.start > lo || (rj.start == lo && j > i)) || rj.start > hi) { return; }
+                const SweepRec& A = i < j ? ri : rj;
+                const SweepRec& Bb = i < j ? rj : ri;
+                if (!(A.flags & kBodyLive) || !(Bb.flags & kBodyLive)) { return; }
+                if (!((A.flags | Bb.flags) & kBodyDynamic)) { return; }
+                if (!((A.flags | Bb.flags) & kBodyMoving)) { return; }
+                const float gg = A.grow + Bb.grow;
+                const Vec3 reach{ gg, gg, gg };
+                if (!boxesOverlap(A.lo - reach, A.hi + reach, Bb.lo, Bb.hi)) { return; }
+                pairShapes(B, wi, B.bodies[wi.bodyFirst + A.body], B.bodies[wi.bodyFirst + Bb.body], A.grow, Bb.grow, A.lo,
+                           A.hi, Bb.lo, Bb.hi, reach, &wc.candRaw);
+            };
+            const uint32_t x0 = sweepCell(grid, 0, lo), x1 = sweepCell(grid, 0, hi);
+            if (part) {
+                const uint32_t c0 = x0 * grid.cells[1], c1 = (x1 + 1) * grid.cells[1] - 1;
+                const uint32_t from = (item - n) % parts * kSweepPart;
+                const uint32_t q0 = max(from, c0 ? start[c0 - 1] : 0u), q1 = min(from + kSweepPart, start[c1]);
+                for (uint32_t q = q0 + lane; q < q1; q += 32) {
+                    const SweepRec rj = recs[q];
+                    if (!(rj.flags & kBodyWide)) { test(rj); }
+                }
+                continue;
+            }
+            for (uint32_t q = lane; q < wide; q += 32) { test(recs[wides[q]]); }
+            if (ri.flags & kBodyWide) { continue; }  // its parts take the others
+            float from, to;
+            sweepInterval(grid.axis == 2 ? ri.lo.z : ri.lo.y, grid.axis == 2 ? ri.hi.z : ri.hi.y, ri.grow, from, to);
+            const uint32_t y0 = grid.cells[1] > 1 ? sweepCell(grid, 1, from - grid.width * 1.001f) : 0u;
+            const uint32_t y1 = grid.cells[1] > 1 ? sweepCell(grid, 1, to) : 0u;
+            for (uint32_t x = x0; x <= x1; ++x) {
+                const uint32_t c0 = x * grid.cells[1] + y0, c1 = x * grid.cells[1] + y1;
+                const uint32_t q1 = start[c1];
+                for (uint32_t q = (c0 ? start[c0 - 1] : 0u) + lane; q < q1; q += 32) {
+                    const SweepRec rj = recs[q];
+                    if (!(rj.flags & kBodyWide)) { test(rj); }
+                }
+            }
         }
     }
 }
@@ -2956,12 +3092,12 @@ __global__ void __launch_bounds__(256) k_refresh_all(const __grid_constant__ Bat
     refreshClass<kClassMesh>(B, P, sub);
 }
 
-// One pass over a world's joints on one thread, before the contacts of that pass (src/world.cpp:1670-1680,
+// One pass over a world's joints, before the contacts of that pass (src/world.cpp:1670-1680,
 // src/joint.cpp:568-590): kind 0 scales warm starts by the speed the ends kept under the speed limits
 // (src/joint.cpp:570-593) and warm starts, 1 is the biased solve, 2 the relaxing solve with its reaction. The
 // ends' velocities come from the substep's store.
-template <class Store>
-__device__ void runJoints(const Batch& B, const StepParams& P, const WorldInfo& wi, const Store& st, int kind) {
+template <class G, class Store>
+__device__ void runJoints(const Batch& B, const StepParams& P, const G& g, const WorldInfo& wi, const Store& st, int kind) {
     const uint32_t nj = wi.jointCount;
     DJoint* js = B.joints + wi.jointFirst;
     auto endOf = [&](uint32_t gbody) {
@@ -2979,7 +3115,7 @@ __device__ void runJoints(const Batch& B, const StepParams& P, const WorldInfo& 
         st.storeVW(gbody - wi.bodyFirst, e);
     };
     if (kind == 0) {
-        for (uint32_t x = 0; x < nj; ++x) {
+        for (uint32_t x = g.tid; x < nj; x += g.size) {
             DJoint& j = js[x];
             const JBody a = endOf(j.bodyA), b = endOf(j.bodyB);
             if (!jointActive(j, a, b)) { continue; }
@@ -2995,17 +3131,19 @@ __device__ void runJoints(const Batch& B, const StepParams& P, const WorldInfo& 
             j.frictionImpulse *= f;
             j.swingImpulse *= f;
         }
-        for (uint32_t x = 0; x < nj; ++x) {
+        g.sync();
+        for (uint32_t x = g.tid; x < nj; x += g.size) {
             const DJoint& j = js[x];
             if (!jointActive(j, endOf(j.bodyA), endOf(j.bodyB))) { continue; }
             if (j.bodyA != kWorldEnd) { B.bodies[j.bodyA].kept = 1.0f; }
             B.bodies[j.bodyB].kept = 1.0f;
         }
+        g.sync();
     }
-    for (uint32_t x = 0; x < nj; ++x) {
+    forEachJoint(B, g, wi, [&](uint32_t x) {
         DJoint& j = js[x];
         JBody a = endOf(j.bodyA), b = endOf(j.bodyB);
-        if (!jointActive(j, a, b)) { continue; }
+        if (!jointActive(j, a, b)) { return; }
         if (kind == 0) {
             warmStartJoint(a, b, j);
         } else {
@@ -3014,7 +3152,7 @@ __device__ void runJoints(const Batch& B, const StepParams& P, const WorldInfo& 
         }
         putEnd(j.bodyA, a);
         putEnd(j.bodyB, b);
-    }
+    });
 }
 
 // Whether the batch's active contacts outweigh its bodies, two to one: solved with rooms then (kRoomWarps). The
@@ -3083,10 +3221,7 @@ __global__ void __launch_bounds__(Rooms ? kRoomWarps * 32 : kMaxBlock) k_substep
             for (uint32_t i = g.tid; i < nb; i += g.size) { st.integrateVelocityAt(i, P); }
             g.sync();
             if constexpr (Joints) {
-                if (nj > 0) {
-                    if (g.tid == 0) { runJoints(B, P, wi, st, 0); }
-                    g.sync();
-                }
+                if (nj > 0) { runJoints(B, P, g, wi, st, 0); }
             }
             forEachColorRecord<Rooms>(B, g, wc.colorStart, wc.colorCount, room, [&](uint32_t x) { return cf + x; },
                                       [&](float4* W, float4*) { warmRecord<kStride>(B, st, base, nb, W); });
@@ -3094,10 +3229,7 @@ __global__ void __launch_bounds__(Rooms ? kRoomWarps * 32 : kMaxBlock) k_substep
             for (int pass = 0; pass < 2; ++pass) {
                 const bool bias = pass == 0;
                 if constexpr (Joints) {
-                    if (nj > 0) {
-                        if (g.tid == 0) { runJoints(B, P, wi, st, bias ? 1 : 2); }
-                        g.sync();
-                    }
+                    if (nj > 0) { runJoints(B, P, g, wi, st, bias ? 1 : 2); }
                 }
                 // The active contacts, then the struck ones again (one call site: the solve is inlined once).
                 for (int struck = 0; struck < (wc.impactCount > 0 ? 2 : 1); ++struck) {
@@ -3281,10 +3413,11 @@ __global__ void __launch_bounds__(256, 2) k_substep_flat(const __grid_constant__
     auto jointsPass = [&](int kind) {
         if constexpr (Joints) {
             if (!skip) {
-                for (uint32_t w = tid; w < nw; w += threads) {
+                const Group g = makeGroup(32);
+                for (uint32_t w = warp; w < nw; w += warps) {
                     const WorldInfo& wi = B.info[w];
                     if (wi.jointCount == 0) { continue; }
-                    runJoints(B, P, wi, FlatStore{ B.flatBodies + (size_t)kFlatBodyWords * wi.bodyFirst, B.bodies + wi.bodyFirst },
+                    runJoints(B, P, g, wi, FlatStore{ B.flatBodies + (size_t)kFlatBodyWords * wi.bodyFirst, B.bodies + wi.bodyFirst },
                               kind);
                 }
             }
@@ -3611,8 +3744,8 @@ static __device__ void sweepWorld(const Batch& B, const StepParams& P, const G& 
 // when the world fits, else in its global scratch.
 // After the solve (src/world.cpp:1685-1691): active joints turn the step's impulses into a force and torque
 // and break past their limits (src/world.cpp:1543-1560), the rest settle positions in order, twice over, and
-// every awake dynamic body's world inverse mass is built again at its settled pose. One thread runs the
-// joints; every thread first finds whether any joint was active.
+// every awake dynamic body's world inverse mass is built again at its settled pose. Every thread first finds
+// whether any joint was active.
 template <class G>
 static __device__ void finishJoints(const Batch& B, const StepParams& P, const G& g, const WorldInfo& wi) {
     DJoint* js = B.joints + wi.jointFirst;
@@ -3623,39 +3756,37 @@ static __device__ void finishJoints(const Batch& B, const StepParams& P, const G
     }
     g.sync();
     if (!anyActive) { return; }
-    if (g.tid == 0) {
-        for (uint32_t x = 0; x < wi.jointCount; ++x) {
-            DJoint& j = js[x];
-            if (!jointActive(j, endOf(j.bodyA), endOf(j.bodyB))) { continue; }
-            j.force = j.force / P.dt;
-            j.torque = j.torque / P.dt;
-            if (length(j.force) > j.breakForce || length(j.torque) > j.breakTorque) {
-                j.broken = 1;
-                j.brokeNow = 1;
-                j.linearImpulse = zero3();
-                j.angularImpulse = zero3();
-                j.frictionTurn = zero3();
-                j.axialImpulse = j.motorImpulse = j.lowerImpulse = j.upperImpulse = 0.0f;
-                j.frictionImpulse = j.swingImpulse = 0.0f;
-            }
-        }
-        auto putPose = [&](uint32_t gbody, const JBody& e) {
-            if (gbody == kWorldEnd || e.type != kDynamic || !e.awake) { return; }
-            B.bodies[gbody].com = e.com;
-            B.bodies[gbody].xf = e.xf;
-        };
-        for (int it = 0; it < kSettleIterations; ++it) {
-            for (uint32_t x = 0; x < wi.jointCount; ++x) {
-                const DJoint& j = js[x];
-                JBody a = endOf(j.bodyA), b = endOf(j.bodyB);
-                if (!jointActive(j, a, b)) { continue; }
-                settleJoint(a, b, j);
-                putPose(j.bodyA, a);
-                putPose(j.bodyB, b);
-            }
+    for (uint32_t x = g.tid; x < wi.jointCount; x += g.size) {
+        DJoint& j = js[x];
+        if (!jointActive(j, endOf(j.bodyA), endOf(j.bodyB))) { continue; }
+        j.force = j.force / P.dt;
+        j.torque = j.torque / P.dt;
+        if (length(j.force) > j.breakForce || length(j.torque) > j.breakTorque) {
+            j.broken = 1;
+            j.brokeNow = 1;
+            j.linearImpulse = zero3();
+            j.angularImpulse = zero3();
+            j.frictionTurn = zero3();
+            j.axialImpulse = j.motorImpulse = j.lowerImpulse = j.upperImpulse = 0.0f;
+            j.frictionImpulse = j.swingImpulse = 0.0f;
         }
     }
     g.sync();
+    auto putPose = [&](uint32_t gbody, const JBody& e) {
+        if (gbody == kWorldEnd || e.type != kDynamic || !e.awake) { return; }
+        B.bodies[gbody].com = e.com;
+        B.bodies[gbody].xf = e.xf;
+    };
+    for (int it = 0; it < kSettleIterations; ++it) {
+        forEachJoint(B, g, wi, [&](uint32_t x) {
+            const DJoint& j = js[x];
+            JBody a = endOf(j.bodyA), b = endOf(j.bodyB);
+            if (!jointActive(j, a, b)) { return; }
+            settleJoint(a, b, j);
+            putPose(j.bodyA, a);
+            putPose(j.bodyB, b);
+        });
+    }
     for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
         DBody& b = B.bodies[wi.bodyFirst + i];
         if (b.alive && b.type == kDynamic && b.awake) { updateInverseMass(b); }

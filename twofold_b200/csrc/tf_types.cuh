@@ -207,6 +207,7 @@ struct WorldInfo {
     // Joints from jointFirst in the world's index order, and the body pairs that joints keep from colliding
     // (sorted keys min << 32 | max of world-local bodies) from the same offset.
     uint32_t jointFirst, jointCount, joinedCount;
+    uint32_t jointLevels;  // levels of the world's joints (Batch::jointOrder)
 };
 
 enum JointType : uint32_t { kJointPoint = 0, kJointFixed, kJointHinge, kJointSlider, kJointDistance, kJointSwingTwist };
@@ -260,10 +261,12 @@ struct WorldCounts {
     uint32_t activePoints;     // contact points of the active list
     uint32_t partCount;        // this step's extra mesh parts and triangle bounds used
     uint32_t boundsCount;
-    // Worlds of more than kSweepBodies bodies: raw pair count of this step's sweep, and the range of the
-    // bodies' intervals along x as order-preserving keys.
+    // Worlds of more than kSweepBodies bodies: raw pair count of this step's sweep, the range of the bodies'
+    // intervals along each axis as order-preserving keys, and of the grid's second axis the bodies wide along it
+    // and the largest width of the others (float bits).
     uint32_t candRaw;
-    uint32_t sweepMinKey, sweepMaxKey;
+    uint32_t sweepMinKey[3], sweepMaxKey[3];
+    uint32_t sweepWide, sweepWidth;
     uint32_t colorStart[kColors + 1];
     uint32_t impactColorStart[kColors + 1];
     // The flat solve: where this world's contacts of each color (and impact color) start in that color's
