@@ -256,6 +256,10 @@ public:
     bool poseCopyPending[2] = {};
     int poseSlot = 0;
     cudaEvent_t callStart = nullptr, callStop = nullptr;
+    // The streams beside the engine's for launches that run side by side, and the events that fork and join them.
+    static constexpr int kSideStreams = kPairClasses;
+    cudaStream_t sideStreams[kSideStreams] = {};
+    cudaEvent_t forkEvent = nullptr, joinEvents[kSideStreams] = {};
     float lastElapsedMs = 0.0f;
     int64_t bodyStepsTotal = 0;
     bool profiling = false;
@@ -311,6 +315,11 @@ public:
         if (callStart) { cudaEventDestroy(callStart); }
         if (callStop) { cudaEventDestroy(callStop); }
         dropGraphs();
+        if (forkEvent) { cudaEventDestroy(forkEvent); }
+        for (int k = 0; k < kSideStreams; ++k) {
+            if (joinEvents[k]) { cudaEventDestroy(joinEvents[k]); }
+            if (sideStreams[k]) { cudaStreamDestroy(sideStreams[k]); }
+        }
         if (stream) { cudaStreamDestroy(stream); }
     }
 
@@ -352,14 +361,39 @@ public:
         TF_CUDA(cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount, device));
         TF_CUDA(cudaEventCreate(&callStart));
         TF_CUDA(cudaEventCreate(&callStop));
+        TF_CUDA(cudaEventCreateWithFlags(&forkEvent, cudaEventDisableTiming));
+        for (int k = 0; k < kSideStreams; ++k) {
+            TF_CUDA(cudaStreamCreateWithFlags(&sideStreams[k], cudaStreamNonBlocking));
+            TF_CUDA(cudaEventCreateWithFlags(&joinEvents[k], cudaEventDisableTiming));
+        }
         return TF_OK;
     }
 
     // Launches kernel `id` on the engine's stream; the arguments must have the kernel's parameter types exactly.
     template <class... Args>
     void launch(int id, unsigned grid, unsigned block, size_t smem, Args... args) {
+        launchOn(stream, id, grid, block, smem, args...);
+    }
+    template <class... Args>
+    void launchOn(cudaStream_t on, int id, unsigned grid, unsigned block, size_t smem, Args... args) {
         void* ptrs[] = { (void*)&args... };
-        cudaLaunchKernel(kernelEntry(id), dim3(grid), dim3(block), ptrs, smem, stream);
+        cudaLaunchKernel(kernelEntry(id), dim3(grid), dim3(block), ptrs, smem, on);
+    }
+
+    // Runs f(k, stream) for every k < n with the launches side by side: the first on the engine's stream, the others
+    // on streams of their own between an event each way, in a captured graph as branches. The pair classes' launches
+    // touch disjoint pairs; one after another, each left most of the device idle behind its slowest pair (a mid-step
+    // refresh of the terrain: 900 us as the sum of its lists, 550 side by side).
+    template <class F>
+    void sideBySide(int n, F&& f) {
+        cudaEventRecord(forkEvent, stream);
+        for (int k = 1; k < n; ++k) {
+            cudaStreamWaitEvent(sideStreams[k - 1], forkEvent, 0);
+            f(k, sideStreams[k - 1]);
+            cudaEventRecord(joinEvents[k - 1], sideStreams[k - 1]);
+        }
+        f(0, stream);
+        for (int k = 1; k < n; ++k) { cudaStreamWaitEvent(stream, joinEvents[k - 1], 0); }
     }
 
     // A cooperative launch (every CTA resident at once, which the flat solve's grid barrier needs); grid must
@@ -1962,7 +1996,10 @@ public:
                 launch(kKCollideAll, *std::max_element(flatGrids, flatGrids + kPairClasses), threads(7), 0, B, P, serial);
                 return;
             }
-            for (int c = 0; c < kPairClasses; ++c) { launch(kKCollide + c, flatGrids[c], flatThreads(c), 0, B, P, serial); }
+            sideBySide(kPairClasses, [&](int k, cudaStream_t on) {
+                const int c = kPairClasses - 1 - k;  // the heaviest pairs first
+                launchOn(on, kKCollide + c, flatGrids[c], flatThreads(c), 0, B, P, serial);
+            });
         });
         timed(1, rec, [&] {
             if (clusters) { launchClusters(kKNarrowphaseBig, threads(1), B, P, splits[1], serial); }
@@ -1985,10 +2022,14 @@ public:
                         launch(kKRefreshAll, flatGrids[6], threads(4), 0, B, P, i, serial);
                         return;
                     }
-                    launch(kKRefresh + kPairClasses, flatGrids[6], threads(4), 0, B, P, i, serial);
-                    for (int c = 0; c < kPairClasses; ++c) {
-                        launch(kKRefresh + c, flatGrids[7 + c], flatThreads(7 + c), 0, B, P, i, serial);
-                    }
+                    sideBySide(kPairClasses + 1, [&](int k, cudaStream_t on) {
+                        const int c = kPairClasses - 1 - k;
+                        if (c < 0) {
+                            launchOn(on, kKRefresh + kPairClasses, flatGrids[6], threads(4), 0, B, P, i, serial);
+                        } else {
+                            launchOn(on, kKRefresh + c, flatGrids[7 + c], flatThreads(7 + c), 0, B, P, i, serial);
+                        }
+                    });
                 });
             }
             timed(5, rec, [&] {
