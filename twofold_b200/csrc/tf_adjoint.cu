@@ -204,6 +204,7 @@ struct Model {
     T* invMAdj;    // 1
     T* invIAdj;    // 9
     PointState<T>* pointAdj;  // contactSlots x 4
+    T* muAdj;                 // contactSlots: each contact's friction over the step
     T* massAdj;      // per body (output, summed)
     T* frictionAdj;  // per shape (output, summed)
     T* log;          // per slot and world: logStride values
@@ -350,6 +351,30 @@ __device__ __forceinline__ T pushAdj(const SBody<T>& a, const SBody<T>& b, const
     return g;
 }
 
+// A push along x in reverse, in two parts: its impulse's adjoint, read from the bodies' velocity adjoints (va, wa, vb,
+// wb) in the chain of rows; and what it adds to the adjoints of inverse mass and inertia, which no row reads.
+template <class T>
+__device__ __forceinline__ T impulseAdj(const SBody<T>& a, const SBody<T>& b, const Axis<T>& x, V3<T> va, V3<T> wa,
+                                        V3<T> vb, V3<T> wb) {
+    T g = 0;
+    if (a.moves) { g -= a.im * dot(x.d, va) + dot(x.angA, wa); }
+    if (b.moves) { g += b.im * dot(x.d, vb) + dot(x.angB, wb); }
+    return g;
+}
+
+template <class T>
+__device__ __forceinline__ void pushMassAdj(const SBody<T>& a, const SBody<T>& b, const Axis<T>& x, T impulse, V3<T> va,
+                                            V3<T> wa, V3<T> vb, V3<T> wb, BodyAdj<T>& ga, BodyAdj<T>& gb) {
+    if (a.moves) {
+        ga.im -= impulse * dot(x.d, va);
+        addOuter(ga.I, wa, x.armA, -impulse);
+    }
+    if (b.moves) {
+        gb.im += impulse * dot(x.d, vb);
+        addOuter(gb.I, wb, x.armB, impulse);
+    }
+}
+
 template <class T>
 __device__ __forceinline__ void speedAdj(const Axis<T>& x, T g, BodyAdj<T>& ga, BodyAdj<T>& gb) {
     ga.v = ga.v - x.d * g;
@@ -418,6 +443,9 @@ __device__ __forceinline__ CPoint<T> pointOf(const CData<T>& c, int i) {
 
 // ---------------------------------------------------------------------------------------------------------
 // Contact operations: forward, and reverse from the logged inputs.
+
+// Threads of the reverse walk's CTA, one world's: 32 contacts at a time.
+constexpr uint32_t kWalkThreads = 128;
 
 enum Op : int { kWarm = 0, kBias = 1, kRelax = 2, kRestitute = 3 };
 
@@ -754,11 +782,200 @@ __device__ __forceinline__ void contactOpAdj(const Model<T>& M, int op, const SB
     }
 }
 
-// Asks for the 128-byte lines of [from, to) in L1, spread over the warp's lanes.
+// The same operations in reverse, four lanes a contact and a lane a point, from the contact's record: each row's input
+// that the reverse needs is the points' state before the operation (a point's rows of one kind run once, so each row
+// starts from it, the friction rows with the normal impulse logged beside them) and the logged speeds.
+//
+// The rows run in reverse one after another, each seeing the velocity adjoints the one before it left; but a row's
+// axes, forces, branches and displacement terms do not depend on them, nor does any row read what a row adds to the
+// adjoints of inverse masses, inertias and displacements. So every lane first prepares its point's row, then the rows'
+// chains run in order (the lane whose row it is hands the velocity adjoints on by shuffles), then every lane adds its
+// row's share, and the four lanes' shares are summed at the end. One lane a contact ran all of that for its points in
+// turn; where few worlds leave the device waiting for their chains this takes a third to three fifths of its time.
 template <class T>
-__device__ __forceinline__ void prefetchRange(const T* from, const T* to, uint32_t lane) {
+struct QuadRow {
+    Axis<T> x;
+    V3<T> va, wa, vb, wb;  // the velocity adjoints the row saw
+};
+
+template <class T>
+__device__ __forceinline__ void handOn(BodyAdj<T>& ga, BodyAdj<T>& gb, int i) {
+    auto take = [&](V3<T>& v) {
+        v.x = __shfl_sync(0xffffffffu, v.x, i, 4);
+        v.y = __shfl_sync(0xffffffffu, v.y, i, 4);
+        v.z = __shfl_sync(0xffffffffu, v.z, i, 4);
+    };
+    take(ga.v), take(ga.w), take(gb.v), take(gb.w);
+}
+
+// Sum over a contact's four lanes, in every one of them, always added in the same order.
+template <class T>
+__device__ __forceinline__ T quadSum(T x) {
+    x += __shfl_xor_sync(0xffffffffu, x, 1, 4);
+    return x + __shfl_xor_sync(0xffffffffu, x, 2, 4);
+}
+
+// ga.v, ga.w, gb.v, gb.w and gp hold the adjoints after the operation on entry (the velocities' alike in the four
+// lanes, gp the lane's own point's) and before it on return; the rest of ga and gb gets the lane's share. Velocities of
+// a and b are not read. n: the contact's points (0 for lanes without one); most: the largest of the warp.
+template <class T>
+__device__ __forceinline__ void quadOpAdj(const Model<T>& M, int op, const SBody<T>& a, const SBody<T>& b, const TapeContact& tc,
+                                          int n, int most, T mu, BodyAdj<T>& ga, BodyAdj<T>& gb, PointState<T>& gp, T& muG,
+                                          const T* rec) {
+    const int q = (int)(threadIdx.x & 3);
+    const bool mine = q < n;
+    V3<T> normal = zeroV<T>(), t1 = normal, t2 = normal, ra = normal, rb = normal;
+    T adjSep = 0, relVel = 0, restitution = 0;
+    PointState<T> p0{ 0, zeroV<T>(), 0 };
+    T speed = 0, row[3] = { 0, 0, 0 };
+    const bool useBias = op == kBias;
+    if (mine) {
+        normal = fl3<T>(tc.normal);
+        t1 = fl3<T>(tc.t1);
+        t2 = fl3<T>(tc.t2);
+        ra = fl3<T>(tc.anchorA[q]);
+        rb = fl3<T>(tc.anchorB[q]);
+        adjSep = T(tc.adjSep[q]);
+        relVel = T(tc.relVel[q]);
+        restitution = T(tc.restitution);
+        p0 = { rec[5 * q], ld3(rec + 5 * q + 1), rec[5 * q + 4] };
+        speed = rec[kSpeedAt + q];
+        const T* r = rec + kFrictionAt + 3 * (useBias ? q : n - 1 - q);
+        row[0] = r[0], row[1] = r[1], row[2] = r[2];
+    }
+    if (op == kWarm) {
+        // No row of a warm start changes a velocity adjoint: the points are independent.
+        if (mine) {
+            const Axis<T> xn = makeAxis(a, b, ra, rb, normal), x1 = makeAxis(a, b, ra, rb, t1), x2 = makeAxis(a, b, ra, rb, t2);
+            pushMassAdj(a, b, xn, p0.n, ga.v, ga.w, gb.v, gb.w, ga, gb);
+            pushMassAdj(a, b, x1, dot(p0.t, t1), ga.v, ga.w, gb.v, gb.w, ga, gb);
+            pushMassAdj(a, b, x2, dot(p0.t, t2), ga.v, ga.w, gb.v, gb.w, ga, gb);
+            gp.n += impulseAdj(a, b, xn, ga.v, ga.w, gb.v, gb.w);
+            gp.t = gp.t + t1 * impulseAdj(a, b, x1, ga.v, ga.w, gb.v, gb.w) + t2 * impulseAdj(a, b, x2, ga.v, ga.w, gb.v, gb.w);
+        }
+        return;
+    }
+    const Softness<T> soft = (!a.moves || !b.moves) ? M.staticSoft : M.contactSoft;
+    if (op != kRestitute) {
+        // The friction rows (frictionRow): backward from the last one solved.
+        QuadRow<T> r1{ makeAxis(a, b, ra, rb, t1) }, r2{ makeAxis(a, b, ra, rb, t2) };
+        const T old1 = dot(p0.t, t1), old2 = dot(p0.t, t2);
+        const T s1 = row[0], s2 = row[1], pn = row[2];
+        const T f1 = old1 - r1.x.mass * s1, f2 = old2 - r2.x.mass * s2;
+        const T limit = mu * pn;
+        const T mag = sqrtT(f1 * f1 + f2 * f2);
+        // With no friction allowed (limit 0) the row adds nothing whatever f is, also at f = 0 where the forward
+        // takes the unclamped branch with the same result: the derivative is that of the clamp.
+        const bool clamp = mag > limit || limit == T(0);
+        const T scale = mag > limit ? (mag > T(0) ? limit / mag : T(0)) : (limit == T(0) ? T(0) : T(1));
+        const T g1 = f1 * scale, g2 = f2 * scale;
+        const T perMag = mag > T(0) ? T(1) / mag : T(0);
+        const T pt1 = dot(gp.t, t1), pt2 = dot(gp.t, t2);
+        T old1G = 0, old2G = 0, f1G = 0, f2G = 0;
+        for (int j = 0; j < most; ++j) {
+            const int i = useBias ? most - 1 - j : j;
+            if (i < n) {
+                const T d1G = impulseAdj(a, b, r1.x, ga.v, ga.w, gb.v, gb.w);
+                const T d2G = impulseAdj(a, b, r2.x, ga.v, ga.w, gb.v, gb.w);
+                const T g1G = d1G + pt1, g2G = d2G + pt2;
+                T h1 = g1G, h2 = g2G, limitG = 0;
+                if (clamp && mag > T(0)) {
+                    const T scaleG = g1G * f1 + g2G * f2;
+                    limitG = scaleG * perMag;
+                    const T magG = -limitG * limit * perMag;
+                    h1 = g1G * scale + magG * f1 * perMag;
+                    h2 = g2G * scale + magG * f2 * perMag;
+                } else if (clamp) {
+                    h1 = 0;
+                    h2 = 0;
+                }
+                if (q == i) {
+                    r1.va = ga.v, r1.wa = ga.w, r1.vb = gb.v, r1.wb = gb.w;
+                    f1G = h1;
+                    f2G = h2;
+                    old1G = h1 - d1G;
+                    old2G = h2 - d2G;
+                    muG += limitG * pn;
+                    gp.n += limitG * mu;
+                }
+                speedAdj(r1.x, -h1 * r1.x.mass, ga, gb);
+                speedAdj(r2.x, -h2 * r2.x.mass, ga, gb);
+            }
+            handOn(ga, gb, i);
+        }
+        if (mine) {
+            pushMassAdj(a, b, r1.x, g1 - old1, r1.va, r1.wa, r1.vb, r1.wb, ga, gb);
+            pushMassAdj(a, b, r2.x, g2 - old2, r1.va, r1.wa, r1.vb, r1.wb, ga, gb);
+            axisMassAdj(r1.x, -f1G * s1, ga.im, ga.I, gb.im, gb.I);
+            axisMassAdj(r2.x, -f2G * s2, ga.im, ga.I, gb.im, gb.I);
+            gp.t = t1 * old1G + t2 * old2G;
+        }
+    }
+    // The normal rows (normalRow), or the restitution rows (restituteRow) of the points that restitute.
+    QuadRow<T> r{ makeAxis(a, b, ra, rb, normal) };
+    T bias = 0, ms = 1, is = 0;
+    int biasKind = 0;  // 0 none, 1 sep * invH, 2 biasRate * sep, 3 clamped at -maxPushout
+    bool solved = true;
+    if (op == kRestitute) {
+        solved = restitution != T(0) && !(relVel > -M.restThreshold || p0.maxN == T(0));
+        bias = restitution * relVel;
+    } else {
+        const V3<T> d = b.dp - a.dp + rotate(b.dq, rb) - rotate(a.dq, ra);
+        const T sep = dot(d, normal) + adjSep;
+        if (sep > T(0)) {
+            bias = sep * M.invH;
+            biasKind = 1;
+        } else if (useBias) {
+            const T b1 = soft.biasRate * sep;
+            biasKind = b1 > -M.maxPushout ? 2 : 3;
+            bias = fmax(b1, -M.maxPushout);
+            ms = soft.massScale;
+            is = soft.impulseScale;
+        }
+    }
+    const T imp = -r.x.mass * ms * (speed + bias) - is * p0.n;
+    const T total = fmax(p0.n + imp, T(0));
+    const T delta = total - p0.n;
+    const bool pushed = p0.n + imp > T(0), grew = delta > p0.maxN;
+    T impG = 0;
+    for (int i = most - 1; i >= 0; --i) {
+        if (i < n && solved) {
+            // Reverse: push, max, total, impulse.
+            T deltaG = impulseAdj(a, b, r.x, ga.v, ga.w, gb.v, gb.w);
+            if (grew) { deltaG += gp.maxN; }
+            const T g = pushed ? gp.n + deltaG : T(0);
+            if (q == i) {
+                r.va = ga.v, r.wa = ga.w, r.vb = gb.v, r.wb = gb.w;
+                impG = g;
+                gp.n = g - deltaG - g * is;
+                if (grew) { gp.maxN = 0; }
+            }
+            speedAdj(r.x, -g * r.x.mass * ms, ga, gb);
+        }
+        handOn(ga, gb, i);
+    }
+    if (mine && solved) {
+        pushMassAdj(a, b, r.x, delta, r.va, r.wa, r.vb, r.wb, ga, gb);
+        axisMassAdj(r.x, -impG * ms * (speed + bias), ga.im, ga.I, gb.im, gb.I);
+        const T biasG = -impG * r.x.mass * ms;
+        T sepG = 0;
+        if (biasKind == 1) { sepG = biasG * M.invH; }
+        if (biasKind == 2) { sepG = biasG * soft.biasRate; }
+        if (sepG != T(0)) {
+            const V3<T> dg = normal * sepG;
+            gb.dp = gb.dp + dg;
+            ga.dp = ga.dp - dg;
+            rotateAdj(b.dq, rb, dg, gb.dq);
+            rotateAdj(a.dq, ra, dg * T(-1), ga.dq);
+        }
+    }
+}
+
+// Asks for the 128-byte lines of [from, to) in L1, spread over a world's threads.
+template <class T>
+__device__ __forceinline__ void prefetchRange(const T* from, const T* to, uint32_t tid, uint32_t threads) {
     const char* end = reinterpret_cast<const char*>(to);
-    for (const char* p = reinterpret_cast<const char*>(from) + 128 * lane; p < end; p += 128 * 32) {
+    for (const char* p = reinterpret_cast<const char*>(from) + 128 * tid; p < end; p += 128 * threads) {
         asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
     }
 }
@@ -770,20 +987,20 @@ template <class T>
 __host__ __device__ constexpr int stageCalls() { return sizeof(T) == 4 ? 48 : 32; }
 
 // Copies `words` values (whole 16-byte pieces, both addresses 16-byte aligned) from global to shared memory
-// with asynchronous copies spread over the warp's lanes, as one commit group of each lane.
+// with asynchronous copies spread over a world's threads, as one commit group of each thread.
 template <class T>
-__device__ __forceinline__ void copyToShared(T* dst, const T* src, uint32_t words, uint32_t lane) {
+__device__ __forceinline__ void copyToShared(T* dst, const T* src, uint32_t words, uint32_t tid, uint32_t threads) {
     const uint32_t pieces = words * (uint32_t)sizeof(T) / 16u;
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     const char* from = reinterpret_cast<const char*>(src);
-    for (uint32_t k = lane; k < pieces; k += 32) {
+    for (uint32_t k = tid; k < pieces; k += threads) {
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16u * k), "l"(from + 16u * k) : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// One world's step, forward (with optional logging) and in reverse. One warp per world.
+// One world's step, forward (with optional logging, a warp a world) and in reverse (a warp or a CTA a world).
 
 struct WorldView {
     uint32_t bodyFirst, bodyCount, shapeFirst;
@@ -855,16 +1072,11 @@ __device__ __forceinline__ int passLists(const WorldView& V, int op, PassList* o
     return n;
 }
 
-// Forward of one step of one world. state: in at `in`, out at `out` (may be the same). When log is non-null the
-// inputs of every contact operation and position update are written there for the reverse pass.
+// A step's start: world inverse inertia at this pose, zero displacement, warm-start impulses. By `threads` threads.
 template <class T>
-__device__ void stepWorld(const Model<T>& M, const Slot<T>& W, int step, uint32_t w, const T* in, T* out, T* log,
-                          T* integLog, unsigned long long* sig = nullptr) {
-    const uint32_t lane = threadIdx.x & 31;
-    const WorldView V = viewOf(M.S, step, w);
-    const int n = M.S.substeps;
-    // Step start: world inverse inertia at this pose, zero displacement, warm-start impulses.
-    for (uint32_t i = lane; i < V.bodyCount; i += 32) {
+__device__ __forceinline__ void stepStart(const Model<T>& M, const Slot<T>& W, const WorldView& V, const T* in, T* out,
+                                          uint32_t tid, uint32_t threads) {
+    for (uint32_t i = tid; i < V.bodyCount; i += threads) {
         const uint32_t g = V.bodyFirst + i;
         const T* s = in + (size_t)g * kState;
         T* o = out + (size_t)g * kState;
@@ -891,7 +1103,7 @@ __device__ void stepWorld(const Model<T>& M, const Slot<T>& W, int step, uint32_
         st4(W.qBase + 4 * (size_t)g, q);
     }
     const uint32_t cf = V.tw->contactFirst;
-    for (uint32_t ci = lane; ci < V.tw->contactCount; ci += 32) {
+    for (uint32_t ci = tid; ci < V.tw->contactCount; ci += threads) {
         const TapeContact& tc = V.contacts[ci];
         for (int i = 0; i < 4; ++i) {
             PointState<T>& p = W.points[(size_t)(cf + ci) * 4 + i];
@@ -900,6 +1112,57 @@ __device__ void stepWorld(const Model<T>& M, const Slot<T>& W, int step, uint32_
             p.maxN = 0;
         }
     }
+}
+
+template <class T>
+__device__ __forceinline__ void velocityUpdate(const Model<T>& M, const WorldView& V, T* out, uint32_t tid, uint32_t threads) {
+    for (uint32_t i = tid; i < V.bodyCount; i += threads) {
+        const uint32_t g = V.bodyFirst + i;
+        if (!movesIn(M, V, g)) { continue; }
+        T* o = out + (size_t)g * kState;
+        const V3<T> v = ld3(o + 7), wv = ld3(o + 10);
+        const T gs = T(M.S.gravityScale[g]);
+        const V3<T> nv = (v + M.gravity * (gs * M.h)) * (T(1) / (T(1) + M.h * T(M.S.linearDamping[g])));
+        const V3<T> nw = wv * (T(1) / (T(1) + M.h * T(M.S.angularDamping[g])));
+        st3(o + 7, nv);
+        st3(o + 10, nw);
+    }
+}
+
+template <class T>
+__device__ __forceinline__ void positionUpdate(const Model<T>& M, const Slot<T>& W, const WorldView& V, T* out, int sub,
+                                               T* integLog, uint32_t tid, uint32_t threads) {
+    for (uint32_t i = tid; i < V.bodyCount; i += threads) {
+        const uint32_t g = V.bodyFirst + i;
+        if (!movesIn(M, V, g)) { continue; }
+        T* o = out + (size_t)g * kState;
+        const V3<T> v = ld3(o + 7), wv = ld3(o + 10);
+        const Q4<T> q = ld4(o + 3);
+        st3(o, ld3(o) + v * M.h);
+        const V3<T> ndp = ld3(W.dp + 3 * (size_t)g) + v * M.h;
+        st3(W.dp + 3 * (size_t)g, ndp);
+        if (integLog) {
+            T* L = integLog + ((size_t)sub * M.S.totalBodies + g) * kIntegWords;
+            st4(L, q);
+            st3(L + 4, wv);
+            st3(L + 7, ndp);
+        }
+        const Q4<T> nq = integrateQ(q, wv, M.h);
+        st4(o + 3, nq);
+        st4(W.dq + 4 * (size_t)g, qmul(nq, conj(ld4(W.qBase + 4 * (size_t)g))));
+    }
+}
+
+// Forward of one step of one world. state: in at `in`, out at `out` (may be the same). When log is non-null the
+// inputs of every contact operation and position update are written there for the reverse pass.
+template <class T>
+__device__ void stepWorld(const Model<T>& M, const Slot<T>& W, int step, uint32_t w, const T* in, T* out, T* log,
+                          T* integLog, unsigned long long* sig = nullptr) {
+    const uint32_t lane = threadIdx.x & 31;
+    const WorldView V = viewOf(M.S, step, w);
+    const int n = M.S.substeps;
+    stepStart(M, W, V, in, out, lane, 32);
+    const uint32_t cf = V.tw->contactFirst;
     __syncwarp();
     uint64_t cursor = 0;  // log index of the next operation; every lane keeps the same count
     auto runOp = [&](int op, uint32_t ci, uint64_t at) {
@@ -947,47 +1210,223 @@ __device__ void stepWorld(const Model<T>& M, const Slot<T>& W, int step, uint32_
         }
     };
     for (int sub = 0; sub < n; ++sub) {
-        for (uint32_t i = lane; i < V.bodyCount; i += 32) {
-            const uint32_t g = V.bodyFirst + i;
-            if (!movesIn(M, V, g)) { continue; }
-            T* o = out + (size_t)g * kState;
-            const V3<T> v = ld3(o + 7), wv = ld3(o + 10);
-            const T gs = T(M.S.gravityScale[g]);
-            const V3<T> nv = (v + M.gravity * (gs * M.h)) * (T(1) / (T(1) + M.h * T(M.S.linearDamping[g])));
-            const V3<T> nw = wv * (T(1) / (T(1) + M.h * T(M.S.angularDamping[g])));
-            st3(o + 7, nv);
-            st3(o + 10, nw);
-        }
+        velocityUpdate(M, V, out, lane, 32);
         __syncwarp();
         pass(kWarm);
         pass(kBias);
-        for (uint32_t i = lane; i < V.bodyCount; i += 32) {
-            const uint32_t g = V.bodyFirst + i;
-            if (!movesIn(M, V, g)) { continue; }
-            T* o = out + (size_t)g * kState;
-            const V3<T> v = ld3(o + 7), wv = ld3(o + 10);
-            const Q4<T> q = ld4(o + 3);
-            st3(o, ld3(o) + v * M.h);
-            const V3<T> ndp = ld3(W.dp + 3 * (size_t)g) + v * M.h;
-            st3(W.dp + 3 * (size_t)g, ndp);
-            if (integLog) {
-                T* L = integLog + ((size_t)sub * M.S.totalBodies + g) * kIntegWords;
-                st4(L, q);
-                st3(L + 4, wv);
-                st3(L + 7, ndp);
-            }
-            const Q4<T> nq = integrateQ(q, wv, M.h);
-            st4(o + 3, nq);
-            st4(W.dq + 4 * (size_t)g, qmul(nq, conj(ld4(W.qBase + 4 * (size_t)g))));
-        }
+        positionUpdate(M, W, V, out, sub, integLog, lane, 32);
         __syncwarp();
         pass(kRelax);
     }
     pass(kRestitute);
 }
 
+// Hands lane i's velocities to the contact's four lanes (every lane of the warp calls it; where the contact has no point
+// i no lane changed them).
+template <class T>
+__device__ __forceinline__ void handOn(SBody<T>& a, SBody<T>& b, int i) {
+    auto take = [&](V3<T>& v) {
+        v.x = __shfl_sync(0xffffffffu, v.x, i, 4);
+        v.y = __shfl_sync(0xffffffffu, v.y, i, 4);
+        v.z = __shfl_sync(0xffffffffu, v.z, i, 4);
+    };
+    take(a.v), take(a.w), take(b.v), take(b.w);
+}
+
+// contactOp four lanes a contact and a lane a point, without a record: every lane prepares its point's row (axes,
+// separation, bias), then the rows run in order, the lane whose row it is handing the velocities on. c holds the lane's
+// own point in place 0; n, most as in quadOpAdj.
+template <class T>
+__device__ __forceinline__ void quadOp(const Model<T>& M, int op, SBody<T>& a, SBody<T>& b, const CData<T>& c, int n, int most,
+                                       PointState<T>& p, T mu, unsigned long long* sig, unsigned long long tag) {
+    const int q = (int)(threadIdx.x & 3);
+    const Softness<T> soft = (!a.moves || !b.moves) ? M.staticSoft : M.contactSoft;
+    if (op == kWarm) {
+        const Axis<T> xn = makeAxis(a, b, c.ra[0], c.rb[0], c.n);
+        const Axis<T> x1 = makeAxis(a, b, c.ra[0], c.rb[0], c.t1);
+        const Axis<T> x2 = makeAxis(a, b, c.ra[0], c.rb[0], c.t2);
+        const T i1 = dot(p.t, c.t1), i2 = dot(p.t, c.t2);
+        for (int i = 0; i < most; ++i) {
+            if (i < n) {
+                push(a, b, xn, p.n);
+                push(a, b, x1, i1);
+                push(a, b, x2, i2);
+            }
+            handOn(a, b, i);
+        }
+        return;
+    }
+    if (op == kRestitute) {
+        const Axis<T> x = makeAxis(a, b, c.ra[0], c.rb[0], c.n);
+        const bool solved = c.restitution != T(0) && restitutes(M, c, 0, p);
+        uint32_t bits = 128u;
+        for (int i = 0; i < most; ++i) {
+            if (i < n && solved) {
+                const T vn = speedAlong(a, b, x);
+                const T imp = -x.mass * (vn + c.restitution * c.relVel[0]);
+                const T total = fmax(p.n + imp, T(0));
+                const T delta = total - p.n;
+                if (q == i) { bits = (x.on ? 1u : 0u) | (p.n + imp > T(0) ? 2u : 0u) | 64u; }
+                push(a, b, x, delta);
+                if (q == i) {
+                    p.n = total;
+                    p.maxN = fmax(p.maxN, delta);
+                }
+            }
+            handOn(a, b, i);
+        }
+        if (sig && q < n && c.restitution != T(0)) { *sig += branchHash(tag, (uint32_t)q, bits); }
+        return;
+    }
+    const bool useBias = op == kBias;
+    uint32_t bits = 0;
+    {
+        const Axis<T> x = makeAxis(a, b, c.ra[0], c.rb[0], c.n);
+        const V3<T> d = b.dp - a.dp + rotate(b.dq, c.rb[0]) - rotate(a.dq, c.ra[0]);
+        const T sep = dot(d, c.n) + c.adjSep[0];
+        T bias = 0, ms = 1, is = 0;
+        uint32_t biasKind = 0;
+        if (sep > T(0)) {
+            bias = sep * M.invH;
+            biasKind = 1;
+        } else if (useBias) {
+            biasKind = soft.biasRate * sep > -M.maxPushout ? 2 : 3;
+            bias = fmax(soft.biasRate * sep, -M.maxPushout);
+            ms = soft.massScale;
+            is = soft.impulseScale;
+        }
+        for (int i = 0; i < most; ++i) {
+            if (i < n) {
+                const T vn = speedAlong(a, b, x);
+                const T imp = -x.mass * ms * (vn + bias) - is * p.n;
+                const T total = fmax(p.n + imp, T(0));
+                const T delta = total - p.n;
+                if (q == i) { bits = (x.on ? 1u : 0u) | biasKind << 1 | (p.n + imp > T(0) ? 8u : 0u); }
+                push(a, b, x, delta);
+                if (q == i) {
+                    p.n = total;
+                    p.maxN = fmax(p.maxN, delta);
+                }
+            }
+            handOn(a, b, i);
+        }
+        if (sig && q < n) { *sig += branchHash(tag, (uint32_t)q, bits); }
+    }
+    // Friction forward in the biased pass and backward in the relax pass; row n + j is the j-th friction row.
+    const Axis<T> x1 = makeAxis(a, b, c.ra[0], c.rb[0], c.t1);
+    const Axis<T> x2 = makeAxis(a, b, c.ra[0], c.rb[0], c.t2);
+    const T old1 = dot(p.t, c.t1), old2 = dot(p.t, c.t2);
+    for (int j = 0; j < most; ++j) {
+        const int i = useBias ? j : most - 1 - j;
+        if (i < n) {
+            const T s1 = speedAlong(a, b, x1), s2 = speedAlong(a, b, x2);
+            T f1 = old1 - x1.mass * s1;
+            T f2 = old2 - x2.mass * s2;
+            const T limit = mu * p.n;
+            const T mag = sqrtT(f1 * f1 + f2 * f2);
+            if (q == i) { bits = (x1.on ? 1u : 0u) | (x2.on ? 2u : 0u) | (mag > limit ? 4u : 0u) | (mag > T(0) ? 8u : 0u) | 32u; }
+            if (mag > limit) {
+                const T scale = mag > T(0) ? limit / mag : T(0);
+                f1 *= scale;
+                f2 *= scale;
+            }
+            if (q == i) { p.t = c.t1 * f1 + c.t2 * f2; }
+            push(a, b, x1, f1 - old1);
+            push(a, b, x2, f2 - old2);
+        }
+        handOn(a, b, i);
+    }
+    if (sig && q < n) { *sig += branchHash(tag, (uint32_t)(n + (useBias ? q : n - 1 - q)), bits); }
+}
+
+// The forward's step with a CTA a world and four lanes a contact.
+template <class T>
+__device__ void stepWorldWide(const Model<T>& M, const Slot<T>& W, int step, uint32_t w, const T* in, T* out,
+                              unsigned long long* sig) {
+    const uint32_t tid = threadIdx.x, q = tid & 3;
+    constexpr uint32_t kThreads = kWalkThreads;
+    const WorldView V = viewOf(M.S, step, w);
+    stepStart(M, W, V, in, out, tid, kThreads);
+    __syncthreads();
+    const uint32_t cf = V.tw->contactFirst;
+    uint64_t cursor = 0;
+    auto runOp = [&](int op, bool on, uint32_t ci, uint64_t at) {
+        const TapeContact& tc = V.contacts[on ? ci : 0];
+        const int n = on ? tc.count : 0;
+        const int most = (int)__reduce_max_sync(0xffffffffu, (uint32_t)n);
+        if (most == 0) { return; }
+        const uint32_t ga = V.bodyFirst + (on ? tc.a : 0u), gb = V.bodyFirst + (on ? tc.b : 0u);
+        SBody<T> a = bodyOf(M, W, V, ga, out), b = bodyOf(M, W, V, gb, out);
+        CData<T> c;
+        PointState<T>* ps = W.points + (size_t)(cf + ci) * 4 + q;
+        PointState<T> p{ 0, zeroV<T>(), 0 };
+        c.n = c.t1 = c.t2 = c.ra[0] = c.rb[0] = zeroV<T>();
+        c.adjSep[0] = c.relVel[0] = c.restitution = 0;
+        if ((int)q < n) {
+            c.n = fl3<T>(tc.normal);
+            c.t1 = fl3<T>(tc.t1);
+            c.t2 = fl3<T>(tc.t2);
+            c.ra[0] = fl3<T>(tc.anchorA[q]);
+            c.rb[0] = fl3<T>(tc.anchorB[q]);
+            c.adjSep[0] = T(tc.adjSep[q]);
+            c.relVel[0] = T(tc.relVel[q]);
+            c.restitution = T(tc.restitution);
+            p = *ps;
+        }
+        quadOp(M, op, a, b, c, n, most, p, on ? contactFriction(M, V, tc) : T(0), sig,
+               (unsigned long long)step << 40 ^ at << 2 ^ (unsigned long long)op);
+        if ((int)q < n) { *ps = p; }
+        if (n > 0 && q == 0 && a.moves) {
+            st3(out + (size_t)ga * kState + 7, a.v);
+            st3(out + (size_t)ga * kState + 10, a.w);
+        }
+        if (n > 0 && q == 1 && b.moves) {
+            st3(out + (size_t)gb * kState + 7, b.v);
+            st3(out + (size_t)gb * kState + 10, b.w);
+        }
+    };
+    auto pass = [&](int op) {
+        PassList lists[4];
+        const int nl = passLists(V, op, lists);
+        for (int l = 0; l < nl; ++l) {
+            const PassList& L = lists[l];
+            if (L.start) {
+                const uint32_t first = L.start[0];
+                for (uint32_t k = 0; k < L.count; ++k) {
+                    const uint32_t end = L.start[k + 1];
+                    for (uint32_t x = L.start[k] + tid / 32 * 8; x < end; x += kThreads / 4) {
+                        const uint32_t mine = x + (tid & 31) / 4;
+                        runOp(op, mine < end, mine < end ? L.list[mine] : 0u, cursor + (mine - first));
+                    }
+                    __syncthreads();
+                }
+                cursor += L.start[L.count] - first;
+            } else {
+                if (tid < 32) {
+                    for (uint32_t x = 0; x < L.count; ++x) {
+                        runOp(op, tid < 4, L.list[x], cursor + x);
+                        __syncwarp();
+                    }
+                }
+                cursor += L.count;
+                __syncthreads();
+            }
+        }
+    };
+    for (int sub = 0; sub < M.S.substeps; ++sub) {
+        velocityUpdate(M, V, out, tid, kThreads);
+        __syncthreads();
+        pass(kWarm);
+        pass(kBias);
+        positionUpdate(M, W, V, out, sub, (T*)nullptr, tid, kThreads);
+        __syncthreads();
+        pass(kRelax);
+    }
+    pass(kRestitute);
+}
+
 // The per-body arrays the reverse walk reads and writes, indexed by the body's place in its world. They are
-// the warp's share of shared memory when the kernel has one for bodies (the adjoint state is copied in at the
+// the world's share of shared memory when the kernel has one for bodies (the adjoint state is copied in at the
 // start of the walk and out at its end, the step's inverse masses and inertias at each step's start), else the
 // global arrays offset to the world's first body.
 template <class T>
@@ -1031,12 +1470,12 @@ __device__ __forceinline__ BodyArrays<T> globalBodies(const Model<T>& M, const S
 
 // Reverse of one world's step: adjoints of the state at the step's end in M.stateAdj become those at its start.
 // Needs the log and integLog that stepWorld wrote for this step, and the bodies' dp/dq of every substep, which
-// it recomputes by replaying the integration from the checkpoint as it goes back. stage: the warp's two
+// it recomputes by replaying the integration from the checkpoint as it goes back. stage: the world's two
 // shared-memory buffers of stageCalls<T>() records each, or null to read every record from the log. bodies:
-// the warp's shared-memory body arrays (sharedBodies) holding the world's adjoint state, or null to use the
+// the world's shared-memory body arrays (sharedBodies) holding the world's adjoint state, or null to use the
 // global arrays.
 template <class T>
-__device__ void stepWorldAdj(const Model<T>& M, const Slot<T>& W, int step, uint32_t w, const T* in, const T* log,
+__device__ void stepWorldAdjWarp(const Model<T>& M, const Slot<T>& W, int step, uint32_t w, const T* in, const T* log,
                              const T* integLog, uint64_t calls, T* stage, T* bodies, uint32_t bodyCap) {
     constexpr int kStage = stageCalls<T>();
     const uint32_t lane = threadIdx.x & 31;
@@ -1146,9 +1585,9 @@ __device__ void stepWorldAdj(const Model<T>& M, const Slot<T>& W, int step, uint
                 auto staged = [&](int k) { return stage != nullptr && L.start[k + 1] - L.start[k] <= (uint32_t)kStage; };
                 auto fetch = [&](int k, int buffer) {
                     if (staged(k)) {
-                        copyToShared(stage + buffer * kStage * kCallWords, records(k), (L.start[k + 1] - L.start[k]) * kCallWords, lane);
+                        copyToShared(stage + buffer * kStage * kCallWords, records(k), (L.start[k + 1] - L.start[k]) * kCallWords, lane, 32);
                     } else {
-                        prefetchRange(records(k), records(k + 1), lane);
+                        prefetchRange(records(k), records(k + 1), lane, 32);
                     }
                     // Its contacts are read one per lane: ask for their lines too.
                     for (uint32_t x = L.start[k] + lane; x < L.start[k + 1]; x += 32) {
@@ -1250,6 +1689,253 @@ __device__ void stepWorldAdj(const Model<T>& M, const Slot<T>& W, int step, uint
     __syncwarp();
 }
 
+// The same with a CTA a world and four lanes a contact (quadOpAdj).
+template <class T>
+__device__ void stepWorldAdj(const Model<T>& M, const Slot<T>& W, int step, uint32_t w, const T* in, const T* log,
+                             const T* integLog, uint64_t calls, T* stage, T* bodies, uint32_t bodyCap) {
+    constexpr int kStage = stageCalls<T>();
+    const uint32_t tid = threadIdx.x;
+    constexpr uint32_t kThreads = kWalkThreads;
+    const WorldView V = viewOf(M.S, step, w);
+    const int n = M.S.substeps;
+    const uint32_t cf = V.tw->contactFirst;
+    const BodyArrays<T> B = bodies ? sharedBodies(bodies, bodyCap) : globalBodies(M, W, V.bodyFirst);
+    // The step's adjoint accumulators start at zero; the inverse masses and inertias the recomputation found.
+    for (uint32_t i = tid; i < V.bodyCount; i += kThreads) {
+        st3(B.dpAdj + 3 * i, zeroV<T>());
+        st4(B.dqAdj + 4 * i, Q4<T>{ 0, 0, 0, 0 });
+        st4(B.qBaseAdj + 4 * i, Q4<T>{ 0, 0, 0, 0 });
+        B.invMAdj[i] = 0;
+        stM(B.invIAdj + 9 * i, zeroM<T>());
+        if (bodies) {
+            const uint32_t g = V.bodyFirst + i;
+            B.invM[i] = W.invM[g];
+            for (int k = 0; k < 9; ++k) { B.invI[9 * i + k] = W.invI[9 * (size_t)g + k]; }
+        }
+    }
+    for (uint32_t ci = tid; ci < V.tw->contactCount; ci += kThreads) {
+        for (int i = 0; i < 4; ++i) { M.pointAdj[(size_t)(cf + ci) * 4 + i] = PointState<T>{ 0, zeroV<T>(), 0 }; }
+        M.muAdj[cf + ci] = 0;
+    }
+    __syncthreads();
+    // dp and dq a body had during substep `sub`'s passes: before its position update (warm start, biased
+    // solve) or after it (relax, restitution), from the integration log of the recomputed step.
+    auto setDisplacement = [&](int sub, bool afterUpdate) {
+        for (uint32_t i = tid; i < V.bodyCount; i += kThreads) {
+            const uint32_t g = V.bodyFirst + i;
+            const int k = afterUpdate ? sub : sub - 1;  // the last position update before the pass
+            if (!movesIn(M, V, g) || k < 0) {
+                st3(B.dp + 3 * i, zeroV<T>());
+                st4(B.dq + 4 * i, Q4<T>{ 0, 0, 0, 1 });
+                continue;
+            }
+            const T* L = integLog + ((size_t)k * M.S.totalBodies + g) * kIntegWords;
+            const Q4<T> qb = ld4(in + (size_t)g * kState + 3);
+            st3(B.dp + 3 * i, ld3(L + 7));
+            st4(B.dq + 4 * i, qmul(integrateQ(ld4(L), ld3(L + 4), M.h), conj(qb)));
+        }
+        __syncthreads();
+    };
+    uint64_t cursor = calls;  // one past the last call of the step
+    // One operation on contact ci (none when `on` is false) by its four lanes; every lane of the warp calls it.
+    auto opAdj = [&](int op, bool on, uint32_t ci, const T* rec) {
+        const uint32_t q = tid & 3;
+        const TapeContact& tc = V.contacts[on ? ci : 0];
+        const int n = on ? tc.count : 0;
+        const int most = (int)__reduce_max_sync(0xffffffffu, (uint32_t)n);
+        if (most == 0) { return; }
+        const uint32_t ia = on ? tc.a : 0, ib = on ? tc.b : 0, ga = V.bodyFirst + ia, gb = V.bodyFirst + ib;
+        SBody<T> a, b;
+        a.v = a.w = b.v = b.w = zeroV<T>();  // the reverse reads no velocity
+        a.dp = ld3(B.dp + 3 * ia), a.dq = ld4(B.dq + 4 * ia), a.im = B.invM[ia];
+        a.I = ldM(B.invI + 9 * ia), a.moves = movesIn(M, V, ga);
+        b.dp = ld3(B.dp + 3 * ib), b.dq = ld4(B.dq + 4 * ib), b.im = B.invM[ib];
+        b.I = ldM(B.invI + 9 * ib), b.moves = movesIn(M, V, gb);
+        T* sa = B.stateAdj + ia * kState;
+        T* sb = B.stateAdj + ib * kState;
+        BodyAdj<T> gA{ zeroV<T>(), zeroV<T>(), zeroV<T>(), Q4<T>{ 0, 0, 0, 0 }, 0, zeroM<T>() };
+        BodyAdj<T> gB = gA;
+        // Moving bodies belong to this contact alone within its color: their adjoints are read and written in
+        // place. Anchored bodies are shared: their contributions are added atomically.
+        if (a.moves) { gA.v = ld3(sa + 7), gA.w = ld3(sa + 10); }
+        if (b.moves) { gB.v = ld3(sb + 7), gB.w = ld3(sb + 10); }
+        PointState<T>* gp = M.pointAdj + (size_t)(cf + ci) * 4 + q;
+        PointState<T> g{ 0, zeroV<T>(), 0 };
+        if ((int)q < n) { g = *gp; }
+        T muG = 0;
+        const T mu = on ? contactFriction(M, V, tc) : T(0);
+        quadOpAdj(M, op, a, b, tc, n, most, mu, gA, gB, g, muG, rec);
+        if ((int)q < n) { *gp = g; }
+        // The lanes' shares.
+        auto sum = [&](BodyAdj<T>& G) {
+            G.dp = { quadSum(G.dp.x), quadSum(G.dp.y), quadSum(G.dp.z) };
+            G.dq = { quadSum(G.dq.x), quadSum(G.dq.y), quadSum(G.dq.z), quadSum(G.dq.w) };
+            G.im = quadSum(G.im);
+            for (int r = 0; r < 3; ++r) { G.I.r[r] = { quadSum(G.I.r[r].x), quadSum(G.I.r[r].y), quadSum(G.I.r[r].z) }; }
+        };
+        sum(gA);
+        sum(gB);
+        muG = quadSum(muG);
+        auto put = [&](bool moves, uint32_t i, uint32_t gi, T* s, const BodyAdj<T>& G) {
+            if (moves) {
+                st3(s + 7, G.v);
+                st3(s + 10, G.w);
+                st3(B.dpAdj + 3 * i, ld3(B.dpAdj + 3 * i) + G.dp);
+                st4(B.dqAdj + 4 * i, qadd(ld4(B.dqAdj + 4 * i), G.dq));
+                B.invMAdj[i] += G.im;
+                T* I = B.invIAdj + 9 * i;
+                for (int r = 0; r < 3; ++r) { I[3 * r] += G.I.r[r].x, I[3 * r + 1] += G.I.r[r].y, I[3 * r + 2] += G.I.r[r].z; }
+            } else if (M.S.dynamic[gi]) {
+                // A sleeping dynamic body: its velocity carries back to steps where it moved. A static body's
+                // never changes, so nothing is added for it.
+                atomicAddT(s + 7, G.v.x), atomicAddT(s + 8, G.v.y), atomicAddT(s + 9, G.v.z);
+                atomicAddT(s + 10, G.w.x), atomicAddT(s + 11, G.w.y), atomicAddT(s + 12, G.w.z);
+            }
+        };
+        if (n > 0 && q == 0) { put(a.moves, ia, ga, sa, gA); }
+        if (n > 0 && q == 1) { put(b.moves, ib, gb, sb, gB); }
+        if (n > 0 && q == 2 && muG != T(0)) { M.muAdj[cf + ci] += muG; }
+    };
+    auto passAdj = [&](int op) {
+        PassList lists[4];
+        const int nl = passLists(V, op, lists);
+        for (int l = nl - 1; l >= 0; --l) {
+            const PassList& L = lists[l];
+            if (L.start) {
+                const uint32_t first = L.start[0];
+                cursor -= L.start[L.count] - first;
+                // Color k's records, consecutive in the log. A color that fits a stage buffer is copied to shared
+                // memory while the color before it in the walk runs; a larger one is read where it lies.
+                auto records = [&](int k) { return log + (cursor + (L.start[k] - first)) * kCallWords; };
+                auto staged = [&](int k) { return stage != nullptr && L.start[k + 1] - L.start[k] <= (uint32_t)kStage; };
+                auto fetch = [&](int k, int buffer) {
+                    if (staged(k)) {
+                        copyToShared(stage + buffer * kStage * kCallWords, records(k), (L.start[k + 1] - L.start[k]) * kCallWords, tid, kThreads);
+                    } else {
+                        prefetchRange(records(k), records(k + 1), tid, kThreads);
+                    }
+                    // Its contacts' lines too.
+                    for (uint32_t x = L.start[k] + tid; x < L.start[k + 1]; x += kThreads) {
+                        const char* tc = reinterpret_cast<const char*>(V.contacts + L.list[x]);
+                        asm volatile("prefetch.global.L1 [%0];" ::"l"(tc));
+                        asm volatile("prefetch.global.L1 [%0];" ::"l"(tc + sizeof(TapeContact) - 1));
+                    }
+                };
+                if (L.count > 0) { fetch((int)L.count - 1, 0); }
+                for (int k = (int)L.count - 1; k >= 0; --k) {
+                    const int buffer = ((int)L.count - 1 - k) & 1;
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    __syncthreads();
+                    if (k > 0) { fetch(k - 1, buffer ^ 1); }
+                    const T* base = staged(k) ? stage + buffer * kStage * kCallWords : records(k);
+                    for (uint32_t x = L.start[k] + tid / 32 * 8; x < L.start[k + 1]; x += kThreads / 4) {
+                        const uint32_t mine = x + (tid & 31) / 4;
+                        const bool on = mine < L.start[k + 1];
+                        opAdj(op, on, on ? L.list[mine] : 0u, base + (mine - L.start[k]) * kCallWords);
+                    }
+                    __syncthreads();
+                }
+            } else {
+                cursor -= L.count;
+                if (tid < 32) {
+                    for (int x = (int)L.count - 1; x >= 0; --x) {
+                        opAdj(op, tid < 4, L.list[x], log + (cursor + (uint64_t)x) * kCallWords);
+                        __syncwarp();
+                    }
+                }
+                __syncthreads();
+            }
+        }
+    };
+    setDisplacement(n - 1, true);
+    passAdj(kRestitute);
+    for (int sub = n - 1; sub >= 0; --sub) {
+        setDisplacement(sub, true);
+        passAdj(kRelax);
+        // Position update in reverse.
+        for (uint32_t i = tid; i < V.bodyCount; i += kThreads) {
+            const uint32_t g = V.bodyFirst + i;
+            if (!movesIn(M, V, g)) { continue; }
+            T* s = B.stateAdj + i * kState;
+            const T* L = integLog + ((size_t)sub * M.S.totalBodies + g) * kIntegWords;
+            const Q4<T> q = ld4(L);
+            const V3<T> wv = ld3(L + 4);
+            const Q4<T> nq = integrateQ(q, wv, M.h);
+            const Q4<T> qb = ld4(in + (size_t)g * kState + 3);
+            // dq' = q' qBase*: its adjoint goes to q' and to qBase.
+            const Q4<T> dqG = ld4(B.dqAdj + 4 * i);
+            Q4<T> qG = qadd(ld4(s + 3), qmulAdjA(dqG, conj(qb)));
+            const Q4<T> cG = qmulAdjB(dqG, nq);
+            st4(B.qBaseAdj + 4 * i, qadd(ld4(B.qBaseAdj + 4 * i), Q4<T>{ -cG.x, -cG.y, -cG.z, cG.w }));
+            st4(B.dqAdj + 4 * i, Q4<T>{ 0, 0, 0, 0 });
+            Q4<T> qPrevG{ 0, 0, 0, 0 };
+            V3<T> wG = ld3(s + 10);
+            integrateQAdj(q, wv, M.h, qG, qPrevG, wG);
+            st4(s + 3, qPrevG);
+            st3(s + 10, wG);
+            // com' = com + v h and dp' = dp + v h.
+            const V3<T> vG = ld3(s + 7) + ld3(s) * M.h + ld3(B.dpAdj + 3 * i) * M.h;
+            st3(s + 7, vG);
+        }
+        __syncthreads();
+        setDisplacement(sub, false);
+        passAdj(kBias);
+        passAdj(kWarm);
+        // Velocity update in reverse.
+        for (uint32_t i = tid; i < V.bodyCount; i += kThreads) {
+            const uint32_t g = V.bodyFirst + i;
+            if (!movesIn(M, V, g)) { continue; }
+            T* s = B.stateAdj + i * kState;
+            st3(s + 7, ld3(s + 7) * (T(1) / (T(1) + M.h * T(M.S.linearDamping[g]))));
+            st3(s + 10, ld3(s + 10) * (T(1) / (T(1) + M.h * T(M.S.angularDamping[g]))));
+        }
+        __syncthreads();
+    }
+    // Step start in reverse: qBase = q, the world inverse inertia r L r^T and the inverse mass 1/m.
+    for (uint32_t i = tid; i < V.bodyCount; i += kThreads) {
+        const uint32_t g = V.bodyFirst + i;
+        T* s = B.stateAdj + i * kState;
+        st4(s + 3, qadd(ld4(s + 3), ld4(B.qBaseAdj + 4 * i)));
+        if (!movesIn(M, V, g)) { continue; }
+        const Q4<T> q = ld4(in + (size_t)g * kState + 3);
+        const T m = M.mass[g];
+        const T scale = T(M.S.mass[g]) / m;
+        M3<T> L;
+        for (int a = 0; a < 3; ++a) {
+            L.r[a] = { T(M.S.invInertiaLocal[9 * g + 3 * a]) * scale, T(M.S.invInertiaLocal[9 * g + 3 * a + 1]) * scale,
+                       T(M.S.invInertiaLocal[9 * g + 3 * a + 2]) * scale };
+        }
+        const M3<T> r = toMat3(q);
+        const M3<T> G = ldM(B.invIAdj + 9 * i);
+        // I = r L r^T: dr = G r L^T + G^T r L, dL = r^T G r.
+        const M3<T> rG = madd(mmul(G, mmul(r, transposeM(L))), mmul(transposeM(G), mmul(r, L)));
+        const M3<T> LG = mmul(transposeM(r), mmul(G, r));
+        T lG = 0;  // sum of dL_ij L_ij, for the mass
+        for (int a = 0; a < 3; ++a) { lG += dot(LG.r[a], L.r[a]); }
+        st4(s + 3, qadd(ld4(s + 3), toMat3Adj(q, rG)));
+        // im = 1/m and L = L0 m0 / m: both scale as 1/m.
+        M.massAdj[g] += -(B.invMAdj[i] / (m * m)) - lG / m;
+    }
+    // The contacts' friction to the shapes', a thread a shape over the contacts in order, so that the sums come out the
+    // same every time. mu = sqrt(fa fb): d mu / d fa = fb / (2 mu).
+    const uint32_t shapes = (w + 1 < (uint32_t)M.S.nWorlds ? M.S.shapeFirst[w + 1] : M.S.totalShapes) - V.shapeFirst;
+    for (uint32_t i = tid; i < shapes; i += kThreads) {
+        T g = 0;
+        for (uint32_t ci = 0; ci < V.tw->contactCount; ++ci) {
+            const TapeContact& tc = V.contacts[ci];
+            if (tc.shapeA != i && tc.shapeB != i) { continue; }
+            const T muG = M.muAdj[cf + ci];
+            if (muG == T(0)) { continue; }
+            const T mu = contactFriction(M, V, tc);
+            if (!(mu > T(0))) { continue; }
+            if (tc.shapeA == i) { g += muG * M.friction[V.shapeFirst + tc.shapeB] / (T(2) * mu); }
+            if (tc.shapeB == i) { g += muG * M.friction[V.shapeFirst + tc.shapeA] / (T(2) * mu); }
+        }
+        if (g != T(0)) { M.frictionAdj[V.shapeFirst + i] += g; }
+    }
+    __syncthreads();
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // Kernels: one warp per world, every step of the run.
 
@@ -1278,9 +1964,37 @@ __global__ void __launch_bounds__(128) k_model_forward(const __grid_constant__ M
     }
 }
 
+// The same with a CTA a world.
+template <class T>
+__global__ void __launch_bounds__(kWalkThreads, 2) k_model_forward_wide(const __grid_constant__ Model<T> M) {
+    __shared__ unsigned long long s_sig[kWalkThreads / 32];
+    const uint32_t w = blockIdx.x, tid = threadIdx.x;
+    const uint32_t b0 = M.S.bodyFirst[w], nb = M.S.bodyCount[w];
+    for (uint32_t k = tid; k < nb * kState; k += kWalkThreads) {
+        M.states[(size_t)b0 * kState + k] = M.init[(size_t)b0 * kState + k];
+    }
+    __syncthreads();
+    const size_t stride = (size_t)M.S.totalBodies * kState;
+    const Slot<T> W = slotOf(M, 0);
+    unsigned long long sig = 0;
+    for (int s = 0; s < M.S.nSteps; ++s) {
+        stepWorldWide<T>(M, W, s, w, M.states + s * stride, M.states + (s + 1) * stride, M.branches ? &sig : nullptr);
+        __syncthreads();
+    }
+    if (M.branches) {
+        for (int o = 16; o > 0; o >>= 1) { sig += __shfl_xor_sync(0xffffffffu, sig, o); }
+        if ((tid & 31) == 0) { s_sig[tid / 32] = sig; }
+        __syncthreads();
+        if (tid == 0) {
+            for (uint32_t k = 1; k < kWalkThreads / 32; ++k) { sig += s_sig[k]; }
+            M.branches[w] = sig;
+        }
+    }
+}
+
 // The backward runs chunk by chunk from the last step. Recomputing a step needs only its checkpoint, so a
 // chunk's steps are recomputed all at once, one warp per world and step, each logging into its own slot; then
-// one warp per world walks the chunk's steps in reverse from those logs, carrying the adjoints back.
+// one warp or CTA per world walks the chunk's steps in reverse from those logs, carrying the adjoints back.
 template <class T>
 __global__ void __launch_bounds__(128) k_model_recompute(const __grid_constant__ Model<T> M, int first, int count,
                                                          uint32_t slotBase) {
@@ -1295,10 +2009,10 @@ __global__ void __launch_bounds__(128) k_model_recompute(const __grid_constant__
 }
 
 template <class T>
-__host__ __device__ constexpr size_t stageBytesPerWarp() { return 2 * (size_t)stageCalls<T>() * kCallWords * sizeof(T); }
+__host__ __device__ constexpr size_t stageBytes() { return 2 * (size_t)stageCalls<T>() * kCallWords * sizeof(T); }
 
 template <class T>
-__host__ __device__ constexpr size_t bodyBytesPerWarp(uint32_t cap) {
+__host__ __device__ constexpr size_t bodyBytes(uint32_t cap) {
     return ((size_t)cap * kBodyWords * sizeof(T) + 15) / 16 * 16;
 }
 
@@ -1312,10 +2026,10 @@ __global__ void __launch_bounds__(128) k_model_reverse(const __grid_constant__ M
     const uint32_t w = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (w >= (uint32_t)M.S.nWorlds) { return; }
     const uint32_t lane = threadIdx.x & 31;
-    const size_t stageBytes = staged ? stageBytesPerWarp<T>() : 0;
-    unsigned char* mine = area + (threadIdx.x / 32) * (stageBytes + bodyBytesPerWarp<T>(bodyCap));
+    const size_t stages = staged ? stageBytes<T>() : 0;
+    unsigned char* mine = area + (threadIdx.x / 32) * (stages + bodyBytes<T>(bodyCap));
     T* stage = staged ? reinterpret_cast<T*>(mine) : nullptr;
-    T* bodies = bodyCap ? reinterpret_cast<T*>(mine + stageBytes) : nullptr;
+    T* bodies = bodyCap ? reinterpret_cast<T*>(mine + stages) : nullptr;
     const uint32_t b0 = M.S.bodyFirst[w], nb = M.S.bodyCount[w];
     if (bodies) {
         T* adj = sharedBodies(bodies, bodyCap).stateAdj;
@@ -1332,13 +2046,47 @@ __global__ void __launch_bounds__(128) k_model_reverse(const __grid_constant__ M
         const uint64_t colored = tw.colorStart[tw.colorCount] + tw.restCount;
         const uint64_t impact = tw.impactColorStart[tw.impactColorCount] + tw.impactRestCount;
         const uint64_t calls = (uint64_t)M.S.substeps * (3 * colored + 2 * impact) + colored;
-        stepWorldAdj(M, W, s, w, M.states + s * stride, W.log + (size_t)w * M.logStride, W.integLog, calls, stage,
+        stepWorldAdjWarp(M, W, s, w, M.states + s * stride, W.log + (size_t)w * M.logStride, W.integLog, calls, stage,
                      bodies, bodyCap);
         __syncwarp();
     }
     if (bodies) {
         const T* adj = sharedBodies(bodies, bodyCap).stateAdj;
         for (uint32_t k = lane; k < nb * kState; k += 32) { M.stateAdj[(size_t)b0 * kState + k] = adj[k]; }
+    }
+}
+
+// The same walk with a CTA a world. The dynamic shared memory holds, when `staged`, the two stage buffers and, when bodyCap is not zero, body arrays for up to bodyCap bodies
+// (no world has more).
+template <class T>
+__global__ void __launch_bounds__(kWalkThreads, 2) k_model_reverse_wide(const __grid_constant__ Model<T> M, int first, int count,
+                                                                           uint32_t slotBase, int staged, uint32_t bodyCap) {
+    extern __shared__ __align__(16) unsigned char area[];
+    const uint32_t w = blockIdx.x;
+    T* stage = staged ? reinterpret_cast<T*>(area) : nullptr;
+    T* bodies = bodyCap ? reinterpret_cast<T*>(area + (staged ? stageBytes<T>() : 0)) : nullptr;
+    const uint32_t b0 = M.S.bodyFirst[w], nb = M.S.bodyCount[w];
+    if (bodies) {
+        T* adj = sharedBodies(bodies, bodyCap).stateAdj;
+        for (uint32_t k = threadIdx.x; k < nb * kState; k += kWalkThreads) { adj[k] = M.stateAdj[(size_t)b0 * kState + k]; }
+        __syncthreads();
+    }
+    const size_t stride = (size_t)M.S.totalBodies * kState;
+    for (int k = count - 1; k >= 0; --k) {
+        const int s = first + k;
+        const Slot<T> W = slotOf(M, slotBase + (uint32_t)k);
+        // The number of contact operations the step logged: every pass walks its lists once.
+        const WorldView V = viewOf(M.S, s, w);
+        const TapeWorld& tw = *V.tw;
+        const uint64_t colored = tw.colorStart[tw.colorCount] + tw.restCount;
+        const uint64_t impact = tw.impactColorStart[tw.impactColorCount] + tw.impactRestCount;
+        const uint64_t calls = (uint64_t)M.S.substeps * (3 * colored + 2 * impact) + colored;
+        stepWorldAdj(M, W, s, w, M.states + s * stride, W.log + (size_t)w * M.logStride, W.integLog, calls, stage,
+                     bodies, bodyCap);
+    }
+    if (bodies) {
+        const T* adj = sharedBodies(bodies, bodyCap).stateAdj;
+        for (uint32_t k = threadIdx.x; k < nb * kState; k += kWalkThreads) { M.stateAdj[(size_t)b0 * kState + k] = adj[k]; }
     }
 }
 
@@ -1355,9 +2103,19 @@ struct Run {
     void* states = nullptr;
     void *invM = nullptr, *invI = nullptr, *dp = nullptr, *dq = nullptr, *qBase = nullptr, *points = nullptr;
     void *stateAdj = nullptr, *dpAdj = nullptr, *dqAdj = nullptr, *qBaseAdj = nullptr, *invMAdj = nullptr,
-         *invIAdj = nullptr, *pointAdj = nullptr, *massAdj = nullptr, *frictionAdj = nullptr, *log = nullptr,
+         *invIAdj = nullptr, *pointAdj = nullptr, *muAdj = nullptr, *massAdj = nullptr, *frictionAdj = nullptr, *log = nullptr,
          *integLog = nullptr, *scratch = nullptr, *branches = nullptr;
     uint64_t logStride = 0;
+    // What the buffers were allocated for; a run of the same sizes keeps them (allocating and freeing up to half the
+    // device's memory took 23 ms of a forward and 15 of a backward on 256 impact worlds x 48 steps).
+    struct Sizes {
+        size_t elem, bodies, shapes, slots, worlds, steps, substeps;
+        uint64_t calls;
+        bool operator==(const Sizes& o) const {
+            return elem == o.elem && bodies == o.bodies && shapes == o.shapes && slots == o.slots && worlds == o.worlds &&
+                   steps == o.steps && substeps == o.substeps && calls == o.calls;
+        }
+    } sizes{};
     int slots = 0;  // steps the backward recomputes at once; two sets of slots alternate
     uint32_t maxBodies = 0;  // the most bodies of a world, read once
     bool forwardDone = false;
@@ -1385,10 +2143,11 @@ struct Run {
         for (void* p : owned) { cudaFree(p); }
         owned.clear();
         for (void** p : { &mass, &friction, &init, &states, &invM, &invI, &dp, &dq, &qBase, &points, &stateAdj, &dpAdj,
-                          &dqAdj, &qBaseAdj, &invMAdj, &invIAdj, &pointAdj, &massAdj, &frictionAdj, &log, &integLog,
+                          &dqAdj, &qBaseAdj, &invMAdj, &invIAdj, &pointAdj, &muAdj, &massAdj, &frictionAdj, &log, &integLog,
                           &scratch, &branches }) {
             *p = nullptr;
         }
+        sizes = Sizes{};
         forwardDone = false;
         slots = 0;
         maxBodies = 0;
@@ -1436,6 +2195,7 @@ Model<T> modelOf(const AdjointSetup& S, Run& r) {
     M.invMAdj = (T*)r.invMAdj;
     M.invIAdj = (T*)r.invIAdj;
     M.pointAdj = (PointState<T>*)r.pointAdj;
+    M.muAdj = (T*)r.muAdj;
     M.massAdj = (T*)r.massAdj;
     M.frictionAdj = (T*)r.frictionAdj;
     M.log = (T*)r.log;
@@ -1463,23 +2223,51 @@ int download(std::vector<double>& dst, const void* src, size_t n, cudaStream_t s
     return TF_OK;
 }
 
+// Worlds an SM up to which the walks in double give a world a CTA and a contact four lanes (measured at backwardT).
+constexpr int kWideWorlds = 4;
+
+// The largest number of contact operations one world logs in one step.
+int maxCalls(const AdjointSetup& S, uint64_t* out) {
+    std::vector<TapeStep> steps(S.nSteps);
+    TF_ADJ_CUDA(cudaMemcpy(steps.data(), S.steps, steps.size() * sizeof(TapeStep), cudaMemcpyDeviceToHost));
+    std::vector<TapeWorld> tw(S.nWorlds);
+    uint64_t most = 1;
+    for (const TapeStep& ts : steps) {
+        TF_ADJ_CUDA(cudaMemcpy(tw.data(), ts.worlds, tw.size() * sizeof(TapeWorld), cudaMemcpyDeviceToHost));
+        for (const TapeWorld& w : tw) {
+            const uint64_t colored = w.colorStart[w.colorCount] + w.restCount;
+            const uint64_t impact = w.impactColorStart[w.impactColorCount] + w.impactRestCount;
+            most = std::max<uint64_t>(most, (uint64_t)S.substeps * (3 * colored + 2 * impact) + colored);
+        }
+    }
+    *out = most;
+    return TF_OK;
+}
+
 template <class T>
 int forwardT(Run& r, const AdjointSetup& S, cudaStream_t stream, const double* init, const double* mass,
              const double* friction, double* finalState) {
     const size_t nb = S.totalBodies, ns = S.totalShapes;
-    r.release();
-    r.elem = sizeof(T);
     int rc;
+    uint64_t calls = 0;
+    if ((rc = maxCalls(S, &calls)) != TF_OK) { return rc; }
+    const Run::Sizes sizes{ sizeof(T), nb, ns, S.contactSlots, (size_t)S.nWorlds, (size_t)S.nSteps, (size_t)S.substeps, calls };
+    if (!(sizes == r.sizes)) { r.release(); }
+    r.forwardDone = false;
+    r.maxBodies = 0;
+    r.elem = sizeof(T);
     const size_t stateBytes = nb * kState * sizeof(T);
-    if ((rc = r.alloc(&r.mass, nb * sizeof(T))) || (rc = r.alloc(&r.friction, ns * sizeof(T))) ||
+    if (!r.states && ((rc = r.alloc(&r.mass, nb * sizeof(T))) || (rc = r.alloc(&r.friction, ns * sizeof(T))) ||
         (rc = r.alloc(&r.init, stateBytes)) || (rc = r.alloc(&r.states, stateBytes * (size_t)(S.nSteps + 2))) ||
         (rc = r.alloc(&r.invM, nb * sizeof(T))) || (rc = r.alloc(&r.invI, 9 * nb * sizeof(T))) ||
         (rc = r.alloc(&r.dp, 3 * nb * sizeof(T))) || (rc = r.alloc(&r.dq, 4 * nb * sizeof(T))) ||
         (rc = r.alloc(&r.qBase, 4 * nb * sizeof(T))) ||
         (rc = r.alloc(&r.points, (size_t)S.contactSlots * 4 * sizeof(PointState<T>))) ||
-        (rc = r.alloc(&r.branches, (size_t)S.nWorlds * sizeof(unsigned long long)))) {
+        (rc = r.alloc(&r.branches, (size_t)S.nWorlds * sizeof(unsigned long long))))) {
+        r.release();
         return rc;
     }
+    r.sizes = sizes;
     // Parameters: the caller's, else the recorded ones.
     std::vector<double> h(nb * kState);
     {
@@ -1514,8 +2302,21 @@ int forwardT(Run& r, const AdjointSetup& S, cudaStream_t stream, const double* i
     TF_ADJ_CUDA(cudaEventCreate(&e0));
     TF_ADJ_CUDA(cudaEventCreate(&e1));
     cudaEventRecord(e0, stream);
-    const int blocks = (S.nWorlds + 3) / 4;
-    k_model_forward<T><<<blocks, 128, 0, stream>>>(M);
+    int device = 0, sms = 0;
+    TF_ADJ_CUDA(cudaGetDevice(&device));
+    TF_ADJ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    // In double, few worlds get a CTA each and a contact four lanes (24 impact worlds 2.82 -> 1.34 ms a step, 256 worlds
+    // 2.75 -> 1.59). In float the same rows compile to other contractions of multiplies and adds, which the contacts
+    // amplify into another trajectory; there a world keeps its warp.
+    bool wide = false;
+    if constexpr (sizeof(T) == 8) {
+        wide = S.nWorlds <= kWideWorlds * sms;
+        if (wide) { k_model_forward_wide<T><<<S.nWorlds, kWalkThreads, 0, stream>>>(M); }
+    }
+    if (!wide) {
+        const int perCta = S.nWorlds <= 4 * sms ? 1 : 4;  // few worlds: an SM's L1 for each
+        k_model_forward<T><<<(S.nWorlds + perCta - 1) / perCta, 32 * perCta, 0, stream>>>(M);
+    }
     cudaEventRecord(e1, stream);
     TF_ADJ_CUDA(cudaGetLastError());
     TF_ADJ_CUDA(cudaStreamSynchronize(stream));
@@ -1529,33 +2330,31 @@ int forwardT(Run& r, const AdjointSetup& S, cudaStream_t stream, const double* i
     return TF_OK;
 }
 
-// The largest number of contact operations one world logs in one step.
-int maxCalls(const AdjointSetup& S, uint64_t* out) {
-    std::vector<TapeStep> steps(S.nSteps);
-    TF_ADJ_CUDA(cudaMemcpy(steps.data(), S.steps, steps.size() * sizeof(TapeStep), cudaMemcpyDeviceToHost));
-    std::vector<TapeWorld> tw(S.nWorlds);
-    uint64_t most = 1;
-    for (const TapeStep& ts : steps) {
-        TF_ADJ_CUDA(cudaMemcpy(tw.data(), ts.worlds, tw.size() * sizeof(TapeWorld), cudaMemcpyDeviceToHost));
-        for (const TapeWorld& w : tw) {
-            const uint64_t colored = w.colorStart[w.colorCount] + w.restCount;
-            const uint64_t impact = w.impactColorStart[w.impactColorCount] + w.impactRestCount;
-            most = std::max<uint64_t>(most, (uint64_t)S.substeps * (3 * colored + 2 * impact) + colored);
-        }
-    }
-    *out = most;
-    return TF_OK;
-}
-
 template <class T>
 int backwardT(Run& r, const AdjointSetup& S, cudaStream_t stream, const double* gradFinal, double* gradInit,
               double* gradMass, double* gradFriction) {
     const size_t nb = S.totalBodies, ns = S.totalShapes;
     int rc;
-    uint64_t calls = 0;
-    if ((rc = maxCalls(S, &calls)) != TF_OK) { return rc; }
-    r.logStride = calls * (uint64_t)kCallWords;
-    if (!r.stateAdj) {
+    // A tape recorded again since the forward run: one of other sizes does not fit the run's buffers, one of more
+    // operations a step needs a larger log.
+    Run::Sizes sizes = r.sizes;
+    if ((rc = maxCalls(S, &sizes.calls)) != TF_OK) { return rc; }
+    if (nb != sizes.bodies || ns != sizes.shapes || S.contactSlots != sizes.slots || (size_t)S.nWorlds != sizes.worlds ||
+        (size_t)S.nSteps != sizes.steps || (size_t)S.substeps != sizes.substeps) {
+        return noteError(TF_E_INVALID, "adjoint: the tape was recorded anew since the forward run");
+    }
+    if (sizes.calls > r.sizes.calls && r.log) {
+        r.owned.erase(std::find(r.owned.begin(), r.owned.end(), r.log));
+        cudaFree(r.log);
+        r.log = nullptr;
+        if ((rc = r.alloc(&r.log, 2 * (size_t)r.slots * (size_t)S.nWorlds * sizes.calls * kCallWords * sizeof(T))) != TF_OK) {
+            r.release();
+            return rc;
+        }
+    }
+    r.sizes.calls = std::max(r.sizes.calls, sizes.calls);
+    r.logStride = r.sizes.calls * (uint64_t)kCallWords;
+    if (!r.log) {
         // Steps recomputed at once: as many slots as fit in a share of the free memory, up to the whole run.
         const size_t perSlot = (size_t)S.nWorlds * r.logStride * sizeof(T) +
                                (size_t)S.substeps * nb * kIntegWords * sizeof(T) + nb * (kState + 21) * sizeof(T) +
@@ -1583,9 +2382,11 @@ int backwardT(Run& r, const AdjointSetup& S, cudaStream_t stream, const double* 
             (rc = r.alloc(&r.dqAdj, 4 * nb * sizeof(T))) || (rc = r.alloc(&r.qBaseAdj, 4 * nb * sizeof(T))) ||
             (rc = r.alloc(&r.invMAdj, nb * sizeof(T))) || (rc = r.alloc(&r.invIAdj, 9 * nb * sizeof(T))) ||
             (rc = r.alloc(&r.pointAdj, (size_t)S.contactSlots * 4 * sizeof(PointState<T>))) ||
+            (rc = r.alloc(&r.muAdj, (size_t)S.contactSlots * sizeof(T))) ||
             (rc = r.alloc(&r.massAdj, nb * sizeof(T))) || (rc = r.alloc(&r.frictionAdj, ns * sizeof(T))) ||
             (rc = r.alloc(&r.integLog, k * (size_t)S.substeps * nb * kIntegWords * sizeof(T))) ||
             (rc = r.alloc(&r.log, k * (size_t)S.nWorlds * r.logStride * sizeof(T)))) {
+            r.release();  // also the forward's arrays that gave way
             return rc;
         }
     }
@@ -1610,10 +2411,22 @@ int backwardT(Run& r, const AdjointSetup& S, cudaStream_t stream, const double* 
     cudaEventRecord(r.ready, stream);
     TF_ADJ_CUDA(cudaStreamWaitEvent(r.side, r.ready, 0));
     TF_ADJ_CUDA(cudaStreamWaitEvent(r.walk, r.ready, 0));
-    const int blocks = (S.nWorlds + 3) / 4;
-    // Each warp of the reverse walk stages color batches in shared memory when the device grants the space
-    // (set on every call: the attribute belongs to the current device).
-    // Each warp of the reverse walk stages color batches and its world's body arrays in shared memory when the
+    // A world's reverse walk is one dependent chain. In double, few worlds get a CTA each and a contact four lanes: 24
+    // impact worlds take 2.92 ms a step of the walk and 9.00 with a warp a world (whose variant spills), 256 worlds 3.88
+    // and 9.49; past what stays resident at once a warp a world has half the instructions. In float the wide walk is
+    // faster too (256 worlds 2.64 and 4.58), but its sums round otherwise, which ill-conditioned worlds amplify: of 60
+    // impact worlds x 48 steps the friction gradients came out 2.5e-5 apart; float keeps the order of a lane
+    // a contact.
+    int device = 0, sms = 0;
+    TF_ADJ_CUDA(cudaGetDevice(&device));
+    TF_ADJ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    constexpr bool kDouble = sizeof(T) == 8;
+    const bool wide = kDouble && S.nWorlds <= kWideWorlds * sms;
+    const int perCta = wide || S.nWorlds <= 4 * sms ? 1 : 4;  // worlds; few worlds: an SM's L1 for each
+    const void* walkFn = (const void*)k_model_reverse<T>;
+    if constexpr (kDouble) { walkFn = wide ? (const void*)k_model_reverse_wide<T> : walkFn; }
+    const int walkThreads = wide ? (int)kWalkThreads : 32 * perCta;
+    // The walk stages color batches and its world's body arrays in shared memory when the
     // device grants the space and that leaves as many worlds resident at once as the walk can have at all (it
     // is one dependent chain per world: worlds beyond those wait for a second wave); else the body arrays, or
     // both, stay in global memory. The attribute is set on every call: it belongs to the current device.
@@ -1622,29 +2435,26 @@ int backwardT(Run& r, const AdjointSetup& S, cudaStream_t stream, const double* 
         TF_ADJ_CUDA(cudaMemcpy(counts.data(), S.bodyCount, counts.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost));
         r.maxBodies = std::max<uint32_t>(1, *std::max_element(counts.begin(), counts.end()));
     }
-    int device = 0, sms = 0;
-    TF_ADJ_CUDA(cudaGetDevice(&device));
-    TF_ADJ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     auto walkBytes = [&](int option) {  // 0: records and bodies staged, 1: records only, 2: nothing
-        return 4 * ((option < 2 ? stageBytesPerWarp<T>() : 0) + bodyBytesPerWarp<T>(option == 0 ? r.maxBodies : 0));
+        return perCta * ((option < 2 ? stageBytes<T>() : 0) + bodyBytes<T>(option == 0 ? r.maxBodies : 0));
     };
     int perSm[3] = { 0, 0, 0 };
     for (int option = 0; option < 3; ++option) {
         const size_t bytes = walkBytes(option);
-        if (cudaFuncSetAttribute(k_model_reverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm[option], k_model_reverse<T>, 128, bytes) != cudaSuccess) {
+        if (cudaFuncSetAttribute(walkFn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm[option], walkFn, walkThreads, bytes) != cudaSuccess) {
             cudaGetLastError();
             perSm[option] = 0;
         }
     }
     // CTAs per SM that hold every world at once, or as many as any option allows.
-    const int wanted = std::min<int>((S.nWorlds + 4 * sms - 1) / (4 * sms), std::max({ perSm[0], perSm[1], perSm[2] }));
+    const int wanted = std::min<int>((S.nWorlds + perCta * sms - 1) / (perCta * sms), std::max({ perSm[0], perSm[1], perSm[2] }));
     int option = 2;
     while (option > 0 && perSm[option - 1] >= std::max(wanted, 1)) { --option; }  // less shared memory, more CTAs
     const int staged = option < 2 ? 1 : 0;
     const uint32_t bodyCap = option == 0 ? r.maxBodies : 0;
     const size_t walkShared = walkBytes(option);
-    if (cudaFuncSetAttribute(k_model_reverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walkShared) != cudaSuccess) {
+    if (cudaFuncSetAttribute(walkFn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walkShared) != cudaSuccess) {
         return noteError(TF_E_CUDA, "adjoint: the reverse walk's shared memory was not granted");
     }
     // Chunk c recomputes into slot set c % 2 on the side stream once the reverse walk of chunk c - 2 has left
@@ -1668,7 +2478,15 @@ int backwardT(Run& r, const AdjointSetup& S, cudaStream_t stream, const double* 
         cudaEventRecord(r.recomputed[set], r.side);
         TF_ADJ_CUDA(cudaStreamWaitEvent(r.walk, r.recomputed[set], 0));
         cudaEventRecord(ev[2], r.walk);
-        k_model_reverse<T><<<blocks, 128, walkShared, r.walk>>>(M, first, count, base, staged, bodyCap);
+        if constexpr (kDouble) {
+            if (wide) {
+                k_model_reverse_wide<T><<<S.nWorlds, kWalkThreads, walkShared, r.walk>>>(M, first, count, base, staged, bodyCap);
+            }
+        }
+        if (!wide) {
+            k_model_reverse<T><<<(S.nWorlds + perCta - 1) / perCta, walkThreads, walkShared, r.walk>>>(M, first, count, base,
+                                                                                                       staged, bodyCap);
+        }
         cudaEventRecord(ev[3], r.walk);
         cudaEventRecord(r.reversed[set], r.walk);
         end = first;
