@@ -41,3 +41,24 @@ def test_big_worlds_do_not_depend_on_their_cluster(kind):
                 assert np.array_equal(np.asarray(a[key]).view(np.uint32), np.asarray(b[key]).view(np.uint32)), (copies, key)
         assert np.array_equal(alone[1], other[1])
         assert alone[2:5] == other[2:5]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("copies", [1, 3])
+def test_a_world_at_the_limit_is_not_a_big_one(copies):
+    # 1024 bodies exactly, alone and beside a world that is one body larger: both step as they do alone.
+    def world(bodies):
+        return scenes.planar(n=bodies - 1, cols=24, spheres=0, seed=2, floor="halfspace")
+    at, above = world(1024), world(1025)
+    assert (len(at.bodies), len(above.bodies)) == (1024, 1025)
+    for other in (at, above):
+        got = _run(at, copies, 10), _run(other, copies, 10)
+        batch = Batch([at] * copies + [other] * copies)
+        for _ in range(10):
+            batch.step_checked(float(np.float32(1.0 / 60.0)))
+        for k, alone in ((0, got[0]), (copies, got[1])):
+            state = batch.world_states(k)
+            for key in state:
+                assert np.array_equal(np.asarray(state[key]).view(np.uint32), np.asarray(alone[0][key]).view(np.uint32)), key
+            assert np.array_equal(batch.candidates(k), alone[1])
+        batch.close()

@@ -2108,7 +2108,7 @@ public:
     // (a power of two, at most kMaxCluster and what the device can place), none if that is one.
     int configureBigWorlds() {
         bigCtas = 0;
-        const size_t n = (size_t)(std::upper_bound(sortedSizes.begin(), sortedSizes.end(), kSweepBodies,
+        const size_t n = (size_t)(std::lower_bound(sortedSizes.begin(), sortedSizes.end(), kSweepBodies,
                                                    std::greater<uint32_t>()) - sortedSizes.begin());
         if (n > 0) {
             for (uint32_t ctas = kMaxCluster; ctas >= 2 && bigCtas == 0; ctas /= 2) {
