@@ -574,7 +574,7 @@ struct PairBody {
 };
 
 __device__ __forceinline__ PairBody pairBodyOf(const Batch& B, uint32_t g) {
-    const DBody& b = B.bodies[g];
+    const DBody b = readBody<kBodySolve | kBodyBounds>(B.bodies[g]);
     PairBody p;
     p.lo = b.lo;
     p.hi = b.hi;
@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(kMaxBlock, 1) k_broadphase(const __grid_consta
         if (wi.jointCount > 0) { wakeJointPulled(B, g, wi, wc, nullptr); }
         if (g.tid == 0) { s_count[g.id] = 0; }
         for (uint32_t i = g.tid; i < n; i += g.size) {
-            const DBody& b = B.bodies[wi.bodyFirst + i];
+            const DBody b = readBody<kBodySolve | kBodyPose | kBodyBounds>(B.bodies[wi.bodyFirst + i]);
             const float gr = growthOf(b, P);
             B.grow[wi.bodyFirst + i] = gr;
             if (useStage) {
@@ -2189,7 +2189,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
         }
         for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
             const uint32_t gb = wi.bodyFirst + i;
-            DBody& b = B.bodies[gb];
+            DBody b = readBody<kBodySolve | kBodyMassReads | kBodyCom>(B.bodies[gb]);
             B.struck[gb] = 0;
             if (!b.alive) { continue; }
             b.q0 = b.xf.q;
@@ -2199,6 +2199,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
             b.dp = zero3();
             b.dq = qid();
             updateInverseMass(b);
+            writeBody<kBodySolve | kBodyMassWrites | kBodyBase | kBodyStart>(B.bodies[gb], b);
         }
         g.sync();
         // Joints: what the step will report for them starts over (src/world.cpp:1647).
@@ -2222,8 +2223,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
                     B.cflags[cf + i] = 0;
                     return false;
                 }
-                const DBody& a = B.bodies[cs[i].bodyA];
-                const DBody& b = B.bodies[cs[i].bodyB];
+                const DBody a = readBody<kBodySolve | kBodyPose | kBodyInertia>(B.bodies[cs[i].bodyA]);
+                const DBody b = readBody<kBodySolve | kBodyPose | kBodyInertia>(B.bodies[cs[i].bodyB]);
                 const bool on = (a.type == kDynamic && a.awake) || (b.type == kDynamic && b.awake);
                 uint8_t f = 0;
                 if (on && relativeTravel(a, b, P.dt) > P.tol.speculative) {
@@ -2506,23 +2507,6 @@ struct SBody {
     uint32_t type, awake;
 };
 
-// What integrateVelocity reads and writes (src/world.cpp:1141-1151).
-struct VelBody {
-    uint32_t alive, type, awake;
-    Vec3 v, w, force, torque;
-    float gravityScale, invMass, linearDamping, angularDamping, kept;
-    Mat3 linearProj, angularProj, invInertiaWorld;
-};
-
-// What integratePosition reads and writes (src/world.cpp:1161-1172).
-struct PosBody {
-    uint32_t alive, type, awake;
-    Vec3 v, w, com, dp, localCenter;
-    Quat dq, qBase;
-    Transform xf;
-    float kept;
-};
-
 // Staged words per body: v 0-2, w 3-5, dp 6-8, dq 9-12, type | awake << 8 in 13: what a laned solve reads
 // and writes. The inverse world inertia (torques, contacts solved on their own) stays in global memory, so
 // more bodies fit a slice.
@@ -2605,7 +2589,7 @@ struct SolverStore {
 
     // Copies a body's solver fields from global memory into the store.
     __device__ void stage(uint32_t i) const {
-        const DBody& d = g[i];
+        const DBody d = readBody<kBodySolve>(g[i]);
         at(0, i) = d.v.x, at(1, i) = d.v.y, at(2, i) = d.v.z;
         at(3, i) = d.w.x, at(4, i) = d.w.y, at(5, i) = d.w.z;
         at(6, i) = d.dp.x, at(7, i) = d.dp.y, at(8, i) = d.dp.z;
@@ -2616,68 +2600,51 @@ struct SolverStore {
     // Writes the fields a substep changes back to global memory.
     __device__ void unstage(uint32_t i) const {
         DBody& d = g[i];
-        d.v = { at(0, i), at(1, i), at(2, i) };
-        d.w = { at(3, i), at(4, i), at(5, i) };
-        d.dp = { at(6, i), at(7, i), at(8, i) };
-        d.dq = { at(9, i), at(10, i), at(11, i), at(12, i) };
+        const LanedBody l = loadLaned(i);
+        DBody b;
+        b.v = l.v;
+        b.w = l.w;
+        b.dp = l.dp;
+        b.dq = l.dq;
+        writeBody<(kBodySolve & ~kBodyState)>(d, b);
+        d.dq.w = l.dq.w;
     }
 
     __device__ void integrateVelocityAt(uint32_t i, const StepParams& P) const {
         DBody& d = g[i];
-        if (!d.alive || d.type != kDynamic || !d.awake) { return; }
-        if (!staged) {
-            integrateVelocity(d, P);
-            return;
+        DBody b = readBody<kBodySolve | kBodyInvInertia | kBodyForce | kBodyProj>(d);
+        if (!b.alive || b.type != kDynamic || !b.awake) { return; }
+        if (staged) {
+            b.v = { at(0, i), at(1, i), at(2, i) };
+            b.w = { at(3, i), at(4, i), at(5, i) };
         }
-        VelBody b;
-        b.alive = d.alive;
-        b.type = d.type;
-        b.awake = d.awake;
-        b.v = { at(0, i), at(1, i), at(2, i) };
-        b.w = { at(3, i), at(4, i), at(5, i) };
-        b.force = d.force;
-        b.torque = d.torque;
-        b.gravityScale = d.gravityScale;
-        b.invMass = d.invMass;
-        b.linearDamping = d.linearDamping;
-        b.angularDamping = d.angularDamping;
-        b.kept = d.kept;
-        b.linearProj = d.linearProj;
-        b.angularProj = d.angularProj;
-        b.invInertiaWorld = d.invInertiaWorld;
+        const float kept = b.kept;
         integrateVelocity(b, P);
-        at(0, i) = b.v.x, at(1, i) = b.v.y, at(2, i) = b.v.z;
-        at(3, i) = b.w.x, at(4, i) = b.w.y, at(5, i) = b.w.z;
-        d.kept = b.kept;
+        storeVW(i, b);
+        if (b.kept != kept) { d.kept = b.kept; }
     }
 
     __device__ void integratePositionAt(uint32_t i, const StepParams& P) const {
         DBody& d = g[i];
-        if (!staged) {
-            integratePosition(d, P);
-            return;
+        DBody b = readBody<kBodySolve | kBodyForce | kBodyPose | kBodyCom | kBodyLocal | kBodyBase>(d);
+        if (staged) {
+            b.v = { at(0, i), at(1, i), at(2, i) };
+            b.w = { at(3, i), at(4, i), at(5, i) };
+            b.dp = { at(6, i), at(7, i), at(8, i) };
+            b.dq = { at(9, i), at(10, i), at(11, i), at(12, i) };
         }
-        PosBody b;
-        b.alive = d.alive;
-        b.type = d.type;
-        b.awake = d.awake;
-        b.v = { at(0, i), at(1, i), at(2, i) };
-        b.w = { at(3, i), at(4, i), at(5, i) };
-        b.dp = { at(6, i), at(7, i), at(8, i) };
-        b.dq = { at(9, i), at(10, i), at(11, i), at(12, i) };
-        b.com = d.com;
-        b.localCenter = d.localCenter;
-        b.qBase = d.qBase;
-        b.xf = d.xf;
-        b.kept = d.kept;
+        if (!b.alive || b.type == kStatic || (b.type == kDynamic && !b.awake)) { return; }
+        const float kept = b.kept;
         integratePosition(b, P);
-        at(0, i) = b.v.x, at(1, i) = b.v.y, at(2, i) = b.v.z;
-        at(3, i) = b.w.x, at(4, i) = b.w.y, at(5, i) = b.w.z;
-        at(6, i) = b.dp.x, at(7, i) = b.dp.y, at(8, i) = b.dp.z;
-        at(9, i) = b.dq.x, at(10, i) = b.dq.y, at(11, i) = b.dq.z, at(12, i) = b.dq.w;
-        d.com = b.com;
-        d.xf = b.xf;
-        d.kept = b.kept;
+        if (staged) {
+            storeVW(i, b);
+            at(6, i) = b.dp.x, at(7, i) = b.dp.y, at(8, i) = b.dp.z;
+            at(9, i) = b.dq.x, at(10, i) = b.dq.y, at(11, i) = b.dq.z, at(12, i) = b.dq.w;
+        } else {
+            writeBody<kBodySolve>(d, b);
+        }
+        writeBody<kBodyPose | kBodyCom>(d, b);
+        if (b.kept != kept) { d.kept = b.kept; }
     }
 };
 
@@ -2880,7 +2847,7 @@ __device__ __forceinline__ void rebuildSolverData(const Batch& B, const WorldInf
 // holds each body's pose (kFlatPoseWords) and the step's velocity-update terms (kFlatMotionWords), so that the
 // body phases of a substep read a few coalesced words instead of the body's whole record.
 constexpr int kFlatBodyWords = 4;
-constexpr int kFlatPoseWords = 5;    // com; xf.p; xf.q; qBase; localCenter
+constexpr int kFlatPoseWords = 5;    // com, sleepTime; xf.p, extent; xf.q; qBase; localCenter
 constexpr int kFlatMotionWords = 7;  // gravity-and-force term, linear damping factor; torque term, angular
                                      // damping factor; linear then angular projection (18 floats, 2 unused)
 
@@ -2967,11 +2934,11 @@ __device__ __forceinline__ void storeMotion(const FlatStore& f, uint32_t i, cons
 
 // The first substep's staging: the body's solver state, pose and velocity terms from its record.
 static __device__ void flatBegin(const FlatStore& f, uint32_t i, const StepParams& P) {
-    const DBody& d = f.g[i];
+    const DBody d = readBody<kBodySolve | kBodyInvInertia | kBodyForce | kBodyProj | kBodyPose | kBodyCom | kBodyLocal | kBodyBase>(f.g[i]);
     f.put(i, d.v, d.w, d.dp, d.dq, d.type | (d.awake << 8) | (d.alive << 16));
     float4* q = f.pose + (size_t)kFlatPoseWords * i;
-    q[0] = f4(d.com, 0.0f);
-    q[1] = f4(d.xf.p, 0.0f);
+    q[0] = f4(d.com, d.sleepTime);
+    q[1] = f4(d.xf.p, d.extent);
     q[2] = q4(d.xf.q);
     q[3] = q4(d.qBase);
     q[4] = f4(d.localCenter, 0.0f);
@@ -3003,24 +2970,38 @@ static __device__ void flatVelocity(const FlatStore& f, uint32_t i, const StepPa
     SpeedBody s;
     s.type = type;
     s.awake = awake;
-    s.kept = f.g[i].kept;
+    const float kept = s.kept = f.g[i].kept;
     s.v = l.v + xyz(m0);
     s.v = L * (s.v * m0.w);
     s.w = l.w + xyz(m1);
     s.w = A * (s.w * m1.w);
     limitSpeed(s, P.maxLinearSpeed, P.maxAngularSpeed);
     f.storeVW(i, s);
-    f.g[i].kept = s.kept;
+    if (s.kept != kept) { f.g[i].kept = s.kept; }
 }
 
-// integratePosition from the store and the pose: the new pose goes to the store and to the body's record (joints
-// of the relaxing pass read it there).
+// The pose in the store, into a body.
+__device__ __forceinline__ void flatPoseOf(const FlatStore& f, uint32_t i, DBody& b) {
+    const float4* q = f.pose + (size_t)kFlatPoseWords * i;
+    const float4 com = q[0], at = q[1];
+    b.com = xyz(com);
+    b.sleepTime = com.w;
+    b.xf.p = xyz(at);
+    b.extent = at.w;
+    b.xf.q = quatOf(q[2]);
+    b.qBase = quatOf(q[3]);
+}
+
+// integratePosition from the store and the pose: the new pose goes to the store, and with joints to the body's record
+// as well (those of the relaxing pass read it there).
+template <bool Joints>
 static __device__ void flatPosition(const FlatStore& f, uint32_t i, const StepParams& P) {
     const uint32_t fl = f.flags(i);
     const LanedBody l = f.loadLaned(i);
     float4* q = f.pose + (size_t)kFlatPoseWords * i;
     DBody& d = f.g[i];
-    PosBody b;
+    DBody b;
+    flatPoseOf(f, i, b);
     b.alive = fl >> 16;
     b.type = l.type;
     b.awake = l.awake;
@@ -3028,20 +3009,15 @@ static __device__ void flatPosition(const FlatStore& f, uint32_t i, const StepPa
     b.w = l.w;
     b.dp = l.dp;
     b.dq = l.dq;
-    b.com = xyz(q[0]);
-    b.xf.p = xyz(q[1]);
-    b.xf.q = quatOf(q[2]);
-    b.qBase = quatOf(q[3]);
     b.localCenter = xyz(q[4]);
-    b.kept = d.kept;
+    const float kept = b.kept = d.kept;
     integratePosition(b, P);
     f.put(i, b.v, b.w, b.dp, b.dq, fl);
-    q[0] = f4(b.com, 0.0f);
-    q[1] = f4(b.xf.p, 0.0f);
+    q[0] = f4(b.com, b.sleepTime);
+    q[1] = f4(b.xf.p, b.extent);
     q[2] = q4(b.xf.q);
-    d.com = b.com;
-    d.xf = b.xf;
-    d.kept = b.kept;
+    if constexpr (Joints) { writeBody<kBodyPose | kBodyCom>(d, b); }
+    if (b.kept != kept) { d.kept = b.kept; }
 }
 
 // The passes of a contact solved on its own, for either store, from the contact and its stored axes; both bodies are
@@ -3301,10 +3277,11 @@ __global__ void __launch_bounds__(Rooms ? kRoomWarps * 32 : kMaxBlock) k_substep
             // every body takes a new base pose (src/world.cpp:1663-1666).
             keepPlacements(B, g, wi);
             for (uint32_t i = g.tid; i < nb; i += g.size) {
-                DBody& d = st.g[i];
-                d.dp = zero3();
-                d.dq = qid();
-                d.qBase = d.xf.q;
+                DBody b = readBody<kBodySolve | kBodyPose>(st.g[i]);
+                b.dp = zero3();
+                b.dq = qid();
+                b.qBase = b.xf.q;
+                writeBody<kBodySolve | kBodyBase>(st.g[i], b);
             }
             g.sync();
         }
@@ -3361,8 +3338,10 @@ __global__ void __launch_bounds__(Rooms ? kRoomWarps * 32 : kMaxBlock) k_substep
             // The next substep starts with a refresh, whose axes use the inverse inertia at the new pose
             // (src/world.cpp:1660-1662).
             for (uint32_t i = g.tid; i < nb; i += g.size) {
-                DBody& d = st.g[i];
-                if (d.alive && d.type == kDynamic && d.awake) { updateInverseMass(d); }
+                DBody b = readBody<kBodyMassReads>(st.g[i]);
+                if (!b.alive || b.type != kDynamic || !b.awake) { continue; }
+                updateInverseInertia(b);
+                writeBody<kBodyInvInertia>(st.g[i], b);
             }
         }
     });
@@ -3582,26 +3561,34 @@ __global__ void __launch_bounds__(256, 2) k_substep_flat(const __grid_constant__
         }
         if (bias) {
             if (!skip) {
-                for (uint32_t gb = tid; gb < nb; gb += threads) { flatPosition(all, gb, P); }
+                for (uint32_t gb = tid; gb < nb; gb += threads) { flatPosition<Joints>(all, gb, P); }
             }
             gridBarrier(B);
         }
     }
-    // Back into the bodies' records (the pose is there already); a world whose next substep starts with a refresh
-    // takes its inverse inertia at the new pose (src/world.cpp:1660-1662), and the torque term with it.
+    // Back into the records of the bodies that something reads before the store is used again: after the last substep
+    // all of them; before, those of the worlds whose next substep starts with a refresh, which takes the inverse
+    // inertia at the new pose (src/world.cpp:1660-1662), and the torque term with it.
     if (!skip) {
+        const bool last = sub + 1 >= P.substeps;
         for (uint32_t gb = tid; gb < nb; gb += threads) {
-            const LanedBody l = all.loadLaned(gb);
             DBody& d = B.bodies[gb];
-            d.v = l.v;
-            d.w = l.w;
-            d.dp = l.dp;
-            d.dq = l.dq;
-            d.qBase = quatOf(B.flatPose[(size_t)kFlatPoseWords * gb + 3]);
-            if (sub + 1 < P.substeps && refreshedAt(B.counts[d.world], sub + 1, P.substeps) && d.alive &&
-                d.type == kDynamic && d.awake) {
-                updateInverseInertia(d);
-                storeTorqueTerm(all, gb, d, P);
+            if (!last && !refreshedAt(B.counts[d.world], sub + 1, P.substeps)) { continue; }
+            DBody b = readBody<kBodyInvInertia | kBodyForce | kBodyInertia>(d);
+            const LanedBody l = all.loadLaned(gb);
+            b.v = l.v;
+            b.w = l.w;
+            b.dp = l.dp;
+            b.dq = l.dq;
+            b.type = l.type;
+            b.awake = l.awake;
+            b.alive = all.flags(gb) >> 16;
+            flatPoseOf(all, gb, b);
+            writeBody<kBodySolve | kBodyPose | kBodyCom | kBodyBase>(d, b);
+            if (!last && b.alive && b.type == kDynamic && b.awake) {
+                updateInverseInertia(b);
+                writeBody<kBodyInvInertia>(d, b);
+                storeTorqueTerm(all, gb, b, P);
             }
         }
     }
@@ -3843,6 +3830,10 @@ static __device__ void sweepWorld(const Batch& B, const StepParams& P, const G& 
     g.sync();
 }
 
+// What the islands ask of a body, a byte each beside one another (Batch::struck, free after the solve): reading it from
+// the bodies cost a scattered load for each end of each contact and for each body, three times over.
+constexpr uint32_t kEndMoves = 1u, kEndDriven = 2u, kEndAlive = 4u;  // awake and dynamic; kinematic and moving
+
 // Union-find is staged in the group's shared slice (parent and island time by body, union pairs by contact)
 // when the world fits, else in its global scratch.
 // After the solve (src/world.cpp:1685-1691): active joints turn the step's impulses into a force and torque
@@ -4020,17 +4011,22 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
         const float threshold = P.sleepThreshold;
         for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
             const uint32_t gb = wi.bodyFirst + i;
-            DBody& b = B.bodies[gb];
+            DBody& d = B.bodies[gb];
+            DBody b = readBody<kBodySolve | kBodyForce | kBodyPose | kBodyCom | kBodyLocal | kBodyInvMass | kBodyStart |
+                               kBodyBounds | kBodyShapes>(d);
             parent[i] = i;
             islandTime[i] = __float_as_uint(FLT_MAX);
+            B.struck[gb] = (uint8_t)((movingBody(b) ? kEndMoves : 0u) |
+                                     (b.type == kKinematic && movingAwake(b) ? kEndDriven : 0u) | (b.alive ? kEndAlive : 0u));
             if (!b.alive) { continue; }
             limitSpeed(b, P.maxLinearSpeed, P.maxAngularSpeed);
             b.force = zero3();
             b.torque = zero3();
             if (b.hasTarget) {
-                b.xf = b.target;
+                b.xf = d.target;
                 b.com = apply(b.xf, b.localCenter);
                 b.hasTarget = 0;
+                writeBody<kBodyPose | kBodyLocal>(d, b);
             }
             if (b.type != kStatic && !(b.type == kDynamic && !b.awake)) {
                 // Leaf refit over the new pose (src/world.cpp:1713-1718).
@@ -4047,13 +4043,11 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
                 }
             }
             // Sleep timers (src/world.cpp:1176-1185).
-            if (b.type != kDynamic || !b.awake) { continue; }
+            const bool moves = b.type == kDynamic && b.awake;
             const float speed = maxf(length(b.v), length(b.w) * b.extent);
-            if (!b.canSleep || speed > threshold) {
-                b.sleepTime = 0.0f;
-            } else {
-                b.sleepTime += P.dt;
-            }
+            if (moves) { b.sleepTime = !b.canSleep || speed > threshold ? 0.0f : b.sleepTime + P.dt; }
+            writeBody<kBodyVelocity | kBodyForce | kBodyCom | kBodyBounds>(d, b);
+            if (!moves) { continue; }
             if (!(isfinite(b.v.x) && isfinite(b.v.y) && isfinite(b.v.z) && isfinite(b.xf.p.x) && isfinite(b.xf.p.y) &&
                   isfinite(b.xf.p.z))) {
                 atomicOr(&wc.flags, kDevNonFinite);
@@ -4072,16 +4066,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
             [&](uint32_t ci) {
                 if (!contactOk(B, wi, wc, ci, 22)) { return false; }
                 const DContact& c = cs[ci];
+                const uint32_t ia = c.bodyA, ib = c.bodyB;
+                const uint32_t a = B.struck[ia], b = B.struck[ib];
                 if (c.count == 0) { return false; }
-                DBody& a = B.bodies[c.bodyA];
-                DBody& b = B.bodies[c.bodyB];
-                const bool da = a.type == kDynamic && a.awake;
-                const bool db = b.type == kDynamic && b.awake;
-                if (da && db) { return true; }
-                if (da && b.type == kKinematic && movingAwake(b)) {
-                    a.sleepTime = 0.0f;
-                } else if (db && a.type == kKinematic && movingAwake(a)) {
-                    b.sleepTime = 0.0f;
+                if (a & b & kEndMoves) { return true; }
+                if ((a & kEndMoves) && (b & kEndDriven)) {
+                    B.bodies[ia].sleepTime = 0.0f;
+                } else if ((b & kEndMoves) && (a & kEndDriven)) {
+                    B.bodies[ib].sleepTime = 0.0f;
                 }
                 return false;
             },
@@ -4116,17 +4108,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
             for (uint32_t x = 0; x < wi.jointCount; ++x) {
                 const DJoint& j = js[x];
                 if (!j.alive || j.broken) { continue; }
-                DBody* a = j.bodyA == kWorldEnd ? nullptr : &B.bodies[j.bodyA];
-                DBody& b = B.bodies[j.bodyB];
-                const bool da = a && a->type == kDynamic && a->awake;
-                const bool db = b.type == kDynamic && b.awake;
-                if (da && db) {
+                const uint32_t a = j.bodyA == kWorldEnd ? 0u : B.struck[j.bodyA], b = B.struck[j.bodyB];
+                if (a & b & kEndMoves) {
                     const uint32_t ra = findRoot(parent, j.bodyA - wi.bodyFirst), rb = findRoot(parent, j.bodyB - wi.bodyFirst);
                     if (ra != rb) { parent[ra > rb ? ra : rb] = ra < rb ? ra : rb; }
-                } else if (da && b.type == kKinematic && movingAwake(b)) {
-                    a->sleepTime = 0.0f;
-                } else if (db && a && a->type == kKinematic && movingAwake(*a)) {
-                    b.sleepTime = 0.0f;
+                } else if ((a & kEndMoves) && (b & kEndDriven)) {
+                    B.bodies[j.bodyA].sleepTime = 0.0f;
+                } else if ((b & kEndMoves) && (a & kEndDriven)) {
+                    B.bodies[j.bodyB].sleepTime = 0.0f;
                 }
             }
         }
@@ -4134,12 +4123,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
         uint32_t awakeHere = 0, islandsHere = 0;
         for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
             DBody& b = B.bodies[wi.bodyFirst + i];
-            if (!b.alive || b.type != kDynamic || !b.awake) { continue; }
+            const uint32_t state = B.struck[wi.bodyFirst + i];
+            const float sleepTime = b.sleepTime;
+            if ((state & (kEndAlive | kEndMoves)) != (kEndAlive | kEndMoves)) { continue; }
             const uint32_t r = rootOf(parent, i);
             b.island = r;
             ++awakeHere;
             if (r == i) { ++islandsHere; }
-            atomicMin(&islandTime[r], __float_as_uint(b.sleepTime));
+            atomicMin(&islandTime[r], __float_as_uint(sleepTime));
         }
         awakeHere = __reduce_add_sync(0xffffffffu, awakeHere);
         islandsHere = __reduce_add_sync(0xffffffffu, islandsHere);
@@ -4150,7 +4141,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
         g.sync();
         for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
             DBody& b = B.bodies[wi.bodyFirst + i];
-            if (!b.alive || b.type != kDynamic || !b.awake) { continue; }
+            if ((B.struck[wi.bodyFirst + i] & (kEndAlive | kEndMoves)) != (kEndAlive | kEndMoves)) { continue; }
             if (__uint_as_float(islandTime[rootOf(parent, i)]) < P.timeToSleep) { continue; }
             b.awake = 0;
             b.v = zero3();

@@ -7,6 +7,9 @@
 // the world-local shape indices, as the reference's keys do (src/world.cpp:42).
 #pragma once
 
+#include <cstddef>
+#include <cstring>
+
 #include "tf_math.cuh"
 
 namespace tfb {
@@ -26,61 +29,134 @@ constexpr uint32_t kLockPlanar = kLockTZ | kLockRX | kLockRY;
 constexpr int kColors = 32;
 constexpr int kNoColor = kColors;
 
+// A body's fields lie by what reads and writes them together, in pieces of 16 bytes that start with a group: a thread
+// that works on a body moves whole pieces at once (readBody, writeBody).
 struct alignas(16) DBody {
     // Read and written by every solve.
     Vec3 v;
     Vec3 w;
     Vec3 dp;
     Quat dq;
-    Mat3 invMassWorld;
-    Mat3 invInertiaWorld;
-    float invMass;
-    float planeInvMass;
-    float planeInvInertia;
     uint32_t type;
     uint32_t awake;
     uint32_t alive;
 
-    Transform xf;
-    Vec3 com;
-    Vec3 localCenter;
-    float extent;
+    Mat3 invInertiaWorld;
+    float invMass;
+    float planeInvMass;
+    float planeInvInertia;
+
     Vec3 force;
     Vec3 torque;
-    float mass;
-    Mat3 inertia;
-    float linearDamping;
-    float angularDamping;
     float gravityScale;
-    uint32_t locks;
-    Quat lockFrame;
-    uint32_t canSleep;
-    float sleepTime;
-    uint32_t island;
-    uint32_t hasTarget;
-    Transform target;
-    // Bounds of the body's shapes other than half-spaces; hasBounds is 0 when it has none (no tree leaf).
-    Vec3 lo, hi;
-    uint32_t hasBounds;
     float kept;
+
     Mat3 linearProj;
     Mat3 angularProj;
+    float linearDamping;
+    float angularDamping;
+
+    Transform xf;
+    float extent;
+    Vec3 com;
+    float sleepTime;
+    Vec3 localCenter;
+    uint32_t hasTarget;
     Quat qBase;
-    Quat q0;
-    Vec3 com0;
-    float expectedTravel;
-    // The body's shapes: shapeList[shapeFirst .. shapeFirst + shapeCount), global shape indices.
-    uint32_t shapeFirst;
-    uint32_t shapeCount;
+
+    Mat3 invMassWorld;
+    float mass;
+    uint32_t island;
+    uint32_t canSleep;
+
+    Mat3 inertia;
+    uint32_t locks;
     uint32_t world;
     // Set by every planar pair that placed the body in the current round of collisions; the round's
     // placement is stored, and this cleared, once all its pairs are done.
     uint32_t posePending;
+    Quat lockFrame;
+
+    Quat q0;
+    Vec3 com0;
+    float expectedTravel;
+
+    // Bounds of the body's shapes other than half-spaces; hasBounds is 0 when it has none (no tree leaf).
+    Vec3 lo;
+    uint32_t hasBounds;
+    Vec3 hi;
+    // The body's shapes: shapeList[shapeFirst .. shapeFirst + shapeCount), global shape indices.
+    uint32_t shapeFirst;
+    uint32_t shapeCount;
+    Transform target;
+
     // The part of the body's pose in a plane that lasts between rounds (src/internal.h:141-148): the plane
     // normal it was placed for, that normal in the body's frame (the key) with the 2D axes around it, and the
     // plane's own 2D axes. Zero until the body is first placed.
     Vec3 poseNormal, poseKey, poseU, poseV, poseAxisU, poseAxisV;
 };
+
+// The pieces of a body that hold its bytes from one offset up to another, a bit each.
+constexpr uint64_t bodyPieces(size_t from, size_t to) {
+    uint64_t pieces = 0;
+    for (size_t k = from / 16; k < (to + 15) / 16; ++k) { pieces |= 1ull << k; }
+    return pieces;
+}
+constexpr uint64_t kBodyVelocity = bodyPieces(offsetof(DBody, v), offsetof(DBody, dp));
+constexpr uint64_t kBodySolve = bodyPieces(offsetof(DBody, v), offsetof(DBody, invInertiaWorld));
+constexpr uint64_t kBodyState = bodyPieces(offsetof(DBody, type), offsetof(DBody, invInertiaWorld));
+constexpr uint64_t kBodyInvInertia = bodyPieces(offsetof(DBody, invInertiaWorld), offsetof(DBody, force));
+constexpr uint64_t kBodyForce = bodyPieces(offsetof(DBody, force), offsetof(DBody, linearProj));
+constexpr uint64_t kBodyProj = bodyPieces(offsetof(DBody, linearProj), offsetof(DBody, xf));
+constexpr uint64_t kBodyPose = bodyPieces(offsetof(DBody, xf), offsetof(DBody, com));
+constexpr uint64_t kBodyCom = bodyPieces(offsetof(DBody, com), offsetof(DBody, localCenter));
+constexpr uint64_t kBodyLocal = bodyPieces(offsetof(DBody, localCenter), offsetof(DBody, qBase));
+constexpr uint64_t kBodyBase = bodyPieces(offsetof(DBody, qBase), offsetof(DBody, invMassWorld));
+constexpr uint64_t kBodyInvMass = bodyPieces(offsetof(DBody, invMassWorld), offsetof(DBody, inertia));
+constexpr uint64_t kBodyInertia = bodyPieces(offsetof(DBody, inertia), offsetof(DBody, q0));
+constexpr uint64_t kBodyStart = bodyPieces(offsetof(DBody, q0), offsetof(DBody, lo));
+constexpr uint64_t kBodyBounds = bodyPieces(offsetof(DBody, lo), offsetof(DBody, shapeCount));
+constexpr uint64_t kBodyShapes = bodyPieces(offsetof(DBody, shapeFirst), offsetof(DBody, target));
+// What updateInverseMass reads and writes.
+constexpr uint64_t kBodyMassReads = kBodyState | kBodyInvInertia | kBodyProj | kBodyPose | kBodyInvMass | kBodyInertia;
+constexpr uint64_t kBodyMassWrites = kBodyInvInertia | kBodyProj | kBodyInvMass;
+static_assert(sizeof(DBody) % 16 == 0 && sizeof(DBody) / 16 <= 64, "a body is whole pieces");
+static_assert((kBodyInvInertia & kBodyForce) == 0 && (kBodyForce & kBodyProj) == 0 && (kBodyProj & kBodyPose) == 0 &&
+                  (kBodyPose & kBodyCom) == 0 && (kBodyBase & kBodyInvMass) == 0 && (kBodyInvMass & kBodyInertia) == 0 &&
+                  (kBodyInertia & kBodyStart) == 0 && (kBodyStart & kBodyBounds) == 0,
+              "the groups start at pieces of their own");
+
+#if defined(__CUDACC__)
+// Some pieces of a body as one copy: the loads are 16 bytes wide and none waits for another. (Field by field, each
+// load of the 32 threads of a warp touches 32 separate lines, four bytes of each, and most wait for a branch or for a
+// store in between: the phases over bodies spent about 1000 cycles on every load they issued.) The fields outside the
+// pieces are not set.
+template <uint64_t Pieces>
+__device__ __forceinline__ DBody readBody(const DBody& d) {
+    DBody b;
+    const float4* from = reinterpret_cast<const float4*>(&d);
+#pragma unroll
+    for (int k = 0; k < (int)(sizeof(DBody) / 16); ++k) {
+        if (Pieces >> k & 1) {
+            const float4 piece = from[k];
+            memcpy(reinterpret_cast<unsigned char*>(&b) + 16 * k, &piece, 16);
+        }
+    }
+    return b;
+}
+template <uint64_t Pieces>
+__device__ __forceinline__ void writeBody(DBody& d, const DBody& b) {
+    float4* to = reinterpret_cast<float4*>(&d);
+#pragma unroll
+    for (int k = 0; k < (int)(sizeof(DBody) / 16); ++k) {
+        if (Pieces >> k & 1) {
+            float4 piece;
+            memcpy(&piece, reinterpret_cast<const unsigned char*>(&b) + 16 * k, 16);
+            to[k] = piece;
+        }
+    }
+}
+#endif
 
 struct alignas(16) DShape {
     uint32_t body;      // global body index
