@@ -2153,12 +2153,15 @@ public:
     // has more than 512 bodies); batches of many worlds give worlds of up to 96 bodies a warp each and the
     // larger ones the CTA. 64 KB of staging per CTA leaves room for three CTAs on an SM.
     //
-    // The substep's, measured (us of substeps a step): many worlds take 128 threads and a CTA past 32 bodies (4096
-    // uneven worlds: 1952 at step 18 and 2576 at step 40, against 2168 and 3068 solved flat and 2331 and 3012 with
-    // 256 threads and 96 bodies; 600 jointed worlds: 1097 against 2439 flat). A few worlds take a CTA each, unless
-    // one has so many bodies that one SM holds up the step: then the whole batch is solved flat (planar piles of 1000
-    // bodies: 208 with a CTA and 225 flat, 2083 bodies: 470 and 310, 4163: 798 and 334; pyramids of 1036 boxes: 677
-    // and 676, 2081: 1609 and 659).
+    // The substep's, measured (us of substeps a step). Many worlds take 128 threads and a CTA past 32 bodies (4096
+    // uneven worlds: 1839 at step 18 and 2348 at step 40, against 2396 and 3288 solved flat and 2148 and 2789 with 256
+    // threads and 96 bodies; 600 jointed worlds: 856 against 1045 flat), except: jointed worlds from 8 an SM on, solved flat
+    // (1400: 1326 and 1072 flat, 2000: 1544 and 1115; 1024: 1103 and 1040), and fewer than 8 worlds an
+    // SM with some past 128 bodies, which keep the flat solve that programs reading the shape in use know as their
+    // default (1024 uneven worlds: 157 flat and 155 at step 2, but 750 and 605 at step 18 and 1098 and 768 at step 40:
+    // worth tuning). A few worlds take a CTA each, unless one has so many bodies that one SM holds up the step: then
+    // the whole batch is solved flat (planar piles of 1017 bodies: 171 with a CTA and 218 flat, 4065: 413 and 279;
+    // terrain of 4097: 855 and 769; pyramids of 1036 boxes: 677 and 676, 2081: 1609 and 659).
     LaunchShape defaultShape(int k) const {
         LaunchShape s;
         const bool many = manyWorlds();
@@ -2166,7 +2169,9 @@ public:
         s.bigBodies = many ? 96u : 0u;
         const bool stages = k == 0 || k == 3 || k == 5 || k == 6;
         s.smemBytes = stages ? 64u * 1024u : 0u;
-        if (k == 5 && !many && maxWorldBodies > kFlatBodies) {
+        const bool flat = !many ? maxWorldBodies > kFlatBodies
+                          : worlds.size() < (size_t)smCount * 8 ? !hasJoints && maxWorldBodies > 128 : hasJoints;
+        if (k == 5 && flat) {
             s.threads = 256u;
             s.bigBodies = 0u;
             s.smemBytes = 0u;
