@@ -2273,10 +2273,10 @@ public:
             TF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, flat[f], threads, 0));
             if (perSm < 1) { return fail(TF_E_INVALID, "launch shape does not fit on an SM"); }
             // No more CTAs than the class list can ever fill: its capacity is the batch's candidate slots (pair
-            // collisions) or contact slots (refreshes), an item a thread (a warp for mesh pairs). A small batch
+            // collisions) or contact slots (refreshes), an item a warp (forSpreadItems). A small batch
             // then launches a handful of CTAs rather than a full device's worth that find no work.
             const size_t cap = f < kPairClasses ? totalCand : totalContacts;
-            const size_t perCta = meshGrid(f) ? (size_t)std::min(threads / 32, kMeshWarps) : (size_t)threads;
+            const size_t perCta = meshGrid(f) ? (size_t)std::min(threads / 32, kMeshWarps) : (size_t)threads / 32;
             const size_t needed = std::max<size_t>(1, (cap + perCta - 1) / perCta);
             flatGrids[f] = (int)std::min<size_t>((size_t)smCount * (size_t)perSm, needed);
         }

@@ -1319,47 +1319,76 @@ __device__ __forceinline__ uint32_t lowerKey(const DContact* c, uint32_t n, uint
     return lo;
 }
 
-// One candidate: keep and measure the old contact when the pair barely moved, else collide it and carry the
-// old impulses over (src/world.cpp:883-959).
-template <int Cls = kClassAny>
-__device__ void narrowOne(const Batch& B, const StepParams& P, const WorldInfo& wi, WorldCounts& wc, uint32_t i,
-                          const DContact* old, uint32_t oldCount) {
+// One candidate (src/world.cpp:883-959), in two halves. narrowKeep finds the pair's old contacts [lo, hi) and keeps and
+// measures the old contact when the pair barely moved; narrowAnew collides a pair it did not keep and carries the old
+// impulses over.
+__device__ __forceinline__ void narrowUsed(const Batch& B, const DShape& sa, const DShape& sb, const DBody& ba, const DBody& bb,
+                                           WorldCounts& wc, DContact& out) {
+    out.friction = sqrtf(sa.friction * sb.friction);
+    out.restitution = maxf(sa.restitution, sb.restitution);
+    out.rollingResistance = maxf(sa.rollingResistance, sb.rollingResistance);
+    if (ba.type == kDynamic && !ba.awake && movingAwake(bb)) {
+        B.wakeMark[sa.body] = 1;
+        wc.wakePending = 1;
+    }
+    if (bb.type == kDynamic && !bb.awake && movingAwake(ba)) {
+        B.wakeMark[sb.body] = 1;
+        wc.wakePending = 1;
+    }
+}
+
+// Whether nothing is left to do.
+__device__ __forceinline__ bool narrowKeep(const Batch& B, const StepParams& P, const WorldInfo& wi, WorldCounts& wc, uint32_t i,
+                                           const DContact* old, uint32_t oldCount, uint32_t& lo, uint32_t& hi) {
     const uint64_t key = B.cand[wi.candFirst + i];
     const uint32_t ia = (uint32_t)(key >> 32), ib = (uint32_t)(key & 0xffffffffu);
     if (!TF_OK_INDEX(B, ia < wi.shapeCount && ib < wi.shapeCount, 1, wi.bodyFirst, ia)) {
         B.stageUsed[wi.candFirst + i] = 0;
-        return;
+        return true;
     }
-    const uint32_t gsa = wi.shapeFirst + ia, gsb = wi.shapeFirst + ib;
-    const DShape sa = B.shapes[gsa];
-    const DShape sb = B.shapes[gsb];
+    const DShape& sa = B.shapes[wi.shapeFirst + ia];
+    const DShape& sb = B.shapes[wi.shapeFirst + ib];
     if (!TF_OK_INDEX(B, sa.body - wi.bodyFirst < wi.bodyCount && sb.body - wi.bodyFirst < wi.bodyCount, 2,
                      wi.bodyFirst, sa.body)) {
         B.stageUsed[wi.candFirst + i] = 0;
-        return;
+        return true;
     }
     if (!TF_OK_INDEX(B, oldCount <= wi.contactCap, 3, wi.bodyFirst, oldCount)) {
         B.stageUsed[wi.candFirst + i] = 0;
-        return;
+        return true;
     }
+    lo = lowerKey(old, oldCount, key);
+    hi = lo;
+    while (hi < oldCount && old[hi].key == key) { ++hi; }
+    if (lo == hi) { return false; }
+    const DBody ba = readBody<kBodySolve | kBodyPose | kBodyCom | kBodyInertia>(B.bodies[sa.body]);
+    const DBody bb = readBody<kBodySolve | kBodyPose | kBodyCom | kBodyInertia>(B.bodies[sb.body]);
+    for (uint32_t it = lo; it < hi; ++it) {
+        if (!stillFits(old[it], ba, bb, P)) { return false; }
+    }
+    DContact& out = B.stage[wi.candFirst + i];
+    if (hi - lo > 1) { atomicOr(&wc.flags, kDevUnsupported); }
+    out = old[lo];
+    measureAgain(ba, bb, out, P);
+    out.boundsFirst = out.boundsCount = 0;
+    narrowUsed(B, sa, sb, ba, bb, wc, out);
+    B.stageUsed[wi.candFirst + i] = 1;
+    return true;
+}
+
+template <int Cls>
+__device__ __forceinline__ void narrowAnew(const Batch& B, const StepParams& P, const WorldInfo& wi, WorldCounts& wc, uint32_t i,
+                                           const DContact* old, uint32_t lo, uint32_t hi) {
+    const uint64_t key = B.cand[wi.candFirst + i];
+    const uint32_t gsa = wi.shapeFirst + (uint32_t)(key >> 32), gsb = wi.shapeFirst + (uint32_t)(key & 0xffffffffu);
+    const DShape sa = B.shapes[gsa];
+    const DShape sb = B.shapes[gsb];
     const DBody& ba = B.bodies[sa.body];
     const DBody& bb = B.bodies[sb.body];
-    const uint32_t lo = lowerKey(old, oldCount, key);
-    uint32_t hi = lo;
-    while (hi < oldCount && old[hi].key == key) { ++hi; }
-    const bool hasOld = lo < hi;
-    bool keep = hasOld;
-    for (uint32_t it = lo; it < hi && keep; ++it) { keep = stillFits(old[it], ba, bb, P); }
-    const bool touched = hasOld && (old[lo].flags & kCTouched);
+    const bool touched = lo < hi && (old[lo].flags & kCTouched);
     DContact& out = B.stage[wi.candFirst + i];
     uint8_t used = 0;
-    if (keep) {
-        if (hi - lo > 1) { atomicOr(&wc.flags, kDevUnsupported); }
-        out = old[lo];
-        measureAgain(ba, bb, out, P);
-        out.boundsFirst = out.boundsCount = 0;
-        used = 1;
-    } else {
+    {
         Manifold m;
         if (!collidePair<Cls>(B, P, sa, sb, P.dt, m, kFeatNone, -1, -1)) { atomicOr(&wc.flags, kDevUnsupported); }
         if (m.count > 0) {
@@ -1409,19 +1438,7 @@ __device__ void narrowOne(const Batch& B, const StepParams& P, const WorldInfo& 
             used = 1;
         }
     }
-    if (used) {
-        out.friction = sqrtf(sa.friction * sb.friction);
-        out.restitution = maxf(sa.restitution, sb.restitution);
-        out.rollingResistance = maxf(sa.rollingResistance, sb.rollingResistance);
-        if (ba.type == kDynamic && !ba.awake && movingAwake(bb)) {
-            B.wakeMark[sa.body] = 1;
-            wc.wakePending = 1;
-        }
-        if (bb.type == kDynamic && !bb.awake && movingAwake(ba)) {
-            B.wakeMark[sb.body] = 1;
-            wc.wakePending = 1;
-        }
-    }
+    if (used) { narrowUsed(B, sa, sb, ba, bb, wc, out); }
     B.stageUsed[wi.candFirst + i] = used;
 }
 
@@ -1623,22 +1640,86 @@ static __device__ void narrowMesh(const Batch& B, const StepParams& P, const Wor
     B.stageUsed[wi.candFirst + i] = (uint8_t)n;
 }
 
+// Calls f(item, whether it is one of the list's) for the items of a list spread over the whole grid, a warp's lanes at
+// once: a lane each when the list has items for every lane, and only as many lanes of a warp as it takes when it is
+// shorter, down to one. The pairs of a list take different paths through the same code, which a warp walks one after the
+// other: of few pairs, each gets a warp to itself. (28 pairs of boxes: 40 us of collisions a step on
+// one warp, 26 spread; 64 uneven worlds: 85 and 54, their refreshes 230 and 165.) `turn` of `turns` lists that one launch works on moves a list's
+// first warp, so that short lists do not queue on the same warps.
+template <class F>
+__device__ __forceinline__ void forSpreadItems(uint32_t n, uint32_t turn, uint32_t turns, F f) {
+    const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t lanes = min(32u, (n + warps - 1) / warps);
+    // Consecutive warps lie on different CTAs while the list is short, and in one, whose items share bodies, when it is
+    // not.
+    const uint32_t at = lanes < 32 ? (threadIdx.x >> 5) * gridDim.x + blockIdx.x : blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const uint32_t warp = (at + warps - warps / turns * turn) % warps;
+    for (uint32_t first = warp * lanes; first < n; first += warps * lanes) {
+        const uint32_t item = first + lane;
+        f(item, lane < lanes && item < n, first + warps * lanes >= n);
+    }
+}
+
+// A convex pair that was not kept, waiting for its warp to have a pair for every lane.
+struct AnewPair {
+    uint32_t world, candidate, lo, hi;
+};
+
 // The candidate pairs of one class, over every world, one thread per pair (src/world.cpp:874-960); each
 // result lands in the pair's own staging slot, so pairs need no order among themselves.
+//
+// Of convex pairs, which cost the most to collide, a warp first keeps those that can be kept and queues the others, and
+// collides them once there is one for every lane. (Collided where they were met, the pairs of 1024 impact worlds, three
+// quarters of them kept, left 6.4 of 32 lanes at work: 1644 us of pair collisions a step, and 920 this way.)
 template <int Cls>
-__device__ __forceinline__ void collideClass(const Batch& B, const StepParams& P, int serial) {
+__device__ __forceinline__ void collideClass(const Batch& B, const StepParams& P, int serial, uint32_t turn = 0, uint32_t turns = 1) {
     const uint32_t n = *(volatile uint32_t*)(B.work + kSlotCandItems + Cls);
     const uint2* items = B.candItems + (size_t)Cls * B.candItemStride;
-    for (uint32_t item = blockIdx.x * blockDim.x + threadIdx.x; item < n; item += gridDim.x * blockDim.x) {
+    if constexpr (Cls == kClassConvex) {
+        __shared__ AnewPair s_anew[256 / 32][64];
+        AnewPair* queue = s_anew[threadIdx.x >> 5];
+        const uint32_t lane = threadIdx.x & 31;
+        uint32_t queued = 0;
+        forSpreadItems(n, turn, turns, [&](uint32_t item, bool mine, bool last) {
+            bool anew = false;
+            AnewPair pair;
+            if (mine) {
+                const uint2 it = items[item];
+                const WorldInfo& wi = B.info[it.x];
+                WorldCounts& wc = B.counts[it.x];
+                pair = { it.x, it.y, 0, 0 };
+                anew = !narrowKeep(B, P, wi, wc, it.y, B.previous + wi.contactFirst, wc.contactCount, pair.lo, pair.hi);
+            }
+            const uint32_t found = __ballot_sync(0xffffffffu, anew);
+            if (anew) { queue[queued + __popc(found & ((1u << lane) - 1u))] = pair; }
+            queued += __popc(found);
+            __syncwarp();
+            while (queued >= 32 || (last && queued > 0)) {
+                const uint32_t now = min(queued, 32u);
+                queued -= now;
+                if (lane < now) {
+                    const AnewPair p = queue[queued + lane];
+                    const WorldInfo wi = B.info[p.world];
+                    narrowAnew<Cls>(B, P, wi, B.counts[p.world], p.candidate, B.previous + wi.contactFirst, p.lo, p.hi);
+                }
+                __syncwarp();
+            }
+        });
+        return;
+    }
+    forSpreadItems(n, turn, turns, [&](uint32_t item, bool mine, bool) {
+        if (!mine) { return; }
         const uint2 it = items[item];
         const WorldInfo wi = B.info[it.x];
         WorldCounts& wc = B.counts[it.x];
+        const DContact* old = B.previous + wi.contactFirst;
         if constexpr (Cls == kClassMesh) {
-            narrowMesh<false>(B, P, wi, wc, it.y, B.previous + wi.contactFirst, wc.contactCount, serial);
+            narrowMesh<false>(B, P, wi, wc, it.y, old, wc.contactCount, serial);
         } else {
-            narrowOne<Cls>(B, P, wi, wc, it.y, B.previous + wi.contactFirst, wc.contactCount);
+            uint32_t lo, hi;
+            if (!narrowKeep(B, P, wi, wc, it.y, old, wc.contactCount, lo, hi)) { narrowAnew<Cls>(B, P, wi, wc, it.y, old, lo, hi); }
         }
-    }
+    });
 }
 
 // The mesh candidates over every world, a warp per pair, the warp's lanes over the pair's triangles: a pair
@@ -1678,12 +1759,12 @@ template <int Unused = 0>
 __global__ void __launch_bounds__(256) k_collide_all(const __grid_constant__ Batch B, const __grid_constant__ StepParams P,
                                                      int serial) {
     if (stepAborted(B, serial)) { return; }
-    collideClass<kClassSpheres>(B, P, serial);
-    collideClass<kClassSpherePoly>(B, P, serial);
-    collideClass<kClassPlane>(B, P, serial);
-    collideClass<kClassConvex>(B, P, serial);
-    collideClass<kClassPlanar>(B, P, serial);
-    collideClass<kClassMesh>(B, P, serial);
+    collideClass<kClassSpheres>(B, P, serial, 0, 6);
+    collideClass<kClassSpherePoly>(B, P, serial, 1, 6);
+    collideClass<kClassPlane>(B, P, serial, 2, 6);
+    collideClass<kClassConvex>(B, P, serial, 3, 6);
+    collideClass<kClassPlanar>(B, P, serial, 4, 6);
+    collideClass<kClassMesh>(B, P, serial, 5, 6);
 }
 
 __device__ __forceinline__ bool keyLess(uint64_t ka, uint32_t pa, uint64_t kb, uint32_t pb) {
@@ -1942,17 +2023,58 @@ static __device__ void buildRow(const Batch& B, const WorldInfo& wi, uint32_t sl
     }
 }
 
-// The impulses a laned contact's record holds, back into the contact.
+// What the solve and the refreshes changed in a laned contact's record, back into the contact: the impulses, and the
+// lever arms and separations a refresh expressed anew. A point's first 12 words, whole pieces at a time.
 __device__ __forceinline__ void returnImpulses(const Batch& B, uint32_t slot, DContact& c) {
+    static_assert(offsetof(DPoint, adjustedSeparation) == 24 && offsetof(DPoint, tangentImpulse) == 32 &&
+                      offsetof(DPoint, relativeVelocity) == 48, "the order of a point's first words");
     constexpr int S = kRowTile;
     const float4* R = rowOf(B, slot);
-    for (int i = 0; i < c.count; ++i) {
+    const int n = c.count;
+    for (int i = 0; i < n; ++i) {
         const int at = kRowPoint + kRowPointWords * i;
-        const float4 m = R[(at + 2) * S];
-        const float4 t = R[(at + 3) * S];
-        c.points[i].normalImpulse = m.z;
-        c.points[i].maxNormalImpulse = m.w;
-        c.points[i].tangentImpulse = xyz(t);
+        const float4 a = R[at * S], b = R[(at + 1) * S], m = R[(at + 2) * S], t = R[(at + 3) * S];
+        float4* p = reinterpret_cast<float4*>(&c.points[i]);
+        p[0] = make_float4(a.x, a.y, a.z, b.x);
+        p[1] = make_float4(b.y, b.z, a.w, m.z);
+        p[2] = make_float4(t.x, t.y, t.z, m.w);
+    }
+}
+
+// A laned contact's record at a refresh that does not collide its pair again: rebaseContact and the axes of buildRow,
+// from the record itself. Its normal and the bodies' inverse masses are what they were, so the head and the linear
+// terms stay; the contact takes the lever arms back with the impulses (returnImpulses). (Through the contact, its
+// impulses and its points first and then the whole record built again, the refreshes of 1024 impact worlds, which
+// collide few pairs again, took 1255 us a step, nearly all of it waiting for scattered four-byte loads; 418 this way.)
+static __device__ void rebaseRow(const Batch& B, uint32_t slot) {
+    constexpr int S = kRowTile;
+    float4* R = rowOf(B, slot);
+    const float4 h = R[kRowHead * S], normal = R[kRowNormal * S], tangent1 = R[kRowT1 * S], tangent2 = R[kRowT2 * S];
+    const SixVec lin = getSix<S>(R, kRowLinear);
+    const DBody a = readBody<kBodySolve | kBodyInvInertia>(B.bodies[__float_as_uint(h.x)]);
+    const DBody b = readBody<kBodySolve | kBodyInvInertia>(B.bodies[__float_as_uint(h.y)]);
+    const int n = (int)__float_as_uint(h.z);
+    const float shift = dot(b.dp - a.dp, xyz(normal));
+    const Vec3 d[3] = { xyz(normal), xyz(tangent1), xyz(tangent2) };
+    for (int i = 0; i < n; ++i) {
+        const int at = kRowPoint + kRowPointWords * i;
+        const float4 pa = R[at * S], pb = R[(at + 1) * S], m = R[(at + 2) * S];
+        const Vec3 ra = rotate(a.dq, xyz(pa)), rb = rotate(b.dq, xyz(pb));
+        Vec3 angular[6];
+        float mass[3];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            // makeAxis's operations, the linear terms taken from the record.
+            const Vec3 armA = cross(ra, d[x]), armB = cross(rb, d[x]);
+            angular[2 * x] = a.invInertiaWorld * armA;
+            angular[2 * x + 1] = b.invInertiaWorld * armB;
+            const float k = dot(d[x], lin.v[2 * x]) + dot(d[x], lin.v[2 * x + 1]) + dot(armA, angular[2 * x]) + dot(armB, angular[2 * x + 1]);
+            mass[x] = k > 1e-6f * (a.invMass + b.invMass) ? 1.0f / k : 0.0f;
+        }
+        R[at * S] = f4(ra, pa.w + shift);
+        R[(at + 1) * S] = f4(rb, mass[0]);
+        R[(at + 2) * S] = make_float4(mass[1], mass[2], m.z, m.w);
+        putSix(R, at + 4, angular);
     }
 }
 
@@ -2240,33 +2362,6 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
             },
             [&](uint32_t i, uint32_t pos) { B.active[cf + pos] = i; });
         const uint32_t* act = B.active + cf;
-        // A world with fast contacts is refreshed between substeps: its fast contacts join the flat list of
-        // their pair class, its other active contacts the light list.
-        const uint32_t nFast = *(volatile uint32_t*)fast;
-        if (nFast > 0) {
-            uint32_t* cls = g.shared(s_class[g.id]);
-            uint32_t* classBase = g.shared(s_classBase[g.id]);
-            if (g.tid <= kPairClasses) { cls[g.tid] = 0; }
-            g.sync();
-            auto listOf = [&](uint32_t x) {
-                const uint32_t ci = act[x];
-                if (!(B.cflags[cf + ci] & kFlagFast)) { return kPairClasses; }
-                return pairClassOf(B, cs[ci].shapeA, cs[ci].shapeB);
-            };
-            for (uint32_t x = g.tid; x < nActive; x += g.size) { takePlace(cls, (uint32_t)listOf(x)); }
-            g.sync();
-            if (g.tid <= kPairClasses) {
-                classBase[g.tid] = atomicAdd(B.work + kSlotFastItems + g.tid, cls[g.tid]);
-                cls[g.tid] = 0;
-            }
-            g.sync();
-            for (uint32_t x = g.tid; x < nActive; x += g.size) {
-                const int l = listOf(x);
-                const uint32_t pos = classBase[l] + takePlace(cls, (uint32_t)l);
-                B.contactItems[(size_t)l * B.contactItemStride + pos] = make_uint2(w, act[x]);
-            }
-            g.sync();
-        }
         const bool staged = wi.bodyCount <= stageBodies && nActive <= stageContacts;
         uint32_t* masks = staged ? reinterpret_cast<uint32_t*>(slice) : B.bodyColors + wi.bodyFirst;
         uint32_t* endA = staged ? masks + stageBodies : B.mergeIdxA + cf;
@@ -2335,6 +2430,34 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
             const DContact& c = cs[ci];
             makeContactAxes(axisBodyOf(B.bodies[c.bodyA]), axisBodyOf(B.bodies[c.bodyB]), c,
                             B.axes + (size_t)(cf + ci) * kAxesPerContact);
+        }
+        // A world with fast contacts is refreshed between substeps: its fast contacts join the flat list of
+        // their pair class, its other active contacts the light list, in the order of their records.
+        if (*(volatile uint32_t*)fast > 0) {
+            uint32_t* cls = g.shared(s_class[g.id]);
+            uint32_t* classBase = g.shared(s_classBase[g.id]);
+            if (g.tid <= kPairClasses) { cls[g.tid] = 0; }
+            g.sync();
+            const uint32_t nListed = nColored + wc.restCount;
+            auto contactAt = [&](uint32_t x) { return x < nColored ? B.colored[cf + x] : B.rest[cf + x - nColored]; };
+            auto listOf = [&](uint32_t ci) {
+                if (!(B.cflags[cf + ci] & kFlagFast)) { return kPairClasses; }
+                return pairClassOf(B, cs[ci].shapeA, cs[ci].shapeB);
+            };
+            for (uint32_t x = g.tid; x < nListed; x += g.size) { takePlace(cls, (uint32_t)listOf(contactAt(x))); }
+            g.sync();
+            if (g.tid <= kPairClasses) {
+                classBase[g.tid] = atomicAdd(B.work + kSlotFastItems + g.tid, cls[g.tid]);
+                cls[g.tid] = 0;
+            }
+            g.sync();
+            for (uint32_t x = g.tid; x < nListed; x += g.size) {
+                const uint32_t ci = contactAt(x);
+                const int l = listOf(ci);
+                const uint32_t pos = classBase[l] + takePlace(cls, (uint32_t)l);
+                B.contactItems[(size_t)l * B.contactItemStride + pos] = make_uint2(w, ci);
+            }
+            g.sync();
         }
         // The one-at-a-time lists by level; the coloring's scratch is free by now.
         for (int which = 0; which < 2; ++which) {
@@ -3054,31 +3177,53 @@ __device__ __forceinline__ bool refreshedAt(const WorldCounts& wc, int sub, int 
 
 // The contact half of a refresh, over the worlds refreshed at this substep: other contacts are rebased,
 // fast ones collided again with the time left, and every active contact's axes built again. One thread per
-// contact; the contacts come from one flat list, a pair class of fast contacts (Cls) or the other active
-// contacts (kClassAny). The body half runs in the substeps around it: the substep before updates the world
-// inverse inertia at its end, the substep after resets dp and dq before anything reads them.
-template <int Cls>
-__device__ __forceinline__ void refreshClass(const Batch& B, const StepParams& P, int sub) {
-    const int n = P.substeps;
-    const uint8_t againFlag = sub == n / 2 ? kFlagFast : kFlagFastSolid;
-    const float remaining = (float)(n - sub) * P.h;
-    const int list = Cls == kClassAny ? kPairClasses : Cls;
-    const uint32_t items = *(volatile uint32_t*)(B.work + kSlotFastItems + list);
-    const uint2* its = B.contactItems + (size_t)list * B.contactItemStride;
+// contact; the contacts come from one flat list, a pair class of fast contacts (refreshClass) or the other active
+// contacts (refreshLight, listed in the order of their records). The body half runs in the substeps around it: the
+// substep before updates the world inverse inertia at its end, the substep after resets dp and dq before anything
+// reads them.
+__device__ __forceinline__ void refreshLight(const Batch& B, const StepParams& P, int sub) {
+    const uint32_t items = *(volatile uint32_t*)(B.work + kSlotFastItems + kPairClasses);
+    const uint2* its = B.contactItems + (size_t)kPairClasses * B.contactItemStride;
     for (uint32_t item = blockIdx.x * blockDim.x + threadIdx.x; item < items; item += gridDim.x * blockDim.x) {
         const uint2 it = its[item];
         const WorldCounts& wc = B.counts[it.x];
-        if (!refreshedAt(wc, sub, n)) { continue; }
+        if (!refreshedAt(wc, sub, P.substeps)) { continue; }
+        const WorldInfo& wi = B.info[it.x];
+        if (!contactOk(B, wi, wc, it.y, 16)) { continue; }
+        const uint32_t slot = B.slotOf[wi.contactFirst + it.y];
+        if (slot != kNoSlot) {
+            rebaseRow(B, slot);
+            continue;
+        }
+        DContact& c = B.contacts[wi.contactFirst + it.y];
+        const DBody& a = B.bodies[c.bodyA];
+        const DBody& b = B.bodies[c.bodyB];
+        rebaseContact(a, b, c);
+        makeContactAxes(axisBodyOf(a), axisBodyOf(b), c, B.axes + (size_t)(wi.contactFirst + it.y) * kAxesPerContact);
+    }
+}
+
+template <int Cls>
+__device__ __forceinline__ void refreshClass(const Batch& B, const StepParams& P, int sub, uint32_t turn = 0, uint32_t turns = 1) {
+    const int n = P.substeps;
+    const uint8_t againFlag = sub == n / 2 ? kFlagFast : kFlagFastSolid;
+    const float remaining = (float)(n - sub) * P.h;
+    const uint32_t items = *(volatile uint32_t*)(B.work + kSlotFastItems + Cls);
+    const uint2* its = B.contactItems + (size_t)Cls * B.contactItemStride;
+    forSpreadItems(items, turn, turns, [&](uint32_t item, bool mine, bool) {
+        if (!mine) { return; }
+        const uint2 it = its[item];
+        const WorldCounts& wc = B.counts[it.x];
+        if (!refreshedAt(wc, sub, n)) { return; }
         const WorldInfo wi = B.info[it.x];
         const uint32_t ci = it.y;
-        if (!contactOk(B, wi, wc, ci, 16)) { continue; }
+        if (!contactOk(B, wi, wc, ci, 16)) { return; }
         DContact& c = B.contacts[wi.contactFirst + ci];
-        bool again = false;
-        if constexpr (Cls != kClassAny) { again = (B.cflags[wi.contactFirst + ci] & againFlag) != 0; }
+        const bool again = (B.cflags[wi.contactFirst + ci] & againFlag) != 0;
         if constexpr (Cls == kClassMesh) {
             // The contacts of a mesh pair share a key and sit together; the first takes the whole run.
             const DContact* cs = B.contacts + wi.contactFirst;
-            if (ci > 0 && cs[ci - 1].key == c.key) { continue; }
+            if (ci > 0 && cs[ci - 1].key == c.key) { return; }
             uint32_t end = ci + 1;
             while (end < wc.contactCount && cs[end].key == c.key) { ++end; }
             DContact* run = B.contacts + wi.contactFirst + ci;
@@ -3090,15 +3235,16 @@ __device__ __forceinline__ void refreshClass(const Batch& B, const StepParams& P
                 for (int x = 0; x < count; ++x) { rebaseContact(B.bodies[run[x].bodyA], B.bodies[run[x].bodyB], run[x]); }
             }
             for (int x = 0; x < count; ++x) { rebuildSolverData(B, wi, ci + x, run[x]); }
-            continue;
+            return;
         }
         takeImpulsesBack(B, wi, ci, c);
-        if constexpr (Cls != kClassAny) {
-            if (again) { refreshContact<Cls>(B, P, c, remaining); }
+        if (again) {
+            refreshContact<Cls>(B, P, c, remaining);
+        } else {
+            rebaseContact(B.bodies[c.bodyA], B.bodies[c.bodyB], c);
         }
-        if (!again) { rebaseContact(B.bodies[c.bodyA], B.bodies[c.bodyB], c); }
         rebuildSolverData(B, wi, ci, c);
-    }
+    });
 }
 
 // The fast mesh pairs' contacts, a warp per item (the first contact of a pair's run takes the run), the warp's
@@ -3151,6 +3297,8 @@ __global__ void __launch_bounds__(256) k_refresh(const __grid_constant__ Batch B
     if (stepAborted(B, serial)) { return; }
     if constexpr (Cls == kClassMesh) {
         refreshMeshPairs(B, P, sub);
+    } else if constexpr (Cls == kClassAny) {
+        refreshLight(B, P, sub);
     } else {
         refreshClass<Cls>(B, P, sub);
     }
@@ -3162,13 +3310,16 @@ template <int Unused = 0>
 __global__ void __launch_bounds__(256) k_refresh_all(const __grid_constant__ Batch B, const __grid_constant__ StepParams P,
                                                      int sub, int serial) {
     if (stepAborted(B, serial)) { return; }
-    refreshClass<kClassAny>(B, P, sub);
-    refreshClass<kClassSpheres>(B, P, sub);
-    refreshClass<kClassSpherePoly>(B, P, sub);
-    refreshClass<kClassPlane>(B, P, sub);
-    refreshClass<kClassConvex>(B, P, sub);
-    refreshClass<kClassPlanar>(B, P, sub);
-    refreshClass<kClassMesh>(B, P, sub);
+    // Most steps of most scenes have nothing to refresh: one look at every list's length.
+    const uint32_t lane = threadIdx.x & 31;
+    if (!__any_sync(0xffffffffu, lane <= kPairClasses && *(volatile uint32_t*)(B.work + kSlotFastItems + lane) != 0)) { return; }
+    refreshLight(B, P, sub);
+    refreshClass<kClassSpheres>(B, P, sub, 1, 7);
+    refreshClass<kClassSpherePoly>(B, P, sub, 2, 7);
+    refreshClass<kClassPlane>(B, P, sub, 3, 7);
+    refreshClass<kClassConvex>(B, P, sub, 4, 7);
+    refreshClass<kClassPlanar>(B, P, sub, 5, 7);
+    refreshClass<kClassMesh>(B, P, sub, 6, 7);
 }
 
 // One pass over a world's joints, before the contacts of that pass (src/world.cpp:1670-1680,
