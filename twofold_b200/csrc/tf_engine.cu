@@ -1973,18 +1973,19 @@ public:
         B.cx.tol = P.tol;
         const bool rec = profiling && !capturing;
         auto threads = [&](int k) { return (int)shapes[k].threads; };
+        auto bigThreads = [&](int k) { return shapes[k].chosen ? threads(k) : std::max(threads(k), 256); };
         auto smem = [&](int k) { return (size_t)splits[k].smemBytes; };
         cudaMemsetAsync(dWork.ptr, 0, kSlotCount * sizeof(uint32_t), stream);
         if (marks) { cudaEventRecord(marks[0], stream); }
         const bool clusters = bigCtas > 0;                              // big worlds have launches of their own
         const bool others = !clusters || bigWorlds.size() < worlds.size();  // and other worlds are left
         timed(0, rec, [&] {
-            if (clusters) { launchClusters(kKBroadBig, threads(0), B, P, serial); }
+            if (clusters) { launchClusters(kKBroadBig, bigThreads(0), B, P, serial); }
             if (others) { launch(kKBroadphase, grids[0], threads(0), smem(0), B, P, splits[0], serial); }
             if (!bigWorlds.empty()) {
                 launch(kKBroadPairs, smCount * 8, 256, 0, B, serial);
                 if (clusters) {
-                    launchClusters(kKBroadFinishBig, threads(0), B, splits[0], serial);
+                    launchClusters(kKBroadFinishBig, bigThreads(0), B, splits[0], serial);
                 } else {
                     launch(kKBroadFinish, grids[0], threads(0), 0, B, splits[0], serial);
                 }
@@ -2002,13 +2003,13 @@ public:
             });
         });
         timed(1, rec, [&] {
-            if (clusters) { launchClusters(kKNarrowphaseBig, threads(1), B, P, splits[1], serial); }
+            if (clusters) { launchClusters(kKNarrowphaseBig, bigThreads(1), B, P, splits[1], serial); }
             if (others) { launch(kKNarrowphase, grids[1], threads(1), 0, B, P, splits[1], serial); }
         });
         timed(2, rec, [&] { launch(kKWake, grids[2], threads(2), 0, B, splits[2], serial); });
         if (marks) { cudaEventRecord(marks[2], stream); }
         timed(3, rec, [&] {
-            if (clusters) { launchClusters(kKPrepareBig, threads(3), B, P, splits[3], serial); }
+            if (clusters) { launchClusters(kKPrepareBig, bigThreads(3), B, P, splits[3], serial); }
             if (others) { launch(kKPrepare, grids[3], threads(3), smem(3), B, P, splits[3], serial); }
         });
         if (recording && !capturing) {
@@ -2043,7 +2044,7 @@ public:
             });
         }
         timed(6, rec, [&] {
-            if (clusters) { launchClusters(hasJoints ? kKFinishJointsBig : kKFinishBig, threads(6), B, P, splits[6], serial); }
+            if (clusters) { launchClusters(hasJoints ? kKFinishJointsBig : kKFinishBig, bigThreads(6), B, P, splits[6], serial); }
             if (others) { launch(hasJoints ? kKFinishJoints : kKFinish, grids[6], threads(6), smem(6), B, P, splits[6], serial); }
         });
         if (marks) { cudaEventRecord(marks[3], stream); }
@@ -2150,25 +2151,31 @@ public:
     }
 
     // Default launch shapes: batches of few worlds give every world a whole CTA (512 threads when a world
-    // has more than 512 bodies); batches of many worlds give worlds of up to 96 bodies a warp each and the
-    // larger ones the CTA. 64 KB of staging per CTA leaves room for three CTAs on an SM.
+    // has more than 512 bodies); batches of many worlds give worlds of up to 32 bodies a warp each and the
+    // larger ones a CTA of 128 threads, with 32 KB of staging. Measured against 256 threads, 64 KB and a warp each up to
+    // 96 bodies, us a step: 1024 impact worlds of 66 bodies: broadphase 130 and 168, narrowphase 207 and 322, prepare
+    // 564 and 673, finish 364 and 501; 4096 uneven worlds of 8 to 232: 210 and 250, 95 and 125, 276 and 345, 439 and
+    // 457; 1024 jointed worlds of 26: 25 and 26, 11 and 11, 22 and 21, 171 and 175.
     //
     // The substep's, measured (us of substeps a step). Many worlds take 128 threads and a CTA past 32 bodies (4096
     // uneven worlds: 1839 at step 18 and 2348 at step 40, against 2396 and 3288 solved flat and 2148 and 2789 with 256
-    // threads and 96 bodies; 600 jointed worlds: 856 against 1045 flat), except: jointed worlds from 8 an SM on, solved flat
-    // (1400: 1326 and 1072 flat, 2000: 1544 and 1115; 1024: 1103 and 1040), and fewer than 8 worlds an
-    // SM with some past 128 bodies, which keep the flat solve that programs reading the shape in use know as their
-    // default (1024 uneven worlds: 157 flat and 155 at step 2, but 750 and 605 at step 18 and 1098 and 768 at step 40:
-    // worth tuning). A few worlds take a CTA each, unless one has so many bodies that one SM holds up the step: then
+    // threads and 96 bodies; 600 jointed worlds: 856 against 1045 flat), except: jointed worlds from 8 an SM on, solved
+    // flat (1400: 1326 and 1072 flat, 2000: 1544 and 1115; 1024: 1103 and 1040), and fewer than 8 worlds an SM with some
+    // past 128 bodies, which keep the flat solve that programs reading the shape in use know as their default (1024
+    // uneven worlds: 157 flat and 155 at step 2, but 750 and 605 at step 18 and 1098 and 768 at step 40: worth tuning). A few worlds take a CTA each, unless one has so many bodies that one SM holds up the step: then
     // the whole batch is solved flat (planar piles of 1017 bodies: 171 with a CTA and 218 flat, 4065: 413 and 279;
     // terrain of 4097: 855 and 769; pyramids of 1036 boxes: 677 and 676, 2081: 1609 and 659).
     LaunchShape defaultShape(int k) const {
         LaunchShape s;
         const bool many = manyWorlds();
         s.threads = !many && maxWorldBodies > 512 && !flatKernel(k) ? 512u : 256u;
-        s.bigBodies = many ? 96u : 0u;
+        s.bigBodies = many ? 32u : 0u;
         const bool stages = k == 0 || k == 3 || k == 5 || k == 6;
         s.smemBytes = stages ? 64u * 1024u : 0u;
+        if (many && !flatKernel(k)) {
+            s.threads = 128u;
+            s.smemBytes = stages ? 32u * 1024u : 0u;
+        }
         const bool flat = !many ? maxWorldBodies > kFlatBodies
                           : worlds.size() < (size_t)smCount * 8 ? !hasJoints && maxWorldBodies > 128 : hasJoints;
         if (k == 5 && flat) {
@@ -2176,10 +2183,6 @@ public:
             s.bigBodies = 0u;
             s.smemBytes = 0u;
             s.flat = true;
-        } else if (k == 5 && many) {
-            s.threads = 128u;
-            s.bigBodies = 32u;
-            s.smemBytes = 32u * 1024u;
         }
         return s;
     }

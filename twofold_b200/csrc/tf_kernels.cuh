@@ -1676,9 +1676,9 @@ static __device__ void narrowMesh(const Batch& B, const StepParams& P, const Wor
 // Calls f(item, whether it is one of the list's) for the items of a list spread over the whole grid, a warp's lanes at
 // once: a lane each when the list has items for every lane, and only as many lanes of a warp as it takes when it is
 // shorter, down to one. The pairs of a list take different paths through the same code, which a warp walks one after the
-// other: of few pairs, each gets a warp to itself. (28 pairs of boxes: 40 us of collisions a step on
-// one warp, 26 spread; 64 uneven worlds: 85 and 54, their refreshes 230 and 165.) `turn` of `turns` lists that one launch works on moves a list's
-// first warp, so that short lists do not queue on the same warps.
+// other: of few pairs, each gets a warp to itself. (28 pairs of boxes: 40 us of collisions a step on one warp, 26 spread;
+// 64 uneven worlds: 85 and 54, their refreshes 230 and 165.) `turn` of `turns` lists that one launch works on moves a
+// list's first warp, so that short lists do not queue on the same warps.
 template <class F>
 __device__ __forceinline__ void forSpreadItems(uint32_t n, uint32_t turn, uint32_t turns, F f) {
     const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
