@@ -2082,7 +2082,7 @@ public:
 
     // The world substep's launch with rooms. A batch of more worlds than the device has warps for at a CTA a world
     // gives worlds up to 96 bodies a warp each, whatever the shape without rooms gives them: 1024 impact worlds of 66
-    // bodies take 2760 us of substeps that way and 8455 with a CTA each.
+    // bodies took 2760 us of substeps that way and 8455 with a CTA each.
     int configureRooms() {
         const LaunchShape& sh = shapes[5];
         if (sh.flat) { return TF_OK; }
