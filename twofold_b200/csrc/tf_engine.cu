@@ -2471,6 +2471,19 @@ public:
         return TF_OK;
     }
 
+    // As copyArray, the contacts that the worlds hold by `counts`.
+    int copyContacts(DevArray<DContact>& to, const DevArray<DContact>& from, const DevArray<WorldCounts>& counts) {
+        int rc = to.alloc(from.n);
+        if (rc != TF_OK) { return rc; }
+        const uint32_t nw = (uint32_t)info.size();
+        if (nw == 0 || from.n == 0) { return TF_OK; }
+        const uint32_t ctas = (uint32_t)smCount * 8, parts = std::max(1u, ctas / nw);
+        launch(kKCopyContacts, std::min(nw * parts, ctas), 256, 0, (const DContact*)from.ptr, to.ptr, (const WorldInfo*)dInfo.ptr,
+               (const WorldCounts*)counts.ptr, nw, parts);
+        TF_CUDA(cudaGetLastError());
+        return TF_OK;
+    }
+
     // Copies the dynamic device state into snapshot `slot` (stream-ordered; nothing waits).
     int saveState(int slot) {
         TF_CUDA(cudaSetDevice(device));
@@ -2481,7 +2494,7 @@ public:
         Snapshot& S = *sp;
         if ((rc = copyArray(S.bodies, dBodies)) != TF_OK) { return rc; }
         if ((rc = copyArray(S.shapes, dShapes)) != TF_OK) { return rc; }
-        if ((rc = copyArray(S.contacts, dContacts[cur])) != TF_OK) { return rc; }
+        if ((rc = copyContacts(S.contacts, dContacts[cur], dCounts)) != TF_OK) { return rc; }
         if ((rc = copyArray(S.counts, dCounts)) != TF_OK) { return rc; }
         if ((rc = copyArray(S.struck, dStruck)) != TF_OK) { return rc; }
         if ((rc = copyArray(S.wakeMark, dWakeMark)) != TF_OK) { return rc; }
@@ -2507,7 +2520,7 @@ public:
         int rc;
         if ((rc = copyArray(dBodies, S.bodies)) != TF_OK) { return rc; }
         if ((rc = copyArray(dShapes, S.shapes)) != TF_OK) { return rc; }
-        if ((rc = copyArray(dContacts[cur], S.contacts)) != TF_OK) { return rc; }
+        if ((rc = copyContacts(dContacts[cur], S.contacts, S.counts)) != TF_OK) { return rc; }
         if ((rc = copyArray(dCounts, S.counts)) != TF_OK) { return rc; }
         if ((rc = copyArray(dStruck, S.struck)) != TF_OK) { return rc; }
         if ((rc = copyArray(dWakeMark, S.wakeMark)) != TF_OK) { return rc; }
@@ -2823,7 +2836,7 @@ public:
         int rc = dSummary.alloc(4);
         if (rc != TF_OK) { return rc; }
         if (!hostSummary) { TF_CUDA(cudaMallocHost(&hostSummary, 4 * sizeof(uint32_t))); }
-        launch(kKStepSummary, 1u, 256u, 0, (const WorldCounts*)dCounts.ptr, (uint32_t)worlds.size(), dSummary.ptr);
+        launch(kKStepSummary, 1u, 1024u, 0, (const WorldCounts*)dCounts.ptr, (uint32_t)worlds.size(), dSummary.ptr);
         ++launches;
         TF_CUDA(cudaGetLastError());
         TF_CUDA(cudaMemcpyAsync(hostSummary, dSummary.ptr, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));

@@ -14,6 +14,7 @@ const void* finishKernels(int id) {
         case kKAddForces: return (const void*)k_add_forces<0>;
         case kKPackPoses: return (const void*)k_pack_poses<0>;
         case kKStepSummary: return (const void*)k_step_summary<0>;
+        case kKCopyContacts: return (const void*)k_copy_contacts<0>;
         default: return nullptr;
     }
 }

@@ -36,6 +36,7 @@ enum KernelId : int {
     kKAddForces,
     kKPackPoses,
     kKStepSummary,
+    kKCopyContacts,
     kKSubstepFlat,
     kKSubstepFlatJoints,
     kKernelIds
