@@ -372,8 +372,34 @@ public:
     // Launches kernel `id` on the engine's stream; the arguments must have the kernel's parameter types exactly.
     template <class... Args>
     void launch(int id, unsigned grid, unsigned block, size_t smem, Args... args) {
-        launchOn(stream, id, grid, block, smem, args...);
+        // A directly launched step's kernel right behind another of them is brought onto the device while that one still
+        // runs; it starts by waiting for the other's end (stepAborted). A step of few worlds is about twenty short
+        // launches, several of which find nothing to do. Measured, us of four steps without and with it: 8 boxes 1550 and
+        // 1495, 96 hulls 1385 and 1333, box pyramid 3040 and 2954, 16 uneven worlds 2635 and 2575, 64 jointed worlds 2900
+        // and 2860. Where the worlds fill the device the next kernel's CTAs are in the way (256 jointed worlds 3615 and
+        // 3780, 1024 impact worlds 17175 and 17475), and a graph's launches are as close without (8 boxes 1360 and 1390,
+        // 64 jointed worlds 2630 and 3013): neither does.
+        const bool step = id < kKTapeRecord;
+        if (step && chained && chains) {
+            void* ptrs[] = { (void*)&args... };
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(grid);
+            cfg.blockDim = dim3(block);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = stream;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            cudaLaunchKernelExC(&cfg, kernelEntry(id), ptrs);
+        } else {
+            launchOn(stream, id, grid, block, smem, args...);
+        }
+        chained = step;
     }
+    bool chained = false;  // the last thing issued on the stream is one of the step's kernels
+    bool chains = false;   // the step's launches are chained
     template <class... Args>
     void launchOn(cudaStream_t on, int id, unsigned grid, unsigned block, size_t smem, Args... args) {
         void* ptrs[] = { (void*)&args... };
@@ -386,6 +412,7 @@ public:
     // refresh of the terrain: 900 us as the sum of its lists, 550 side by side).
     template <class F>
     void sideBySide(int n, F&& f) {
+        chained = false;
         cudaEventRecord(forkEvent, stream);
         for (int k = 1; k < n; ++k) {
             cudaStreamWaitEvent(sideStreams[k - 1], forkEvent, 0);
@@ -394,12 +421,14 @@ public:
         }
         f(0, stream);
         for (int k = 1; k < n; ++k) { cudaStreamWaitEvent(stream, joinEvents[k - 1], 0); }
+        chained = false;
     }
 
     // A cooperative launch (every CTA resident at once, which the flat solve's grid barrier needs); grid must
     // not exceed what fits on the device.
     template <class... Args>
     void launchCooperative(int id, unsigned grid, unsigned block, Args... args) {
+        chained = false;
         void* ptrs[] = { (void*)&args... };
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
@@ -417,6 +446,7 @@ public:
     // A launch of a cluster of bigCtas CTAs for every big world.
     template <class... Args>
     void launchClusters(int id, unsigned block, Args... args) {
+        chained = false;
         void* ptrs[] = { (void*)&args... };
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)bigWorlds.size() * bigCtas);
@@ -443,8 +473,10 @@ public:
                 KernelTimer& t = (*captureTimers)[captureUsed++];
                 t.kind = kind;
                 cudaEventRecordWithFlags(t.start, stream, cudaEventRecordExternal);
+                chained = false;
                 launch();
                 cudaEventRecordWithFlags(t.stop, stream, cudaEventRecordExternal);
+                chained = false;
                 return;
             }
             launch();
@@ -463,8 +495,10 @@ public:
             }
         }
         cudaEventRecord(eventPool[eventsUsed], stream);
+        chained = false;
         launch();
         cudaEventRecord(eventPool[eventsUsed + 1], stream);
+        chained = false;
         eventKind[eventsUsed] = kind;
         eventsUsed += 2;
     }
@@ -1972,11 +2006,18 @@ public:
         Batch B = batch(into);
         B.cx.tol = P.tol;
         const bool rec = profiling && !capturing;
+        chains = !capturing && worlds.size() <= (size_t)smCount / 2;
         auto threads = [&](int k) { return (int)shapes[k].threads; };
         auto bigThreads = [&](int k) { return shapes[k].chosen ? threads(k) : std::max(threads(k), 256); };
         auto smem = [&](int k) { return (size_t)splits[k].smemBytes; };
+        auto mark = [&](int k) {
+            if (!marks) { return; }
+            cudaEventRecord(marks[k], stream);
+            chained = false;
+        };
         cudaMemsetAsync(dWork.ptr, 0, kSlotCount * sizeof(uint32_t), stream);
-        if (marks) { cudaEventRecord(marks[0], stream); }
+        chained = false;
+        mark(0);
         const bool clusters = bigCtas > 0;                              // big worlds have launches of their own
         const bool others = !clusters || bigWorlds.size() < worlds.size();  // and other worlds are left
         timed(0, rec, [&] {
@@ -1991,7 +2032,7 @@ public:
                 }
             }
         });
-        if (marks) { cudaEventRecord(marks[1], stream); }
+        mark(1);
         timed(7, rec, [&] {
             if (smallBatch) {
                 launch(kKCollideAll, *std::max_element(flatGrids, flatGrids + kPairClasses), threads(7), 0, B, P, serial);
@@ -2007,7 +2048,7 @@ public:
             if (others) { launch(kKNarrowphase, grids[1], threads(1), 0, B, P, splits[1], serial); }
         });
         timed(2, rec, [&] { launch(kKWake, grids[2], threads(2), 0, B, splits[2], serial); });
-        if (marks) { cudaEventRecord(marks[2], stream); }
+        mark(2);
         timed(3, rec, [&] {
             if (clusters) { launchClusters(kKPrepareBig, bigThreads(3), B, P, splits[3], serial); }
             if (others) { launch(kKPrepare, grids[3], threads(3), smem(3), B, P, splits[3], serial); }
@@ -2047,7 +2088,7 @@ public:
             if (clusters) { launchClusters(hasJoints ? kKFinishJointsBig : kKFinishBig, bigThreads(6), B, P, splits[6], serial); }
             if (others) { launch(hasJoints ? kKFinishJoints : kKFinish, grids[6], threads(6), smem(6), B, P, splits[6], serial); }
         });
-        if (marks) { cudaEventRecord(marks[3], stream); }
+        mark(3);
         launches += smallBatch ? 5 + 1 + P.substeps + (P.substeps - 1)
                                : 5 + kPairClasses + P.substeps + (kPairClasses + 1) * (P.substeps - 1);
         launches += (bigWorlds.empty() ? 0 : 2) + (clusters && others ? 4 : 0) + (shapes[5].flat ? 0 : P.substeps);

@@ -335,11 +335,15 @@ __device__ uint32_t groupExpand(const G& g, uint32_t n, Count count, Emit emit) 
     return base;
 }
 
-// Reads the abort word once per CTA (with Cluster, once per cluster: its CTAs have to agree) at a kernel's start: true when an earlier step of this launch sequence
-// overflowed a list, or this step did in an earlier kernel.
+// What every kernel of a step does first. The kernel behind it in the step may be brought onto the device from now on,
+// and nothing goes on before the kernels ahead of it are over and their writes can be seen. Then the abort word is read
+// once per CTA (with Cluster, once per cluster: its CTAs have to agree): true when an earlier step of this launch
+// sequence overflowed a list, or this step did in an earlier kernel.
 template <bool Cluster = false>
 __device__ __forceinline__ bool stepAborted(const Batch& B, int serial) {
     __shared__ int s_skip;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if constexpr (Cluster) {
         const GroupOf<true> g = makeClusterGroup();
         if (g.tid == 0) { s_skip = *(volatile uint32_t*)B.abortStep <= (uint32_t)serial; }
