@@ -1,10 +1,11 @@
 // The step kernels. Each kernel walks whole worlds with thread groups: a group (one warp, or 64 to 512
 // threads) steps one world at a time, and groups take worlds in largest-first order from a per-launch
 // counter, so small worlds pack many to an SM and large ones get whole CTAs. Within a world a group's threads
-// split bodies, candidates or one color's contacts, with a group barrier between dependent phases. Work that
-// the reference does in one sequential pass whose result depends on order (graph coloring, union-find unions,
-// the wake flood and contacts solved one at a time) runs on the group's first thread, in the reference's
-// order, over shared memory when the world fits the group's slice and over L1/L2-cached scratch otherwise.
+// split bodies, candidates or one color's contacts, with a group barrier between dependent phases, over shared memory
+// when the world fits the group's slice and over L1/L2-cached scratch otherwise. Worlds of more than 1024 bodies have a
+// cluster of CTAs each. Work that the reference does in one sequential pass whose result depends on order (coloring,
+// unions, joints, contacts solved one at a time) runs in rounds or levels that give each item what the pass gives it;
+// the wake flood, which is rare, runs on the group's first thread in the reference's order.
 //
 // Kernel sequence of one step (src/world.cpp:1564-1727):
 //   k_broadphase   growth, body-pair and half-space candidates, sorted unique keys (world.cpp:752-870)

@@ -9,9 +9,8 @@
 // (src/world.cpp:868-869). The step's other rules (category/mask filters, jointed pairs, half-space pairs)
 // are not applied: the inputs carry no filters, joints or planes.
 //
-// Scratch: g_pairScratch below, a fixed-size array in the library's device image. Its address on a device is
-// looked up once, with that device current, on the first call made there; later calls on that device reuse
-// it, so the library must not be called on a device again after a cudaDeviceReset there. Nothing here
+// Scratch: g_pairScratch below, a fixed-size array in the library's device image, its address looked up on every call
+// (a context made after a device reset may place the module elsewhere). Nothing here
 // allocates device or host memory through CUDA or any other library. Because the scratch is one per device,
 // calls whose work overlaps on the device (different streams, or different host threads) race on it and give
 // wrong results; issue them on one stream or serialise them.
