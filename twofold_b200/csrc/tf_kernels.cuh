@@ -616,6 +616,25 @@ __device__ __forceinline__ float sweepSlack(float x) { return 1e-3f + 1e-6f * fa
 // body of the terrain's 32 x 32 columns met the 1,500 bodies of its x range: 65 million tests, 1.9 ms.)
 constexpr uint32_t kBodyWide = 8u;
 
+// The range of a big world's intervals along x and along its second axis, from the keys alone.
+struct SweepRange {
+    float lo[2], hi[2];
+    int axis;  // the second axis
+};
+
+__device__ __forceinline__ SweepRange sweepRange(const WorldCounts& wc) {
+    float lo[3], hi[3];
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = fromOrderedKey(wc.sweepMinKey[k]);
+        hi[k] = fromOrderedKey(wc.sweepMaxKey[k]);
+    }
+    SweepRange r;
+    r.axis = hi[2] - lo[2] > hi[1] - lo[1] ? 2 : 1;
+    r.lo[0] = lo[0], r.hi[0] = hi[0];
+    r.lo[1] = r.axis == 2 ? lo[2] : lo[1], r.hi[1] = r.axis == 2 ? hi[2] : hi[1];
+    return r;
+}
+
 struct SweepGrid {
     float lo[2], scale[2];
     uint32_t cells[2];
@@ -623,23 +642,19 @@ struct SweepGrid {
     float width;  // no body that is not wide is wider along it
 };
 
+// The grid of a world whose wide bodies are counted.
 __device__ __forceinline__ SweepGrid sweepGrid(const WorldInfo& wi, const WorldCounts& wc) {
+    const SweepRange r = sweepRange(wc);
     SweepGrid s;
-    float lo[3], hi[3];
-    for (int k = 0; k < 3; ++k) {
-        lo[k] = fromOrderedKey(wc.sweepMinKey[k]);
-        hi[k] = fromOrderedKey(wc.sweepMaxKey[k]);
-    }
-    s.axis = hi[2] - lo[2] > hi[1] - lo[1] ? 2 : 1;
+    s.axis = r.axis;
     const bool flat = wc.sweepWide > wi.bodyCount / 16;
     const uint32_t side = (uint32_t)sqrtf((float)(wi.bodyCount / 4 + 1));
     s.cells[0] = flat ? wi.bodyCount / 4 + 1 : side;
     s.cells[1] = flat ? 1u : side;
-    const float a = lo[0], b = hi[0], c = s.axis == 2 ? lo[2] : lo[1], d = s.axis == 2 ? hi[2] : hi[1];
-    s.lo[0] = a;
-    s.lo[1] = c;
-    s.scale[0] = b > a ? (float)s.cells[0] / (b - a) : 0.0f;
-    s.scale[1] = d > c ? (float)s.cells[1] / (d - c) : 0.0f;
+    for (int k = 0; k < 2; ++k) {
+        s.lo[k] = r.lo[k];
+        s.scale[k] = r.hi[k] > r.lo[k] ? (float)s.cells[k] / (r.hi[k] - r.lo[k]) : 0.0f;
+    }
     s.width = __uint_as_float(wc.sweepWidth);
     return s;
 }
@@ -698,16 +713,18 @@ static __device__ void prepareSweep(const Batch& B, const G& g, const WorldInfo&
         }
     }
     g.sync();
-    SweepGrid grid = sweepGrid(wi, wc);
+    // Every thread takes the axis and what counts as wide from the keys, which stand: faster threads add to the count of
+    // wide bodies, and with it to what the grid will be, while others are still here.
+    const SweepRange span = sweepRange(wc);
     auto second = [&](uint32_t i, float& lo, float& hi) {
         const uint32_t gb = wi.bodyFirst + i;
         const DBody& b = B.bodies[gb];
         lo = FLT_MAX, hi = -FLT_MAX;
         if (!b.alive || !b.hasBounds) { return; }
         const Vec3 bl = b.lo, bh = b.hi;
-        sweepInterval(grid.axis == 2 ? bl.z : bl.y, grid.axis == 2 ? bh.z : bh.y, B.grow[gb], lo, hi);
+        sweepInterval(span.axis == 2 ? bl.z : bl.y, span.axis == 2 ? bh.z : bh.y, B.grow[gb], lo, hi);
     };
-    const float range = (float)grid.cells[1] / grid.scale[1];
+    const float range = span.hi[1] - span.lo[1];
     auto wideAt = [&](float lo, float hi) { return !((hi - lo) * 8.0f < range); };
     uint32_t wide = 0, width = 0;
     for (uint32_t i = g.tid; i < n; i += g.size) {
@@ -727,7 +744,7 @@ static __device__ void prepareSweep(const Batch& B, const G& g, const WorldInfo&
         atomicMax(&wc.sweepWidth, width);
     }
     g.sync();
-    grid = sweepGrid(wi, wc);
+    const SweepGrid grid = sweepGrid(wi, wc);
     const uint32_t cells = grid.cells[0] * grid.cells[1];
     uint32_t* start = B.sweepStart + wi.bodyFirst + w;
     auto cellOf = [&](uint32_t i) {
