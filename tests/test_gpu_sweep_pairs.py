@@ -102,3 +102,22 @@ def test_pairs_of_big_worlds():
         for k in range(len(worlds) * copies):
             assert np.array_equal(batch.candidates(k), expected[k % len(worlds)]), (copies, KINDS[k % len(worlds)].__name__)
         batch.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [31, 32, 33, 70])
+def test_pairs_where_the_worlds_share_the_warps(count):
+    # Worlds are taken 32 at a time, each one's items from where the last one's ended: sizes and wide bodies differ.
+    worlds = []
+    for k in range(count):
+        w = _sphere_world(1025 + 37 * (k % 5), _span(1025), 20 + k % 5)
+        if k % 5 == 2:
+            w.shapes["radius"][5:1025:100] = 0.5 * _span(1025)
+        worlds.append(w)
+    scene = scenes.Scene("spheres", worlds)
+    expected = [_expected(*_pair_inputs(w, scene.settings)) for w in worlds[:5]]
+    batch = Batch.from_scene(scene)
+    batch.step_checked(float(DT))
+    for k in range(count):
+        assert np.array_equal(batch.candidates(k), expected[k % 5]), k
+    batch.close()

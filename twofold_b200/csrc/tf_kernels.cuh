@@ -1092,9 +1092,76 @@ static __device__ void finishCandidates(const Batch& B, const G& g, const WorldI
 // The pair half of a big world's broadphase: each body takes the bodies whose intervals along x start within its own
 // (the one starting first takes a pair, so each pair is taken once) among the wide ones and those of the cells whose
 // bodies can reach it along the second axis, and applies the same pair test as the small worlds, in the pair's
-// lower-body-first order. A warp per body, its lanes across the contiguous run of records of each x column, over
-// every big world; a wide body's run is the whole of its x range, a warp a part of it (kSweepPart).
+// lower-body-first order. A warp per body, its lanes across the contiguous run of records of each x column; a wide
+// body's run is the whole of its x range, a warp a part of it (kSweepPart). The worlds' items are one list that the
+// warps take in turn. (Each world's items started at warp 0 once, so that 76 worlds queued on the same ninth of the
+// device: 1029 us of broadphase a step for 76 planar worlds of 1119 bodies and 558 for 40, 164 and 128 as one list; 712
+// and 295 for 76 pyramids of 1036.)
 constexpr uint32_t kSweepPart = 1024;  // records of a wide body's run a warp takes
+
+// A big world's wide bodies, none when its grid has x columns only, and what its pairs are taken by: its records, then
+// the wide ones' parts.
+__device__ __forceinline__ uint32_t sweepWides(const WorldInfo& wi, const WorldCounts& wc) {
+    return wc.sweepWide > wi.bodyCount / 16 ? 0u : wc.sweepWide;
+}
+__device__ __forceinline__ uint32_t sweepParts(const WorldInfo& wi) { return (wi.bodyCount + kSweepPart - 1) / kSweepPart; }
+
+// The items from first on, every step-th one, of one world.
+static __device__ __forceinline__ void pairsOfWorld(const Batch& B, uint32_t w, uint32_t first, uint32_t items, uint32_t step,
+                                                    uint32_t lane) {
+    const WorldInfo wi = B.info[w];
+    WorldCounts& wc = B.counts[w];
+    const uint32_t n = wi.bodyCount, parts = sweepParts(wi), wide = sweepWides(wi, wc);
+    const SweepRec* recs = B.sweepRecs + wi.bodyFirst;
+    const uint32_t* start = B.sweepStart + wi.bodyFirst + w;
+    const uint32_t* wides = B.sweepOrder + wi.bodyFirst;
+    const SweepGrid grid = sweepGrid(wi, wc);
+    for (uint32_t item = first; item < items; item += step) {
+        const bool part = item >= n;
+        const SweepRec ri = recs[part ? wides[(item - n) / parts] : item];
+        if (!(ri.flags & kBodyLive)) { continue; }
+        const float lo = ri.start, hi = B.sweepHi[wi.bodyFirst + ri.body];
+        auto test = [&](const SweepRec& rj) {
+            const uint32_t i = ri.body, j = rj.body;
+            if (j == i || !(rj.start > lo || (rj.start == lo && j > i)) || rj.start > hi) { return; }
+            const SweepRec& A = i < j ? ri : rj;
+            const SweepRec& Bb = i < j ? rj : ri;
+            if (!(A.flags & kBodyLive) || !(Bb.flags & kBodyLive)) { return; }
+            if (!((A.flags | Bb.flags) & kBodyDynamic)) { return; }
+            if (!((A.flags | Bb.flags) & kBodyMoving)) { return; }
+            const float gg = A.grow + Bb.grow;
+            const Vec3 reach{ gg, gg, gg };
+            if (!boxesOverlap(A.lo - reach, A.hi + reach, Bb.lo, Bb.hi)) { return; }
+            pairShapes(B, wi, B.bodies[wi.bodyFirst + A.body], B.bodies[wi.bodyFirst + Bb.body], A.grow, Bb.grow, A.lo,
+                       A.hi, Bb.lo, Bb.hi, reach, &wc.candRaw);
+        };
+        const uint32_t x0 = sweepCell(grid, 0, lo), x1 = sweepCell(grid, 0, hi);
+        if (part) {
+            const uint32_t c0 = x0 * grid.cells[1], c1 = (x1 + 1) * grid.cells[1] - 1;
+            const uint32_t from = (item - n) % parts * kSweepPart;
+            const uint32_t q0 = max(from, c0 ? start[c0 - 1] : 0u), q1 = min(from + kSweepPart, start[c1]);
+            for (uint32_t q = q0 + lane; q < q1; q += 32) {
+                const SweepRec rj = recs[q];
+                if (!(rj.flags & kBodyWide)) { test(rj); }
+            }
+            continue;
+        }
+        for (uint32_t q = lane; q < wide; q += 32) { test(recs[wides[q]]); }
+        if (ri.flags & kBodyWide) { continue; }  // its parts take the others
+        float from, to;
+        sweepInterval(grid.axis == 2 ? ri.lo.z : ri.lo.y, grid.axis == 2 ? ri.hi.z : ri.hi.y, ri.grow, from, to);
+        const uint32_t y0 = grid.cells[1] > 1 ? sweepCell(grid, 1, from - grid.width * 1.001f) : 0u;
+        const uint32_t y1 = grid.cells[1] > 1 ? sweepCell(grid, 1, to) : 0u;
+        for (uint32_t x = x0; x <= x1; ++x) {
+            const uint32_t c0 = x * grid.cells[1] + y0, c1 = x * grid.cells[1] + y1;
+            const uint32_t q1 = start[c1];
+            for (uint32_t q = (c0 ? start[c0 - 1] : 0u) + lane; q < q1; q += 32) {
+                const SweepRec rj = recs[q];
+                if (!(rj.flags & kBodyWide)) { test(rj); }
+            }
+        }
+    }
+}
 
 template <int Unused = 0>
 __global__ void __launch_bounds__(256) k_broad_pairs(const __grid_constant__ Batch B, int serial) {
@@ -1102,61 +1169,25 @@ __global__ void __launch_bounds__(256) k_broad_pairs(const __grid_constant__ Bat
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    for (uint32_t k = 0; k < B.nBigWorlds; ++k) {
-        const uint32_t w = B.bigWorlds[k];
-        const WorldInfo wi = B.info[w];
-        WorldCounts& wc = B.counts[w];
-        const uint32_t n = wi.bodyCount, parts = (n + kSweepPart - 1) / kSweepPart;
-        const SweepRec* recs = B.sweepRecs + wi.bodyFirst;
-        const uint32_t* start = B.sweepStart + wi.bodyFirst + w;
-        const uint32_t* wides = B.sweepOrder + wi.bodyFirst;
-        const SweepGrid grid = sweepGrid(wi, wc);
-        const uint32_t wide = grid.cells[1] > 1 ? wc.sweepWide : 0u;
-        // Items: the records, then the wide ones' parts.
-        for (uint32_t item = warp; item < n + wide * parts; item += warps) {
-            const bool part = item >= n;
-            const SweepRec ri = recs[part ? wides[(item - n) / parts] : item];
-            if (!(ri.flags & kBodyLive)) { continue; }
-            const float lo = ri.start, hi = B.sweepHi[wi.bodyFirst + ri.body];
-            auto test = [&](const SweepRec& rj) {
-                const uint32_t i = ri.body, j = rj.body;
-                if (j == i || !(rj.start > lo || (rj.start == lo && j > i)) || rj.start > hi) { return; }
-                const SweepRec& A = i < j ? ri : rj;
-                const SweepRec& Bb = i < j ? rj : ri;
-                if (!(A.flags & kBodyLive) || !(Bb.flags & kBodyLive)) { return; }
-                if (!((A.flags | Bb.flags) & kBodyDynamic)) { return; }
-                if (!((A.flags | Bb.flags) & kBodyMoving)) { return; }
-                const float gg = A.grow + Bb.grow;
-                const Vec3 reach{ gg, gg, gg };
-                if (!boxesOverlap(A.lo - reach, A.hi + reach, Bb.lo, Bb.hi)) { return; }
-                pairShapes(B, wi, B.bodies[wi.bodyFirst + A.body], B.bodies[wi.bodyFirst + Bb.body], A.grow, Bb.grow, A.lo,
-                           A.hi, Bb.lo, Bb.hi, reach, &wc.candRaw);
-            };
-            const uint32_t x0 = sweepCell(grid, 0, lo), x1 = sweepCell(grid, 0, hi);
-            if (part) {
-                const uint32_t c0 = x0 * grid.cells[1], c1 = (x1 + 1) * grid.cells[1] - 1;
-                const uint32_t from = (item - n) % parts * kSweepPart;
-                const uint32_t q0 = max(from, c0 ? start[c0 - 1] : 0u), q1 = min(from + kSweepPart, start[c1]);
-                for (uint32_t q = q0 + lane; q < q1; q += 32) {
-                    const SweepRec rj = recs[q];
-                    if (!(rj.flags & kBodyWide)) { test(rj); }
-                }
-                continue;
-            }
-            for (uint32_t q = lane; q < wide; q += 32) { test(recs[wides[q]]); }
-            if (ri.flags & kBodyWide) { continue; }  // its parts take the others
-            float from, to;
-            sweepInterval(grid.axis == 2 ? ri.lo.z : ri.lo.y, grid.axis == 2 ? ri.hi.z : ri.hi.y, ri.grow, from, to);
-            const uint32_t y0 = grid.cells[1] > 1 ? sweepCell(grid, 1, from - grid.width * 1.001f) : 0u;
-            const uint32_t y1 = grid.cells[1] > 1 ? sweepCell(grid, 1, to) : 0u;
-            for (uint32_t x = x0; x <= x1; ++x) {
-                const uint32_t c0 = x * grid.cells[1] + y0, c1 = x * grid.cells[1] + y1;
-                const uint32_t q1 = start[c1];
-                for (uint32_t q = (c0 ? start[c0 - 1] : 0u) + lane; q < q1; q += 32) {
-                    const SweepRec rj = recs[q];
-                    if (!(rj.flags & kBodyWide)) { test(rj); }
-                }
-            }
+    uint32_t before = 0;  // items of the worlds before
+    for (uint32_t k0 = 0; k0 < B.nBigWorlds; k0 += 32) {
+        // A lane a world: its items, and this warp's first among them.
+        uint32_t items = 0;
+        if (k0 + lane < B.nBigWorlds) {
+            const uint32_t w = B.bigWorlds[k0 + lane];
+            const WorldInfo& wi = B.info[w];
+            items = wi.bodyCount + sweepWides(wi, B.counts[w]) * sweepParts(wi);
+        }
+        uint32_t upTo = items;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, upTo, o);
+            if ((int)lane >= o) { upTo += y; }
+        }
+        const uint32_t first = (warp + warps - (before + upTo - items) % warps) % warps;
+        before += __shfl_sync(0xffffffffu, upTo, 31);
+        for (uint32_t left = __ballot_sync(0xffffffffu, first < items); left; left &= left - 1) {
+            const int k = __ffs(left) - 1;
+            pairsOfWorld(B, B.bigWorlds[k0 + k], __shfl_sync(0xffffffffu, first, k), __shfl_sync(0xffffffffu, items, k), warps, lane);
         }
     }
 }
