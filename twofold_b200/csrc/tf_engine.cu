@@ -1495,14 +1495,18 @@ public:
 
     // A world's joints level by level: each joint one level past the last earlier joint at either of its dynamic
     // bodies, kinds together within a level. A body's type only changes with a new layout; whether it is awake, and
-    // whether a joint holds, does not matter (a joint that does nothing at a body may as well come in its turn).
+    // whether a joint holds, does not matter (a joint that does nothing at a body may as well come in its turn). No levels
+    // (0) where they hold fewer than 4 joints in 3: what a level costs beside its joint is more than the joints side by
+    // side save (forEachJoint).
     static void levelJoints(const HostWorld& W, uint32_t* order, uint32_t* levelEnd, uint32_t& levels) {
         const size_t n = W.joints.size();
         std::vector<uint32_t> last(W.bodies.size(), 0u), level(n, 0u);
+        size_t alive = 0;
         levels = 0;
         for (size_t k = 0; k < n; ++k) {
             const DJoint& j = W.joints[k].d;
             if (!j.alive) { continue; }
+            ++alive;
             for (const uint32_t b : { j.bodyA, j.bodyB }) {
                 if (b < W.bodies.size() && W.bodies[b].d.type == kDynamic) { level[k] = std::max(level[k], last[b]); }
             }
@@ -1518,6 +1522,7 @@ public:
             return level[a] != level[b] ? level[a] < level[b] : W.joints[a].d.type < W.joints[b].d.type;
         });
         for (size_t k = 0; k < n; ++k) { levelEnd[level[order[k]]] = (uint32_t)k + 1; }
+        if (3 * alive < 4 * (size_t)levels) { levels = 0; }
     }
 
     int layout() {

@@ -495,15 +495,22 @@ static __device__ void wakeJointPulled(const Batch& B, const G& g, const WorldIn
 // and every dynamic body meets its joints in index order, which is what the reference's pass in index order gives it;
 // other ends take nothing from a joint. A warp takes the joints of one kind among 32 of a level, which keeps it on one
 // code path. Bounded by the longest chain of joint solves: 256 worlds of 22 joints of every kind, chains of 6 at most,
-// take 601 us of substeps and 119 of end of step, against 868 and 202 with a world's joints on one thread.
+// take 601 us of substeps and 119 of end of step, against 868 and 202 with a world's joints on one thread. A world that
+// is nearly all one chain (WorldInfo::jointLevels is 0) has its joints on one thread, in index order: a level costs its
+// barrier and the reads that find its joints. Substeps and end of step by levels and on one thread, us a step: a chain of
+// 64, 2234 + 336 and 1677 + 289; with one of 16 beside it 2340 + 353 and 2167 + 357, with one of 32 2332 + 366 and 2676 +
+// 419; 300 worlds with chains of 6 and 2 499 + 96 and 470 + 97, of 6 and 3 478 + 95 and 519 + 105.
 template <class G, class F>
 __device__ __forceinline__ void forEachJoint(const Batch& B, const G& g, const WorldInfo& wi, F&& f) {
+    // One loop for both, with one call of f: a second copy of the joints' code put a tenth on the levels.
+    const bool chain = wi.jointLevels == 0;
+    const uint32_t levels = chain ? 1u : wi.jointLevels, stride = chain ? 1u : 32u;
     uint32_t begin = 0;
-    for (uint32_t l = 0; l < wi.jointLevels; ++l) {
-        const uint32_t end = B.jointLevel[wi.jointFirst + l];
-        for (uint32_t i = begin + g.lane, k = 0; i < end; i += 32, ++k) {
-            const uint32_t x = B.jointOrder[wi.jointFirst + i];
-            if ((k + B.joints[wi.jointFirst + x].type) % g.warps == g.warp) { f(x); }
+    for (uint32_t l = 0; l < levels; ++l) {
+        const uint32_t end = chain ? (g.tid == 0 ? wi.jointCount : 0u) : B.jointLevel[wi.jointFirst + l];
+        for (uint32_t i = begin + (chain ? 0u : g.lane), k = 0; i < end; i += stride, ++k) {
+            const uint32_t x = chain ? i : B.jointOrder[wi.jointFirst + i];
+            if (chain || (k + B.joints[wi.jointFirst + x].type) % g.warps == g.warp) { f(x); }
         }
         g.sync();
         begin = end;

@@ -283,7 +283,7 @@ struct WorldInfo {
     // Joints from jointFirst in the world's index order, and the body pairs that joints keep from colliding
     // (sorted keys min << 32 | max of world-local bodies) from the same offset.
     uint32_t jointFirst, jointCount, joinedCount;
-    uint32_t jointLevels;  // levels of the world's joints (Batch::jointOrder)
+    uint32_t jointLevels;  // levels of the world's joints (Batch::jointOrder), 0 where they are solved one after another
 };
 
 enum JointType : uint32_t { kJointPoint = 0, kJointFixed, kJointHinge, kJointSlider, kJointDistance, kJointSwingTwist };
