@@ -134,6 +134,10 @@ struct Batch {
     uint32_t* debug;
     uint32_t nPolys;
     uint32_t totalBodies;
+
+    // Where the world substep's rooms pay (contactsOutweigh): contacts a body of the batch, and of a world its bodies, and
+    // its contacts a color unless it has at most roomWarpBodies bodies and so a warp.
+    uint32_t roomContacts, roomBodies, roomWarpBodies, roomThreads;
 };
 
 #if defined(TF_DEVICE_CHECKS)

@@ -210,6 +210,8 @@ public:
     Split roomsSplit{};
     uint32_t roomsThreads = 0;
     int roomsGrid = 0;
+    static constexpr uint32_t kNoRooms = ~0u;
+    uint32_t roomContacts = kNoRooms;  // contacts a body from which that launch takes the batch
     // k_collide per pair class, then k_refresh for the light list and per pair class.
     static constexpr int kFlatGrids = 2 * kPairClasses + 1;
     int flatGrids[kFlatGrids] = {};
@@ -2001,6 +2003,10 @@ public:
         B.debug = dDebug.ptr;
         B.nPolys = (uint32_t)nPolys;
         B.totalBodies = (uint32_t)totalBodies;
+        B.roomContacts = roomContacts;
+        B.roomBodies = shapes[5].chosen || !manyWorlds() ? ~0u : roomsSplit.bigBodies;
+        B.roomWarpBodies = roomsSplit.bigBodies;
+        B.roomThreads = shapes[5].chosen ? ~0u : roomsThreads;
         return B;
     }
 
@@ -2084,8 +2090,10 @@ public:
                     launchCooperative(hasJoints ? kKSubstepFlatJoints : kKSubstepFlat, grids[5], threads(5), B, P, i, serial);
                 } else {
                     launch(hasJoints ? kKSubstepJoints : kKSubstep, grids[5], threads(5), smem(5), B, P, splits[5], i, serial);
-                    launch(hasJoints ? kKSubstepRoomsJoints : kKSubstepRooms, roomsGrid, roomsThreads,
-                           roomsSplit.smemBytes + roomsThreads / 32 * kRoomBytes, B, P, roomsSplit, i, serial);
+                    if (roomContacts != kNoRooms) {
+                        launch(hasJoints ? kKSubstepRoomsJoints : kKSubstepRooms, roomsGrid, roomsThreads,
+                               roomsSplit.smemBytes + roomsThreads / 32 * kRoomBytes, B, P, roomsSplit, i, serial);
+                    }
                 }
             });
         }
@@ -2096,7 +2104,7 @@ public:
         mark(3);
         launches += smallBatch ? 5 + 1 + P.substeps + (P.substeps - 1)
                                : 5 + kPairClasses + P.substeps + (kPairClasses + 1) * (P.substeps - 1);
-        launches += (bigWorlds.empty() ? 0 : 2) + (clusters && others ? 4 : 0) + (shapes[5].flat ? 0 : P.substeps);
+        launches += (bigWorlds.empty() ? 0 : 2) + (clusters && others ? 4 : 0) + (roomContacts == kNoRooms ? 0 : P.substeps);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) { return fail(TF_E_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e)); }
         return TF_OK;
@@ -2129,8 +2137,18 @@ public:
     // The world substep's launch with rooms. A batch of more worlds than the device has warps for at a CTA a world
     // gives worlds up to 96 bodies a warp each, whatever the shape without rooms gives them: 1024 impact worlds of 66
     // bodies took 2760 us of substeps that way and 8455 with a CTA each.
+    //
+    // An SM holds one CTA with rooms and two without, so it matters how the worlds fill the rounds of either: two contacts
+    // a body are enough up to a world an SM and in a third round, eight are needed in a second one that is mostly empty,
+    // four in one that is nearly full and in a fourth. Measured, us of substeps a step with and without, 148 SMs: 148
+    // impact worlds (7.4 contacts a body) 1114 and 1693, 170 2030 and 1739, 220 2111 and 2021, 296 2174 and 2377, 440
+    // 3189 and 4121, 590 4229 and 4691; pyramids of 79 boxes (2.7) 301 and 396, 546 and 417, 551 and 425, 558 and 443,
+    // 815 and 812, 1072 and 844; blocks of 125 boxes (8.4) 1169 and 2457, 2142 and 2533, 2157 and 2574, 2278 and 2607,
+    // 3373 and 4933, 4475 and 5135; pyramids of 211 (2.8) 358 and 494, 638 and 612, 647 and 690, 674 and 745, 968 and 1208, 1268 and
+    // 1429; of 407 520 and 758, 882 and 802, 911 and 833, 975 and 889, 1415 and 1611, 1867 and 1720.
     int configureRooms() {
         const LaunchShape& sh = shapes[5];
+        roomContacts = kNoRooms;
         if (sh.flat) { return TF_OK; }
         const void* fn = kernelEntry(hasJoints ? kKSubstepRoomsJoints : kKSubstepRooms);
         const size_t limit = dynSmemLimit[fn];
@@ -2142,7 +2160,10 @@ public:
         roomsSplit.smemBytes = (uint32_t)std::min<size_t>(std::max(sh.smemBytes, 32u * 1024u), limit - rooms) / (16 * warps) * (16 * warps);
         roomsSplit.big = stageFor(5, roomsSplit.smemBytes);
         roomsSplit.small = stageFor(5, roomsSplit.smemBytes / warps);
-        roomsGrid = std::min<int>(worldsGrid(roomsSplit.bigBodies, warps), smCount);
+        const int wanted = worldsGrid(roomsSplit.bigBodies, warps), rounds = (wanted + smCount - 1) / smCount;
+        roomsGrid = std::min(wanted, smCount);
+        const bool emptySecond = rounds == 2 && 4 * wanted <= 7 * smCount;
+        roomContacts = manyWorlds() || sh.chosen || rounds == 1 || rounds == 3 ? 2u : emptySecond ? 8u : 4u;
         return TF_OK;
     }
 

@@ -55,8 +55,8 @@ enum WorkSlot : int {
     kSlotFlatMaxRestLevels = kSlotFlatMaxImpact + 1,
     kSlotFlatMaxImpactRestLevels = kSlotFlatMaxRestLevels + 1,
     kSlotFlatBarrier = kSlotFlatMaxImpactRestLevels + 1,  // arrivals, then barriers passed
-    kSlotActive = kSlotFlatBarrier + 2,  // active contacts of every world
-    kSlotFast = kSlotActive + 1,  // whether any world has fast contacts (bit 0), any of solid bodies (bit 1)
+    kSlotRoomContacts = kSlotFlatBarrier + 2,  // active contacts of the worlds that rooms suit
+    kSlotFast = kSlotRoomContacts + 1,  // whether any world has fast contacts (bit 0), any of solid bodies (bit 1)
     kSlotCount = kSlotFast + 1
 };
 
@@ -2430,6 +2430,29 @@ __device__ void forEachLevel(const G& g, const uint32_t* list, const uint32_t* l
     }
 }
 
+// Whether a world's contacts are better solved with rooms (kRoomWarps), as far as the world itself goes: it has five
+// contact points a body (a room holds four points of a contact whether it has them or not), no more contacts a color
+// than its group has lanes (a second round waits for its records), and no more bodies than roomBodies (past it a CTA
+// without rooms shares its SM with others). Measured, us of substeps a step with rooms and without. One world: 208 boxes
+// in a pyramid (11.2 points a body, 98 contacts a color) 324 and 387, 497 (11.5 and 238) 480 and 497, 562 (270) 597 and
+// 467, 991 (480) 1150 and 601; 512 boxes in a block (27 and 197) 1534 and 1676; balls on a box, 400 (2.7 and 215) 303 and
+// 214, in a block, 216 (2.7) 207 and 185, packed tight, 343 (4.8) 422 and 390. 100 worlds of bullets and boxes (14 points
+// a body, later 5) 1407 and 1664. 1200 worlds: 79 boxes 1189 and 1473, 137 boxes 2459 and 1881, 216 in a block 10568 and
+// 7654.
+__device__ __forceinline__ bool roomsSuit(const Batch& B, const WorldInfo& wi, uint32_t points, uint32_t colored,
+                                          uint32_t colors) {
+    return points >= 5 * wi.bodyCount && wi.bodyCount <= B.roomBodies &&
+           (wi.bodyCount <= B.roomWarpBodies || colored <= (uint64_t)colors * B.roomThreads);
+}
+
+// Whether the contacts of the worlds that rooms suit outweigh the batch's bodies: the batch is solved with rooms then.
+// By how much they have to (roomContacts) depends on the launch. The lines measured lie at 7.4 contacts a body (impact
+// walls) and 2.8 (the pyramid) on one side, 0.5 and less on the other (the uneven batch's worlds: 3312 us with rooms and
+// 1952 without).
+__device__ __forceinline__ bool contactsOutweigh(const Batch& B) {
+    return *(volatile uint32_t*)(B.work + kSlotRoomContacts) >= (uint64_t)B.roomContacts * B.totalBodies;
+}
+
 // Coloring is staged in the group's shared slice (masks by body, endpoints by active contact) when the world
 // fits stageBodies bodies and stageContacts active contacts, else in the world's global scratch.
 template <bool Cluster>
@@ -2623,7 +2646,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_prepare(const __grid_constant__ B
             g.sync();
         }
         if (g.tid == 0) {
-            atomicAdd(B.work + kSlotActive, nActive);
+            if (roomsSuit(B, wi, *pointSum, nColored, wc.colorCount)) { atomicAdd(B.work + kSlotRoomContacts, nActive); }
             if (*fast > 0) { atomicOr(B.work + kSlotFast, *fastSolid > 0 ? 3u : 1u); }
             wc.activeCount = nActive;
             wc.impactCount = nImpact;
@@ -2934,10 +2957,8 @@ __device__ __forceinline__ Axis rowAxis(const Vec3& ra, const Vec3& rb, const Ve
 
 // A warp's room in shared memory for the records of the contacts it is about to solve, a lane's own record words a
 // lane apart (word k of lane l at [k * 32 + l]). The copies are asynchronous and each lane waits for its own, so a
-// color's records arrive while the group is still at the color before it. Rooms pay where contacts outweigh bodies:
-// 16 impact worlds (66 bodies, 490 contacts in 26 colors each) take 1840 us of substeps a step with them and 2570
-// without, 1024 of them 2760 and 4281, the box pyramid 344 and 377; but they leave an SM eight warps, and the 121-body
-// worlds of the uneven batch (0.2 to 0.5 contacts a body) then take 3312 us where they take 1952 without.
+// color's records arrive while the group is still at the color before it. They leave an SM eight warps, so they pay
+// where the contacts outweigh the bodies by far and each color's records fit the group's rooms at once.
 constexpr uint32_t kRoomWarps = 8;  // warps of a CTA with rooms
 constexpr uint32_t kRoomBytes = kRowWords * 32 * (uint32_t)sizeof(float4);
 
@@ -3531,13 +3552,6 @@ __device__ void runJoints(const Batch& B, const StepParams& P, const G& g, const
         putEnd(j.bodyA, a);
         putEnd(j.bodyB, b);
     });
-}
-
-// Whether the batch's active contacts outweigh its bodies, two to one: solved with rooms then (kRoomWarps). The
-// lines measured lie at 7.4 contacts a body (impact walls) and 2.8 (the pyramid) on one side, 0.5 and less on the
-// other.
-__device__ __forceinline__ bool contactsOutweigh(const Batch& B) {
-    return *(volatile uint32_t*)(B.work + kSlotActive) >= 2 * B.totalBodies;
 }
 
 // Integrate velocities, warm start, biased solve, integrate positions, relax (src/world.cpp:1669-1680). The
