@@ -2118,6 +2118,9 @@ __device__ __forceinline__ SixVec getSix(const float4* R, int first) {
 template <int First, int End, class T>
 __device__ __forceinline__ T readPieces(const T& x) {
     T out;
+#if defined(TF_DEVICE_CHECKS)
+    memset(&out, 0x3f, sizeof(out));
+#endif
     const float4* from = reinterpret_cast<const float4*>(&x);
 #pragma unroll
     for (int k = First; k < End; ++k) {
@@ -4327,8 +4330,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_finish(const __grid_constant__ Ba
         for (uint32_t i = g.tid; i < wi.bodyCount; i += g.size) {
             const uint32_t gb = wi.bodyFirst + i;
             DBody& d = B.bodies[gb];
-            DBody b = readBody<kBodySolve | kBodyForce | kBodyPose | kBodyCom | kBodyLocal | kBodyInvMass | kBodyStart |
-                               kBodyBounds | kBodyShapes>(d);
+            DBody b = readBody<kBodySolve | kBodyForce | kBodyPose | kBodyCom | kBodyLocal | kBodyInvMass | kBodyLocks |
+                               kBodyStart | kBodyBounds | kBodyShapes>(d);
             parent[i] = i;
             islandTime[i] = __float_as_uint(FLT_MAX);
             B.struck[gb] = (uint8_t)((movingBody(b) ? kEndMoves : 0u) |

@@ -114,6 +114,7 @@ constexpr uint64_t kBodyLocal = bodyPieces(offsetof(DBody, localCenter), offseto
 constexpr uint64_t kBodyBase = bodyPieces(offsetof(DBody, qBase), offsetof(DBody, invMassWorld));
 constexpr uint64_t kBodyInvMass = bodyPieces(offsetof(DBody, invMassWorld), offsetof(DBody, inertia));
 constexpr uint64_t kBodyInertia = bodyPieces(offsetof(DBody, inertia), offsetof(DBody, q0));
+constexpr uint64_t kBodyLocks = bodyPieces(offsetof(DBody, locks), offsetof(DBody, q0));
 constexpr uint64_t kBodyStart = bodyPieces(offsetof(DBody, q0), offsetof(DBody, lo));
 constexpr uint64_t kBodyBounds = bodyPieces(offsetof(DBody, lo), offsetof(DBody, shapeCount));
 constexpr uint64_t kBodyShapes = bodyPieces(offsetof(DBody, shapeFirst), offsetof(DBody, target));
@@ -130,10 +131,14 @@ static_assert((kBodyInvInertia & kBodyForce) == 0 && (kBodyForce & kBodyProj) ==
 // Some pieces of a body as one copy: the loads are 16 bytes wide and none waits for another. (Field by field, each
 // load of the 32 threads of a warp touches 32 separate lines, four bytes of each, and most wait for a branch or for a
 // store in between: the phases over bodies spent about 1000 cycles on every load they issued.) The fields outside the
-// pieces are not set.
+// pieces are not set; builds that check (TF_DEVICE_CHECKS) give them a value that none of them has, a flag, a count and
+// a length of about 0.75 alike, so that a phase that asks for one comes out differently.
 template <uint64_t Pieces>
 __device__ __forceinline__ DBody readBody(const DBody& d) {
     DBody b;
+#if defined(TF_DEVICE_CHECKS)
+    memset(&b, 0x3f, sizeof(b));
+#endif
     const float4* from = reinterpret_cast<const float4*>(&d);
 #pragma unroll
     for (int k = 0; k < (int)(sizeof(DBody) / 16); ++k) {
