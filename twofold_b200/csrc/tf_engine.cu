@@ -2019,7 +2019,6 @@ public:
         const bool rec = profiling && !capturing;
         chains = !capturing && worlds.size() <= (size_t)smCount / 2;
         auto threads = [&](int k) { return (int)shapes[k].threads; };
-        auto bigThreads = [&](int k) { return shapes[k].chosen ? threads(k) : std::max(threads(k), 256); };
         auto smem = [&](int k) { return (size_t)splits[k].smemBytes; };
         auto mark = [&](int k) {
             if (!marks) { return; }
@@ -2171,6 +2170,8 @@ public:
     static constexpr int kBigKernels[6] = { kKBroadBig, kKBroadFinishBig, kKNarrowphaseBig, kKPrepareBig, kKFinishBig,
                                             kKFinishJointsBig };
     static constexpr int kBigShapes[6] = { 0, 0, 1, 3, 6, 6 };
+    // A CTA's threads in a cluster: the shape's, at least 256 where it is the default (batches of many worlds have 128).
+    uint32_t bigThreads(int k) const { return shapes[k].chosen ? shapes[k].threads : std::max(shapes[k].threads, 256u); }
 
     // The clusters the big worlds' kernels run on: as many CTAs a world as leaves every world's cluster an SM a CTA
     // (a power of two, at most kMaxCluster and what the device can place), none if that is one.
@@ -2185,7 +2186,7 @@ public:
                 for (int i = 0; i < 6 && fits; ++i) {
                     cudaLaunchConfig_t cfg = {};
                     cfg.gridDim = dim3(ctas);
-                    cfg.blockDim = dim3(shapes[kBigShapes[i]].threads);
+                    cfg.blockDim = dim3(bigThreads(kBigShapes[i]));
                     cudaLaunchAttribute attr[1];
                     attr[0].id = cudaLaunchAttributeClusterDimension;
                     attr[0].val.clusterDim.x = ctas;
