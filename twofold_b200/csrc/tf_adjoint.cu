@@ -2131,15 +2131,16 @@ struct Run {
          *integLog = nullptr, *scratch = nullptr, *branches = nullptr;
     uint64_t logStride = 0;
     // What the buffers were allocated for; a run of the same sizes keeps them (allocating and freeing up to half the
-    // device's memory took 23 ms of a forward and 15 of a backward on 256 impact worlds x 48 steps).
+    // device's memory took 23 ms of a forward and 15 of a backward on 256 impact worlds x 48 steps), also over a tape
+    // recorded anew, whose largest step hardly ever has the same number of contact operations: the log has a capacity.
     struct Sizes {
-        size_t elem, bodies, shapes, slots, worlds, steps, substeps;
-        uint64_t calls;
+        size_t elem, bodies, shapes, contacts, worlds, steps, substeps;
         bool operator==(const Sizes& o) const {
-            return elem == o.elem && bodies == o.bodies && shapes == o.shapes && slots == o.slots && worlds == o.worlds &&
-                   steps == o.steps && substeps == o.substeps && calls == o.calls;
+            return elem == o.elem && bodies == o.bodies && shapes == o.shapes && contacts == o.contacts &&
+                   worlds == o.worlds && steps == o.steps && substeps == o.substeps;
         }
     } sizes{};
+    uint64_t calls = 0;  // operations of a world and step that the log holds
     int slots = 0;  // steps the backward recomputes at once; two sets of slots alternate
     uint32_t maxBodies = 0;  // the most bodies of a world, read once
     bool forwardDone = false;
@@ -2163,16 +2164,31 @@ struct Run {
         if (side) { cudaStreamDestroy(side); }
         if (walk) { cudaStreamDestroy(walk); }
     }
+    // The buffers that the backward allocates, and the forward's that it makes larger.
+    void releaseBackward() {
+        for (void** p : { &invM, &invI, &dp, &dq, &qBase, &points, &stateAdj, &dpAdj, &dqAdj, &qBaseAdj, &invMAdj, &invIAdj,
+                          &pointAdj, &muAdj, &muShares, &shareNext, &shareFirst, &massAdj, &frictionAdj, &log, &integLog,
+                          &scratch }) {
+            auto it = std::find(owned.begin(), owned.end(), *p);
+            if (it != owned.end()) {
+                cudaFree(*p);
+                owned.erase(it);
+            }
+            *p = nullptr;
+        }
+        calls = 0;
+        slots = 0;
+    }
     void release() {
         for (void* p : owned) { cudaFree(p); }
         owned.clear();
         for (void** p : { &mass, &friction, &init, &states, &invM, &invI, &dp, &dq, &qBase, &points, &stateAdj, &dpAdj,
-                          &dqAdj, &qBaseAdj, &invMAdj, &invIAdj, &pointAdj, &muAdj,
-                          &muShares, &shareNext, &shareFirst, &massAdj, &frictionAdj, &log, &integLog,
-                          &scratch, &branches }) {
+                          &dqAdj, &qBaseAdj, &invMAdj, &invIAdj, &pointAdj, &muAdj, &muShares, &shareNext, &shareFirst,
+                          &massAdj, &frictionAdj, &log, &integLog, &scratch, &branches }) {
             *p = nullptr;
         }
         sizes = Sizes{};
+        calls = 0;
         forwardDone = false;
         slots = 0;
         maxBodies = 0;
@@ -2254,6 +2270,11 @@ int download(std::vector<double>& dst, const void* src, size_t n, cudaStream_t s
 // Worlds an SM up to which the walks in double give a world a CTA and a contact four lanes (measured at backwardT).
 constexpr int kWideWorlds = 4;
 
+template <class T>
+Run::Sizes sizesOf(const AdjointSetup& S) {
+    return { sizeof(T), S.totalBodies, S.totalShapes, S.contactSlots, (size_t)S.nWorlds, (size_t)S.nSteps, (size_t)S.substeps };
+}
+
 // The largest number of contact operations one world logs in one step.
 int maxCalls(const AdjointSetup& S, uint64_t* out) {
     std::vector<TapeStep> steps(S.nSteps);
@@ -2277,9 +2298,7 @@ int forwardT(Run& r, const AdjointSetup& S, cudaStream_t stream, const double* i
              const double* friction, double* finalState) {
     const size_t nb = S.totalBodies, ns = S.totalShapes;
     int rc;
-    uint64_t calls = 0;
-    if ((rc = maxCalls(S, &calls)) != TF_OK) { return rc; }
-    const Run::Sizes sizes{ sizeof(T), nb, ns, S.contactSlots, (size_t)S.nWorlds, (size_t)S.nSteps, (size_t)S.substeps, calls };
+    const Run::Sizes sizes = sizesOf<T>(S);
     if (!(sizes == r.sizes)) { r.release(); }
     r.forwardDone = false;
     r.maxBodies = 0;
@@ -2363,44 +2382,30 @@ int backwardT(Run& r, const AdjointSetup& S, cudaStream_t stream, const double* 
               double* gradMass, double* gradFriction) {
     const size_t nb = S.totalBodies, ns = S.totalShapes;
     int rc;
-    // A tape recorded again since the forward run: one of other sizes does not fit the run's buffers, one of more
-    // operations a step needs a larger log.
-    Run::Sizes sizes = r.sizes;
-    if ((rc = maxCalls(S, &sizes.calls)) != TF_OK) { return rc; }
-    if (nb != sizes.bodies || ns != sizes.shapes || S.contactSlots != sizes.slots || (size_t)S.nWorlds != sizes.worlds ||
-        (size_t)S.nSteps != sizes.steps || (size_t)S.substeps != sizes.substeps) {
+    if (!(sizesOf<T>(S) == r.sizes)) {
         return noteError(TF_E_INVALID, "adjoint: the tape was recorded anew since the forward run");
     }
-    if (sizes.calls > r.sizes.calls && r.log) {
-        r.owned.erase(std::find(r.owned.begin(), r.owned.end(), r.log));
-        cudaFree(r.log);
-        r.log = nullptr;
-        if ((rc = r.alloc(&r.log, 2 * (size_t)r.slots * (size_t)S.nWorlds * sizes.calls * kCallWords * sizeof(T))) != TF_OK) {
-            r.release();
-            return rc;
-        }
-    }
-    r.sizes.calls = std::max(r.sizes.calls, sizes.calls);
-    r.logStride = r.sizes.calls * (uint64_t)kCallWords;
-    if (!r.log) {
+    uint64_t calls = 0;
+    if ((rc = maxCalls(S, &calls)) != TF_OK) { return rc; }
+    if (!r.log || calls > r.calls) {
+        // Also where a tape of more operations a step needs a larger log: then with a fourth to spare for the next one,
+        // where that leaves room for every step.
+        const bool again = r.log != nullptr;
+        // The forward's single-slot working arrays give way to one per slot.
+        r.releaseBackward();
         // Steps recomputed at once: as many slots as fit in a share of the free memory, up to the whole run.
-        const size_t perSlot = (size_t)S.nWorlds * r.logStride * sizeof(T) +
-                               (size_t)S.substeps * nb * kIntegWords * sizeof(T) + nb * (kState + 21) * sizeof(T) +
-                               (size_t)S.contactSlots * 4 * sizeof(PointState<T>);
+        auto perSlot = [&](uint64_t c) {
+            return (size_t)S.nWorlds * c * kCallWords * sizeof(T) + (size_t)S.substeps * nb * kIntegWords * sizeof(T) +
+                   nb * (kState + 21) * sizeof(T) + (size_t)S.contactSlots * 4 * sizeof(PointState<T>);
+        };
         size_t freeBytes = 0, totalBytes = 0;
         TF_ADJ_CUDA(cudaMemGetInfo(&freeBytes, &totalBytes));
         const size_t budget = std::min<size_t>(freeBytes / 2, (size_t)32 << 30);
-        r.slots = (int)std::max<size_t>(1, std::min<size_t>((size_t)S.nSteps, budget / 2 / std::max<size_t>(perSlot, 1)));
+        if (again && perSlot(calls + calls / 4) * (size_t)S.nSteps <= budget / 2) { calls += calls / 4; }
+        r.slots = (int)std::max<size_t>(1, std::min<size_t>((size_t)S.nSteps, budget / 2 / std::max<size_t>(perSlot(calls), 1)));
+        r.calls = calls;
+        r.logStride = calls * (uint64_t)kCallWords;
         const size_t k = 2 * (size_t)r.slots;
-        // The forward's single-slot working arrays give way to one per slot.
-        for (void** p : { &r.invM, &r.invI, &r.dp, &r.dq, &r.qBase, &r.points }) {
-            auto it = std::find(r.owned.begin(), r.owned.end(), *p);
-            if (it != r.owned.end()) {
-                cudaFree(*p);
-                r.owned.erase(it);
-            }
-            *p = nullptr;
-        }
         if ((rc = r.alloc(&r.invM, k * nb * sizeof(T))) || (rc = r.alloc(&r.invI, k * 9 * nb * sizeof(T))) ||
             (rc = r.alloc(&r.dp, k * 3 * nb * sizeof(T))) || (rc = r.alloc(&r.dq, k * 4 * nb * sizeof(T))) ||
             (rc = r.alloc(&r.qBase, k * 4 * nb * sizeof(T))) ||
