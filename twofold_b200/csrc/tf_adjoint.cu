@@ -2079,8 +2079,8 @@ __global__ void __launch_bounds__(128) k_model_reverse(const __grid_constant__ M
     }
 }
 
-// The same walk with a CTA a world. The dynamic shared memory holds, when `staged`, the two stage buffers and, when bodyCap is not zero, body arrays for up to bodyCap bodies
-// (no world has more).
+// The same walk with a CTA a world. The dynamic shared memory holds, when `staged`, the two stage buffers and, when
+// bodyCap is not zero, body arrays for up to bodyCap bodies (no world has more).
 template <class T>
 __global__ void __launch_bounds__(kWalkThreads, 2) k_model_reverse_wide(const __grid_constant__ Model<T> M, int first, int count,
                                                                            uint32_t slotBase, int staged, uint32_t bodyCap) {

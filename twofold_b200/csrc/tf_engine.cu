@@ -2222,7 +2222,7 @@ public:
     // has more than 512 bodies); batches of many worlds give worlds of up to 32 bodies a warp each and the
     // larger ones a CTA of 128 threads, with 32 KB of staging. Measured against 256 threads, 64 KB and a warp each up to
     // 96 bodies, us a step: 1024 impact worlds of 66 bodies: broadphase 130 and 168, narrowphase 207 and 322, prepare
-    // 564 and 673, finish 364 and 501; 4096 uneven worlds of 8 to 232: 210 and 250, 95 and 125, 276 and 345, 439 and
+    // 564 and 673, finish 364 and 501; 4096 uneven worlds of 8 to 512: 210 and 250, 95 and 125, 276 and 345, 439 and
     // 457; 1024 jointed worlds of 26: 25 and 26, 11 and 11, 22 and 21, 171 and 175.
     //
     // The substep's, measured (us of substeps a step). Many worlds take 128 threads and a CTA past 32 bodies (4096
@@ -2230,9 +2230,10 @@ public:
     // threads and 96 bodies; 600 jointed worlds: 856 against 1045 flat), except: jointed worlds from 8 an SM on, solved
     // flat (1400: 1326 and 1072 flat, 2000: 1544 and 1115; 1024: 1103 and 1040), and fewer than 8 worlds an SM with some
     // past 128 bodies, which keep the flat solve that programs reading the shape in use know as their default (1024
-    // uneven worlds: 157 flat and 155 at step 2, but 750 and 605 at step 18 and 1098 and 768 at step 40: worth tuning). A few worlds take a CTA each, unless one has so many bodies that one SM holds up the step: then
-    // the whole batch is solved flat (planar piles of 1017 bodies: 171 with a CTA and 218 flat, 4065: 413 and 279;
-    // terrain of 4097: 855 and 769; pyramids of 1036 boxes: 677 and 676, 2081: 1609 and 659).
+    // uneven worlds: 157 flat and 155 at step 2, but 750 and 605 at step 18 and 1098 and 768 at step 40: worth tuning). A
+    // few worlds take a CTA each, unless one has so many bodies that one SM holds up the step: then the whole batch is
+    // solved flat (planar piles of 1017 bodies: 171 with a CTA and 218 flat, 4065: 413 and 279; terrain of 4097: 855 and
+    // 769; pyramids of 1036 boxes: 677 and 676, 2081: 1609 and 659).
     LaunchShape defaultShape(int k) const {
         LaunchShape s;
         const bool many = manyWorlds();

@@ -73,9 +73,6 @@ TF_HD Mat3 skewOf(const Vec3& v) {
 
 TF_HD float traceOf(const Mat3& m) { return m.r[0].x + m.r[1].y + m.r[2].z; }
 
-// The inverse of m on the directions it acts in (src/joint.cpp:21-70): the plain inverse when m is well
-// conditioned, else cyclic Jacobi rotations of its symmetric part and the reciprocals of its eigenvalues above
-// a relative floor.
 // One Jacobi rotation of rows and columns p and q, known to the compiler so that the matrices stay in registers.
 template <int p, int q>
 TF_HD void jacobiTurn(float (&a)[3][3], float (&v)[3][3]) {
@@ -103,8 +100,10 @@ TF_HD void jacobiTurn(float (&a)[3][3], float (&v)[3][3]) {
     }
 }
 
-// Out of line: the joints of a pass reach it from a dozen places, and inlined its copies overran the instruction
-// cache.
+// The inverse of m on the directions it acts in (src/joint.cpp:21-70): the plain inverse when m is well
+// conditioned, else cyclic Jacobi rotations of its symmetric part and the reciprocals of its eigenvalues above
+// a relative floor. Out of line: the joints of a pass reach it from a dozen places, and inlined its copies overran
+// the instruction cache.
 TF_HD_OUTLINE Mat3 pseudoInverse(const Mat3& m) {
     const float tr = traceOf(m);
     if (tr <= 0.0f) { return mzero(); }

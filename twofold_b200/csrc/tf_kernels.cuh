@@ -974,7 +974,8 @@ __global__ void __launch_bounds__(kMaxBlock, 1) k_broadphase(const __grid_consta
         // bodies at a time are held against the block's common bounds, and only those that reach them are tested. The
         // pairs found wait in the warp's queue until a lane each can work on them. (A warp per first body, its lanes
         // over the second ones, read both from shared memory for each test and followed a found pair's shapes with
-        // its other lanes waiting: 741 us of broadphase for the 4096 uneven worlds and 187 for 64 of them, 274 and 56 now.)
+        // its other lanes waiting: 741 us of broadphase for the 4096 uneven worlds and 187 for 64 of them, 274 and 56 with
+        // blocks at the same launch shape, 210 for the 4096 at the default one.)
         uint32_t* queue = s_queue[threadIdx.x >> 5];
         uint32_t queued = 0;
         auto work = [&](uint32_t items) {  // the queue's first items
