@@ -2004,9 +2004,9 @@ public:
         B.nPolys = (uint32_t)nPolys;
         B.totalBodies = (uint32_t)totalBodies;
         B.roomContacts = roomContacts;
-        B.roomBodies = shapes[5].chosen || !manyWorlds() ? ~0u : roomsSplit.bigBodies;
+        B.roomBodies = manyWorlds() && !shapes[5].chosen ? roomsSplit.bigBodies : ~0u;
         B.roomWarpBodies = roomsSplit.bigBodies;
-        B.roomThreads = shapes[5].chosen ? ~0u : roomsThreads;
+        B.roomThreads = roomsThreads;
         return B;
     }
 
@@ -2139,7 +2139,9 @@ public:
     //
     // An SM holds one CTA with rooms and two without, so it matters how the worlds fill the rounds of either: two contacts
     // a body are enough up to a world an SM and in a third round, eight are needed in a second one that is mostly empty,
-    // four in one that is nearly full and in a fourth. Measured, us of substeps a step with and without, 148 SMs: 148
+    // four in one that is nearly full and in a fourth. A shape that was chosen goes by the same lines. (With rooms whenever
+    // there were two contacts a body, a tuned batch of 32 pyramids of 562 boxes took 660 us with 512 threads chosen, 483
+    // now, 170 pyramids of 211 624 and 569.) Measured, us of substeps a step with and without, 148 SMs: 148
     // impact worlds (7.4 contacts a body) 1114 and 1693, 170 2030 and 1739, 220 2111 and 2021, 296 2174 and 2377, 440
     // 3189 and 4121, 590 4229 and 4691; pyramids of 79 boxes (2.7) 301 and 396, 546 and 417, 551 and 425, 558 and 443,
     // 815 and 812, 1072 and 844; blocks of 125 boxes (8.4) 1169 and 2457, 2142 and 2533, 2157 and 2574, 2278 and 2607,
@@ -2162,7 +2164,7 @@ public:
         const int wanted = worldsGrid(roomsSplit.bigBodies, warps), rounds = (wanted + smCount - 1) / smCount;
         roomsGrid = std::min(wanted, smCount);
         const bool emptySecond = rounds == 2 && 4 * wanted <= 7 * smCount;
-        roomContacts = manyWorlds() || sh.chosen || rounds == 1 || rounds == 3 ? 2u : emptySecond ? 8u : 4u;
+        roomContacts = (manyWorlds() && !sh.chosen) || rounds == 1 || rounds == 3 ? 2u : emptySecond ? 8u : 4u;
         return TF_OK;
     }
 
